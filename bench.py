@@ -137,8 +137,9 @@ def measured_peak_hbm():
 
 
 def launches_per_step(precision, periodic_x):
-    """Kernel launches of one step: stage (a), the flux kernel and, in FP64 and
-    the 16-bit forms with periodic x, the separate ghost pass of f-bar-plus."""
+    """Kernel launches of one step: stage (a), the flux kernel and, in FP64, the
+    redo of steps out of the fixed-point range (or, where the FP64 kernels run, the
+    ghost pass of f-bar-plus, as in the 16-bit forms with periodic x)."""
     if precision == "fp32" or (precision in ("fp16", "bf16") and not periodic_x):
         return 2
     return 3
@@ -159,28 +160,6 @@ def ncu_traffic(precision, grid):
         return None, None
     return e["dram_bytes"], {"source": "profiles/traffic.json (committed ncu capture, not measured in this run)",
                              "kernel": e["kernel"], "command": d.get("command")}
-
-
-def fp64_inst_per_cell(kernel):
-    """FP64 thread instructions per cell of `kernel` from the committed ncu capture."""
-    p = os.path.join(ROOT, "profiles", "traffic.json")
-    try:
-        return json.load(open(p))["fp64_inst_per_cell"][kernel]
-    except Exception:
-        return None
-
-
-def fp64_pipe_peak(stream):
-    """FP64 FMA thread instructions per second, measured now (dugks-gpu_gb300/libdg_peak.so)."""
-    import ctypes
-    L = ctypes.CDLL(os.path.join(ROOT, "dugks-gpu_gb300", "libdg_peak.so"))
-    L.dg_probe_fp64_fma_rate.restype = ctypes.c_int
-    L.dg_probe_fp64_fma_rate.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
-    rate = ctypes.c_double(0.0)
-    rc = L.dg_probe_fp64_fma_rate(ctypes.c_void_p(stream), 20, ctypes.byref(rate))
-    if rc != 0:
-        raise RuntimeError(f"FP64 probe failed with CUDA error {rc}")
-    return rate.value
 
 
 def combine_ranks(world, n_cells, steps, ms_local, dist=None, device="cpu"):
@@ -404,24 +383,13 @@ def main():
     achieved = flux_bytes / (ms_b / K / 1e3) / 1e9
     peak, peak_kind = measured_peak_hbm()
     traffic, traffic_src = ncu_traffic(args.precision, grid)
-    roof = {"bound": "hbm", "kernel": "flux_kernel", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    names = ("fbar_fx_kernel", "flux_fx_kernel") if args.precision == "fp64" else ("fbar_kernel", "flux_tma_kernel")
+    roof = {"bound": "hbm", "kernel": names[1], "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic, "traffic_from": traffic_src,
             "peak_source": peak_kind, "alg_bytes_per_cell": 57 * info_bytes,
-            "kernel_ms": {"fbar_kernel": ms_a / K, "flux_kernel": ms_b / K},
+            "kernel_ms": {names[0]: ms_a / K, names[1]: ms_b / K},
             "step_alg_bytes_per_cell": 95 * info_bytes,
             "step_frac": 95 * info_bytes * n * K / (ms / 1e3) / 1e9 / peak}
-    if args.precision == "fp64":
-        # the FP64 step is bound by FP64 instruction issue: its compute roofline
-        per_cell = fp64_inst_per_cell("flux_kernel")
-        dp_peak = fp64_pipe_peak(torch.cuda.current_stream().cuda_stream)
-        comp = {"bound": "fp64 pipe", "kernel": "flux_kernel", "unit": "T FP64 inst/s", "peak": dp_peak / 1e12,
-                "peak_source": "measured in this run: FP64 FMA chains on every SM (libdg_peak.so)",
-                "fp64_inst_per_cell": per_cell}
-        if per_cell:
-            comp["achieved"] = per_cell * n / (ms_b / K / 1e3) / 1e12
-            comp["frac"] = comp["achieved"] / comp["peak"]
-        roof["compute"] = comp
-
     extras = {}
     if rank == 0 and world == 1 and not args.no_extras:
         forms = {}

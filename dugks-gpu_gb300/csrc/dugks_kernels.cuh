@@ -441,16 +441,15 @@ __device__ __forceinline__ void fbar_one_axis(T r, T u, T vv, T w, T B, T Kb, T 
     pair(16, 17, w3 - v3, 2);
 }
 
+// One block of the grid, block (bx, j, k) of bdim threads; tid: the thread within it.
 template <class T, class S, int GHOST>
-__global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> P,
-                                                   int xoff)
+__device__ __forceinline__ void fbar_block(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> &P,
+                                           int xoff, int tid, int bx, int bdim, int j, int k)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x - xoff;
-    const int j = blockIdx.y;
-    const int k = blockIdx.z;
+    const int i = bx * bdim + tid - xoff;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const bool in = i >= 0 && i < nx;
-    const int wbase = blockIdx.x * blockDim.x + (threadIdx.x & ~31) - xoff;  // cell of lane 0
+    const int wbase = bx * bdim + (tid & ~31) - xoff;  // cell of lane 0
     const bool wall_warp =
         GHOST == 1 && !P.periodic_x && ((wbase <= 1 && wbase + 31 >= 0) || (wbase <= nx - 1 && wbase + 31 >= nx - 2));
     if (!in && !wall_warp) return;
@@ -626,7 +625,7 @@ __global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *_
         }
     };
     const long long rowb = cb - (ic + 1);  // stored column 0 of this row and plane
-    const int wl = threadIdx.x >> 5;
+    const int wl = tid >> 5;
 #pragma unroll
     for (int p = 0; p < NPOP; ++p) {
         const T out = ob[p];
@@ -650,7 +649,7 @@ __global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *_
     }
     if (wall_warp) {
         __syncwarp();
-        const int lane = threadIdx.x & 31;
+        const int lane = tid & 31;
         if (lane < NPOP) {
             const int p = lane;
             S *pl = fb + p * P.ps_b + rowb;
@@ -668,6 +667,13 @@ __global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *_
     }
 }
 
+template <class T, class S, int GHOST>
+__global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> P,
+                                                   int xoff)
+{
+    fbar_block<T, S, GHOST>(f, fb, P, xoff, threadIdx.x, blockIdx.x, blockDim.x, blockIdx.y, blockIdx.z);
+}
+
 // ---------------------------------------------------------------------------
 // Ghost layer of f-bar-plus: every ghost cell takes its value from the
 // interior -- the periodic image in y and z (the reference's extend_fb_y and
@@ -680,14 +686,18 @@ __global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *_
 // y rows 0 and ny+1 for interior columns and all planes, z planes 0 and nz+1
 // for the interior columns and rows.
 // ---------------------------------------------------------------------------
+__host__ __device__ inline long long fb_ghosts(int nx, int ny, int nz)
+{
+    return 2LL * (ny + 2) * (nz + 2) + 2LL * nx * (nz + 2) + 2LL * nx * ny;
+}
+
 template <class T, class S>
-__global__ void __launch_bounds__(256) fb_ghost_kernel(S *__restrict__ fb, const StepParams<T, S> P)
+__device__ __forceinline__ void fb_ghost_cell(S *__restrict__ fb, const StepParams<T, S> &P, long long q)
 {
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const long long nxg = 2LL * (ny + 2) * (nz + 2);
     const long long nyg = 2LL * nx * (nz + 2);
     const long long nzg = 2LL * nx * ny;
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int gi, gj, gk;
     if (q < nxg) {
         gi = (q & 1) ? nx + 1 : 0;
@@ -731,6 +741,12 @@ __global__ void __launch_bounds__(256) fb_ghost_kernel(S *__restrict__ fb, const
     }
 }
 
+template <class T, class S>
+__global__ void __launch_bounds__(256) fb_ghost_kernel(S *__restrict__ fb, const StepParams<T, S> P)
+{
+    fb_ghost_cell(fb, P, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // ---------------------------------------------------------------------------
 // Stages (b)/(c), (d), (e): face reconstruction, face flux, finite-volume update.
 //
@@ -764,6 +780,19 @@ struct FbRead {
     __device__ __forceinline__ T dec(int p, T x) const { return codec.dec(p, x); }
     __device__ __forceinline__ T dec_e(int p, T x) const { return codec.dec_e(p, x); }
     __device__ __forceinline__ float2 dec_e2(int p, int q, float2 x) const { return codec.dec_e2(p, q, x); }
+};
+
+// The same for f-bar-plus written earlier in the same launch by other SMs (coherent loads)
+template <class T, class S>
+struct FbReadCoherent : FbRead<T, S> {
+    using FbRead<T, S>::fb;
+    using FbRead<T, S>::ps;
+    using FbRead<T, S>::codec;
+    __device__ __forceinline__ T operator()(int p, long long row, int col) const
+    {
+        return codec.dec(p, T(__ldcg(fb + p * ps + row + col)));
+    }
+    __device__ __forceinline__ T raw(int p, long long row, int col) const { return T(__ldcg(fb + p * ps + row + col)); }
 };
 
 // 19 reconstructed values of one face, trilinear characteristic interpolation
@@ -1464,20 +1493,20 @@ __device__ __forceinline__ void face_fluxes(const StepParams<T, S> &P, const RD 
     face_flux<T, S, AX, FF>(P, v, out, FF ? face_field<T, S, AX>(P, i, j, k) : T(0));
 }
 
-template <class T, class S, int W, int RECON, int MINB, bool FF>
-__global__ void __launch_bounds__(32 * W, MINB) flux_kernel(const S *__restrict__ fb, const S *f_in, S *f_out,
-                                                       const StepParams<T, S> P, int kchunk)
+template <class T, class S, int W, int RECON, bool FF, class RD = FbRead<T, S>>
+__device__ __forceinline__ void flux_block(const S *__restrict__ fb, const S *f_in, S *f_out,
+                                           const StepParams<T, S> &P, int kchunk, int bx, int by, int bz)
 {
     static_assert(4 * (W - 1) <= 32, "the halo warp evaluates 4 planes x (W-1) rows of -x faces at once");
     __shared__ T ysh[2][W][10][32];  // +y face fluxes of every warp row (double buffer)
     __shared__ T xsh[2][4][W][10];   // -x face fluxes of the first column: [batch parity][plane of batch][row]
     const int lane = threadIdx.x, wr = threadIdx.y;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
-    const int i0 = blockIdx.x * 32 + 1;           // first column of the tile (1-based)
-    const int j0 = blockIdx.y * (W - 1) + 1;      // first row of the tile (1-based)
-    const int kb = blockIdx.z * kchunk + 1;
+    const int i0 = bx * 32 + 1;           // first column of the tile (1-based)
+    const int j0 = by * (W - 1) + 1;      // first row of the tile (1-based)
+    const int kb = bz * kchunk + 1;
     const int ke = min(kb + kchunk, nz + 1);
-    const FbRead<T, S> R{fb, P.ps_b, P.pitch_b, ny, nz, P.codec};
+    const RD R{fb, P.ps_b, P.pitch_b, ny, nz, P.codec};
 
     // warps 1..W-1: cell (gi, gj); warp 0: halo
     const int gi = i0 + lane;
@@ -1553,6 +1582,13 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_kernel(const S *__restrict_
         }
         buf ^= 1;
     }
+}
+
+template <class T, class S, int W, int RECON, int MINB, bool FF>
+__global__ void __launch_bounds__(32 * W, MINB) flux_kernel(const S *__restrict__ fb, const S *f_in, S *f_out,
+                                                       const StepParams<T, S> P, int kchunk)
+{
+    flux_block<T, S, W, RECON, FF>(fb, f_in, f_out, P, kchunk, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------

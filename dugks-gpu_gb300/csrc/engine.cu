@@ -33,6 +33,7 @@
 
 #include "../../include/dugks_gb300.h"
 #include "config.h"
+#include "fixed_launch.cuh"
 #include "launch.cuh"
 #include "spectral_kernels.cuh"
 
@@ -161,6 +162,13 @@ struct dg_ctx {
     cudaGraphExec_t step_graph = nullptr;
     long long acc_count = 0;
     bool macro_valid = false;
+    // fixed-point FP64 step (fixed_kernels.cuh): plan of the handles whose parameters fit,
+    // its per-column table and flags on the device
+    std::unique_ptr<FxPlan> fx;
+    FxMul *fx_tab = nullptr;
+    int *fx_flag = nullptr;  // [0] range flag, [1] last step redone in FP64
+    bool fb_fixed = false;  // f-bar-plus holds fixed-point values
+    bool fb_shown = false;  // the caller holds f-bar-plus's address: it is kept in FP64
 
     ~dg_ctx()
     {
@@ -176,6 +184,8 @@ struct dg_ctx {
         if (dev_err) cudaFree(dev_err);
         if (step_graph) cudaGraphExecDestroy(step_graph);
         if (cap_stream) cudaStreamDestroy(cap_stream);
+        if (fx_tab) cudaFree(fx_tab);
+        if (fx_flag) cudaFree(fx_flag);
         if (spec) cudaFree(spec);
         if (spec_order) cudaFree(spec_order);
         if (spec_off) cudaFree(spec_off);
@@ -652,19 +662,40 @@ bool graph_eligible(const dg_ctx *h)
     return true;
 }
 
+// FP64 steps that run in fixed point: the plan exists, no force field is set and
+// the caller has not asked for f-bar-plus
+bool uses_fixed(const dg_ctx *h) { return h->fx && !h->ffield && !h->fb_shown; }
+
+// the two parts of one step, f-bar-plus of `in`, then the state `out` from it
+template <class T, class S>
+cudaError_t launch_stage_a(dg_ctx *h, const S *in, const StepParams<T, S> &P, cudaStream_t st)
+{
+    if constexpr (std::is_same<S, double>::value) {
+        h->fb_fixed = uses_fixed(h);
+        if (h->fb_fixed) return launch_fixed_a(*h->fx, in, h->fb, h->fx_flag, st);
+    }
+    return Kern<T, S>::fbar(in, static_cast<S *>(h->fb), P, st);
+}
+template <class T, class S>
+cudaError_t launch_flux(dg_ctx *h, const S *in, S *out, const StepParams<T, S> &P, cudaStream_t st)
+{
+    if constexpr (std::is_same<S, double>::value) {
+        if (h->fb_fixed) return launch_fixed_flux(*h->fx, in, out, h->fb, h->fx_flag, st);
+    }
+    return Kern<T, S>::flux(static_cast<S *>(h->fb), in, out, P, h->recon, h->have_tmap ? &h->tmap : nullptr, st);
+}
+
 template <class T, class S>
 int ensure_step_graph(dg_ctx *h, const StepParams<T, S> &P)
 {
-    using K = Kern<T, S>;
     if (h->step_graph) return DG_OK;
     if (!h->cap_stream) CK(cudaStreamCreateWithFlags(&h->cap_stream, cudaStreamNonBlocking), "stream create");
     S *f = static_cast<S *>(h->f);
-    S *fb = static_cast<S *>(h->fb);
     CK(cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal), "graph capture begin");
     cudaError_t le = cudaSuccess;
     for (int s = 0; s < kGraphSteps && le == cudaSuccess; ++s) {
-        le = K::fbar(f, fb, P, h->cap_stream);
-        if (le == cudaSuccess) le = K::flux(fb, f, f, P, h->recon, h->have_tmap ? &h->tmap : nullptr, h->cap_stream);
+        le = launch_stage_a(h, f, P, h->cap_stream);
+        if (le == cudaSuccess) le = launch_flux(h, f, f, P, h->cap_stream);
     }
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(h->cap_stream, &g);
@@ -688,23 +719,22 @@ int ensure_step_graph(dg_ctx *h, const StepParams<T, S> &P)
 template <class T, class S>
 int step_form(dg_ctx *h, int istep0, int n, cudaEvent_t *ev)
 {
-    using K = Kern<T, S>;
     S *f = static_cast<S *>(h->f);
-    S *fb = static_cast<S *>(h->fb);
     StepParams<T, S> P = params_for<T, S>(h, istep0);
     int s = 0;
     if (!ev && n >= 2 * kGraphSteps && graph_eligible<T, S>(h)) {
         const int rc = ensure_step_graph<T, S>(h, P);
         if (rc) return rc;
         for (; s + kGraphSteps <= n; s += kGraphSteps) CK(cudaGraphLaunch(h->step_graph, h->stream), "graph launch");
+        h->fb_fixed = uses_fixed(h);
     }
     if (ev) CK(cudaEventRecord(ev[0], h->stream), "event record");
     for (; s < n; ++s) {
         if (h->perturb && s > 0) P = params_for<T, S>(h, istep0 + s);
         set_round_seed<T, S>(h, P.codec, istep0 + s);
-        CK(K::fbar(f, fb, P, h->stream), "stage (a) launch");
+        CK(launch_stage_a(h, f, P, h->stream), "stage (a) launch");
         if (ev) CK(cudaEventRecord(ev[2 * s + 1], h->stream), "event record");
-        CK(K::flux(fb, f, f, P, h->recon, h->have_tmap ? &h->tmap : nullptr, h->stream), "flux launch");
+        CK(launch_flux(h, f, f, P, h->stream), "flux launch");
         if (ev) CK(cudaEventRecord(ev[2 * s + 2], h->stream), "event record");
     }
     h->macro_valid = false;
@@ -718,17 +748,15 @@ int step_form(dg_ctx *h, int istep0, int n, cudaEvent_t *ev)
 template <class T, class S>
 int step_between_form(dg_ctx *h, int istep0, int n, const void *src, void *dst)
 {
-    using K = Kern<T, S>;
     const S *fi = static_cast<const S *>(src);
     S *fo = static_cast<S *>(dst);
-    S *fb = static_cast<S *>(h->fb);
     StepParams<T, S> P = params_for<T, S>(h, istep0);
     for (int s = 0; s < n; ++s) {
         if (h->perturb && s > 0) P = params_for<T, S>(h, istep0 + s);
         set_round_seed<T, S>(h, P.codec, istep0 + s);
         const S *in = s == 0 ? fi : fo;
-        CK(K::fbar(in, fb, P, h->stream), "stage (a) launch");
-        CK(K::flux(fb, in, fo, P, h->recon, h->have_tmap ? &h->tmap : nullptr, h->stream), "flux launch");
+        CK(launch_stage_a(h, in, P, h->stream), "stage (a) launch");
+        CK(launch_flux(h, in, fo, P, h->stream), "flux launch");
     }
     if (fo == h->f) h->macro_valid = false;
     return DG_OK;
@@ -740,6 +768,7 @@ int step_between_form(dg_ctx *h, int istep0, int n, const void *src, void *dst)
 double *state_staging(dg_ctx *h, size_t bytes, bool *owned)
 {
     *owned = false;
+    h->fb_fixed = false;
     if (h->fb && size_t(h->ps_b) * 19 * storage_bytes(h->prec) >= bytes) return static_cast<double *>(h->fb);
     double *tmp = nullptr;
     if (cudaMalloc(&tmp, bytes) != cudaSuccess) return nullptr;
@@ -896,6 +925,7 @@ int adjoint_form(dg_ctx *h, int istep, const void *f_n, const void *lam_next, vo
         CK(cudaMalloc(&h->dphi, h->ncell() * sizeof(double)), "cudaMalloc (field gradient)");
         CK(cudaMemsetAsync(h->dphi, 0, h->ncell() * sizeof(double), h->stream), "cudaMemset (field gradient)");
     }
+    h->fb_fixed = false;
     CK(K::adjoint(static_cast<const S *>(f_n), static_cast<S *>(h->fb), static_cast<const S *>(lam_next),
                   static_cast<S *>(lam_out), static_cast<T *>(h->adj), params_for<T, S>(h, istep),
                   h->ffield ? h->dphi : nullptr, h->have_tmap ? &h->tmap_adj : nullptr, h->stream),
@@ -1123,6 +1153,103 @@ int make_tmap_form(dg_ctx *h)
     return DG_OK;
 }
 
+// Parameters of the fixed-point FP64 step, if this handle's fit its scaling
+// (fixed_kernels.cuh): trilinear reconstruction, a force along one axis at most and
+// no perturbation; every interpolation weight within (0, 1/2), every product's
+// multiplier below the limit of its scale (1/2 for dt/dx).  dt/dx stops at 0.45
+// (CFL 0.64), short of that limit: at CFL 0.7 the reference's laminar example runs,
+// whose profiles-2.dat is recorded byte for byte, with the FP64 kernels' rounding of
+// velocities near 1e-17 in it.  Otherwise h->fx stays empty and the FP64 kernels run.
+int make_fixed_plan(dg_ctx *h)
+{
+    const RefCoef<double> &c = h->c64;
+    const int nx = h->nx;
+    const int nf = (c.F[0] != 0) + (c.F[1] != 0) + (c.F[2] != 0);
+    if (h->prec != DG_PREC_FP64 || h->recon != 0 || h->perturb || nf > 1) return DG_OK;
+    std::unique_ptr<FxPlan> L(new FxPlan());
+    FxParams &P = L->P;
+    P.nx = nx; P.ny = h->ny; P.nz = h->nz; P.pitch = h->pitch; P.ps = h->ps;
+    P.pitch_b = h->pitch_b;
+    if ((long long)h->ny * h->pitch_b * NPOP >= (1LL << 31)) return DG_OK;
+    P.rs = h->pitch_b * NPOP;
+    P.periodic_x = h->periodic[0];
+    L->fax = c.F[0] != 0 ? 0 : (c.F[1] != 0 ? 1 : (c.F[2] != 0 ? 2 : 3));
+    bool fit = true;
+    // multiplier of m at scale 2^64 m / unit: |m| must stay below unit / 2
+    auto mul = [&](double m, double unit) {
+        if (!(std::fabs(m / unit) < 0.4999)) {
+            fit = false;
+            return FxMul{0, 0};
+        }
+        return fx_split(i64(std::llrint(std::ldexp(m / unit, 64))));
+    };
+    auto weight = [&](double m) {
+        if (!(m >= 0)) fit = false;
+        return mul(m, 1);
+    };
+    std::vector<double> dxx(h->dxx);
+    if (h->mesh == 0) std::fill(dxx.begin(), dxx.end(), c.dx);
+    const double dmin = *std::min_element(dxx.begin(), dxx.end());
+    // flux scale: fw1 2^esh in (1/2, 1], one lower if dt/dx needs it
+    const double cmax = c.dt / std::min(dmin, std::min(c.dy, c.dz));
+    if (!(cmax < 0.45)) return DG_OK;
+    P.esh = 0;
+    while (P.esh < 30 && std::ldexp(c.fw1, P.esh) <= 0.5) ++P.esh;
+    if (P.esh > 0 && std::ldexp(c.fw1, P.esh) * cmax >= 0.4999) --P.esh;
+    const double s = std::ldexp(c.fw1, P.esh);
+    const double F = L->fax < 3 ? c.F[L->fax] : 0.0;
+    auto force = [&](double w0, double w2, double shift) {
+        FxForce f;
+        if (!(std::fabs(shift) < 0.01)) fit = false;
+        f.shift = i64(std::llrint(std::ldexp(3 * shift, 61)));
+        f.B = i64(std::llrint(std::ldexp(std::min(w2 / 18, 0.4999), 64)));
+        f.C = mul(w0 * F / 18, 1.0 / 8);
+        f.Kf = mul(3 * w0 * F / 18, 1);
+        // K = (w2 + force terms) rho / 18 with rho < 1.98 below 1/4
+        if (!((w2 + std::fabs(3 * w0 * F) * 2) * 1.98 / 18 < 0.2499)) fit = false;
+        return f;
+    };
+    P.cell = force(c.bw0, c.bw2, c.hdt * F);
+    P.face = force(c.fw0 / s, c.fw2 / s, 0.5 * c.hdt * F);
+    // bw1 = 1 - bw2 to the last place: the rest population takes the difference of the
+    // density and the others
+    P.bw1 = fx_split(i64((1ull << 63) - 9ull * u64(P.cell.B)));
+    P.third = fx_split(0x5555555555555555ll);
+    const double ty = c.hdt / c.dy, tz = c.hdt / c.dz;
+    P.ty = weight(ty); P.tz = weight(tz);
+    P.my = weight(0.5 - ty); P.mz = weight(0.5 - tz);
+    P.cy = mul(s * (c.dt / c.dy), 1); P.cz = mul(s * (c.dt / c.dz), 1);
+    double q0 = 2, q1 = 2;
+    if (h->mesh) {
+        q0 = (h->xc[2] - h->xc[0]) / (h->xc[2] - h->xc[1]);
+        q1 = (h->xc[nx + 1] - h->xc[nx - 1]) / (h->xc[nx] - h->xc[nx - 1]);
+    }
+    P.q0 = mul(q0 - 2, 1); P.q1 = mul(q1 - 2, 1);
+    P.stretched = h->mesh != 0;
+    std::vector<FxMul> tab(size_t(FXT_ROWS) * (nx + 2), FxMul{0, 0});
+    auto at = [&](int row, int col) -> FxMul & { return tab[size_t(row) * (nx + 2) + col]; };
+    for (int i = 0; i <= nx; ++i) {
+        const double a = dxx[i], b = dxx[i + 1], d = 0.5 * a + 0.5 * b;
+        at(FXT_MP, i) = weight((a / 2 - c.hdt) / d);
+        at(FXT_MM, i) = weight((b / 2 - c.hdt) / d);
+        at(FXT_D0, i) = mul((a / 2) / d - 0.5, 1);
+        if (i == 0) continue;
+        at(FXT_TXP, i) = weight(c.hdt / (0.5 * dxx[i] + 0.5 * dxx[i - 1]));
+        at(FXT_TXM, i) = weight(c.hdt / (0.5 * dxx[i] + 0.5 * dxx[i + 1]));
+        at(FXT_CX, i) = mul(s * (c.dt / dxx[i]), 1);
+    }
+    if (!fit) return DG_OK;
+    CK(cudaMalloc(&h->fx_tab, tab.size() * sizeof(FxMul)), "cudaMalloc (fixed-point table)");
+    CK(cudaMemcpy(h->fx_tab, tab.data(), tab.size() * sizeof(FxMul), cudaMemcpyHostToDevice), "table upload");
+    CK(cudaMalloc(&h->fx_flag, 2 * sizeof(int)), "cudaMalloc (range flag)");
+    CK(cudaMemset(h->fx_flag, 0, 2 * sizeof(int)), "cudaMemset (range flag)");
+    P.tab = h->fx_tab;
+    L->D = params_for<double, double>(h, 0);
+    CK(fixed_plan_setup(*L), "fixed-point kernel setup");
+    h->fx = std::move(L);
+    return DG_OK;
+}
+
 int allocate(dg_ctx *h)
 {
     const size_t sb = storage_bytes(h->prec);
@@ -1142,6 +1269,8 @@ int allocate(dg_ctx *h)
     CK(cudaMalloc(&h->dev_err, sizeof(int)), "cudaMalloc (error flag)");
     CK(cudaMemset(h->dev_err, 0, sizeof(int)), "cudaMemset (error flag)");
     int rc = h->prec == DG_PREC_FP64 ? upload_tables<double>(h) : upload_tables<float>(h);
+    if (rc) return rc;
+    rc = make_fixed_plan(h);
     if (rc) return rc;
     return DISPATCH(h, make_tmap_form);
 }
@@ -1775,13 +1904,44 @@ int dg_read_dump(dg_t *h, int step)
     return dg_set_state(h, f.data());
 }
 
+// The caller gets f-bar-plus's address: from here on it is kept in FP64, and what
+// the last fixed-point step left there is converted (unless that step was redone in
+// FP64).  NULL when the conversion fails.
+static const void *show_fb(dg_t *h)
+{
+    if (h->fx && !h->fb_shown) {
+        if (h->fb_fixed) {
+            const size_t bytes = size_t(h->ps_b) * 19 * sizeof(double);
+            int redone = 0;
+            cudaError_t e = cudaMemcpyAsync(&redone, h->fx_flag + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+            if (e == cudaSuccess && !redone) {
+                double *tmp = nullptr;
+                e = cudaMalloc(&tmp, bytes);
+                if (e == cudaSuccess) e = launch_fixed_decode(*h->fx, h->fb, tmp, h->stream);
+                if (e == cudaSuccess) e = cudaMemcpyAsync(h->fb, tmp, bytes, cudaMemcpyDeviceToDevice, h->stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+                if (tmp) cudaFree(tmp);
+            }
+            if (e != cudaSuccess) {
+                h->cuda_fail(e, "f-bar-plus in FP64");
+                return nullptr;
+            }
+            h->fb_fixed = false;
+        }
+        h->fb_shown = true;
+        h->drop_graph();
+    }
+    return h->fb;
+}
+
 const void *dg_device_ptr(const dg_t *h, int which)
 {
     if (!h) return nullptr;
     const size_t g = h->ghosted();
     switch (which) {
     case DG_BUF_F: return h->f;
-    case DG_BUF_FB: return h->fb;
+    case DG_BUF_FB: return show_fb(const_cast<dg_t *>(h));
     case DG_BUF_RHO: return h->macro;
     case DG_BUF_UX: return h->macro ? h->macro + g : nullptr;
     case DG_BUF_UY: return h->macro ? h->macro + 2 * g : nullptr;

@@ -1,0 +1,567 @@
+// The FP64 step in 64-bit fixed point (fixed.cuh): stage (a) and the flux / update
+// kernel of dugks_kernels.cuh with every distribution value an integer scaled 2^62.
+//
+// What bounds the FP64 step is FP64 issue (2.1 lanes per SM and clock, 861
+// instructions per cell), not memory; integer adds and products run on pipes that
+// are 4 to 30 times wider (fixed.cuh).  f-tilde stays FP64 in memory; it is read
+// exactly (its values have fewer bits than the fixed point) and rounded once when
+// written.  f-bar-plus, written and read by these two kernels only, is held in
+// fixed point.  Step of the 256 x 128 x 128 channel: 6.65 ms with the FP64 kernels,
+// 1.65 ms here (stage (a) 0.21, flux 1.45); 64^3 box 0.63 -> 0.18 ms, 64 x 32 x 32
+// channel 0.229 -> 0.078 ms.
+//
+// Error of the state against an 80-bit run of the same scheme (relative 2-norm):
+// 5e-17 after one step, the rounding of the stored values (FP64 kernels 2.4e-16 to
+// 3.2e-16), 6e-16 to 2e-15 after 1000 steps (2e-14 to 2.3e-13); total mass drifts by
+// 1e-17 in 1000 steps between walls (2e-13).
+//
+// Range.  The scaling is chosen for states near unit density: every f-tilde and
+// f-bar-plus (wall ghosts included) within (FX_LO, FX_HI) w_p, which holds up to
+// velocities of about 0.25.  Face values are convex combinations of f-bar-plus and
+// stay in that box, which bounds density (0.4 .. 1.98), momentum (|j| < 0.27),
+// 3 c_p.u (< 1.67, reached with the populations moving along c_p at the upper and
+// the others at the lower end) and the equilibrium polynomial (< 3.9) at every cell
+// and face, so that no sum or product overflows.  Stage (a) checks the box per value
+// (NaN and infinities fail it) and raises a device flag; the flux kernel then does
+// nothing and fp64_redo_kernel does the whole step in FP64.  The parameters have to
+// fit too (make_fixed_plan in engine.cu): a single force axis, interpolation weights
+// within (0, 1/2), dt/dx below about 1/2.
+#pragma once
+#ifdef __CUDACC__
+#include <cuda_runtime.h>
+#endif
+
+#include "d3q19.cuh"
+#include "fixed.cuh"
+
+namespace dg {
+
+constexpr double FX_LO = 0.4, FX_HI = 1.98;
+constexpr i64 FX_ONE = 1ll << 62;
+
+// Equilibrium coefficients of a cell (stage (a)) or a face:
+//   K_p = w_p rho (B + c_p.Kf - Cf u), see fx_eq.
+struct FxForce {
+    i64 shift;   // 3 x velocity shift along the force axis, scaled 2^61
+    i64 B;       // (coefficient of feq without force) / 18, scaled 2^64
+    FxMul C;     // 3 u_a (scaled 2^61) -> its share of B (scaled 2^64)
+    FxMul Kf;    // rho (2^62) -> force term of K of an axis population along +a, scaled 2^62
+};
+
+struct FxParams {
+    int nx, ny, nz, pitch;  // f-tilde as in StepParams
+    long long ps;
+    int pitch_b, rs;        // f-bar-plus: columns per row (nx + 2 rounded up to 16), elements per row (19 pitch_b)
+    int periodic_x;
+    int esh;                // fluxes are held divided by fw1 2^esh, fw1 2^esh in (1/4, 1]
+    int stretched;          // x-face weights of the c_x = 0 populations differ from 1/2
+    FxForce cell, face;
+    FxMul bw1;              // 2 f (2^63) -> bw1 f (2^62)
+    FxMul third;            // 1/3
+    FxMul ty, tz;           // transverse weights hdt/dy, hdt/dz
+    FxMul my, mz;           // normal weight of the upwind-side cell, 1/2 - hdt/dy, 1/2 - hdt/dz
+    FxMul cy, cz;           // fw1 2^esh dt/dy, dt/dz
+    FxMul q0, q1;           // wall ghosts: extrapolation weight q, less 2
+    const FxMul *tab;       // [FXT_ROWS][nx + 2] per column / x face
+};
+constexpr int FXT_TXP = 0;  // transverse x weight of c_x > 0 at column i
+constexpr int FXT_TXM = 1;  // ... of c_x < 0
+constexpr int FXT_MP = 2;   // x face I: weight of cell I+1 for c_x > 0
+constexpr int FXT_MM = 3;   // ... of cell I for c_x < 0
+constexpr int FXT_D0 = 4;   // ... of cell I+1 for c_x = 0, less 1/2
+constexpr int FXT_CX = 5;   // column i: fw1 2^esh dt/dx
+constexpr int FXT_ROWS = 6;
+
+// f-bar-plus layout: row (k, j) of 0-based cells holds pitch_b columns in blocks of
+// 16, the 19 populations of a block one after another: a population step is the
+// constant 16 elements (an immediate of the load) and a warp's 32 cells are two
+// 128-byte pieces.  Column c = 0 .. nx-1: cells; nx: the ghost past the upper
+// wall (or image); nx + 1: the lower ghost.
+DG_FX int fx_col(int c) { return (c >> 4) * (NPOP * 16) + (c & 15); }
+
+// K_p coefficients, velocities and the equilibrium polynomial of a cell or face:
+//   feq_p = w_p rho (1 + x + x^2/2 - 1.5 u.u), x = 3 c_p.u
+struct FxEq {
+    i64 u3[3];       // 3 u, scaled 2^61 (force shift included)
+    i64 sq[3];       // (3 u_a)^2 / 2, scaled 2^61
+    i64 base;        // 1 - 1.5 u.u, scaled 2^61
+    FxMul K1[3], K2[3];  // K of axis / diagonal populations with c_a = 0, +1, -1 along the force axis, scaled 2^65
+};
+
+template <int FAX>
+DG_FX FxEq fx_eq(i64 rho, const i64 j[3], const FxForce &c, FxMul third)
+{
+    FxEq E;
+    const FxMul M = fx_recip3(rho);
+DG_UNROLL
+    for (int a = 0; a < 3; ++a) {
+        E.u3[a] = fx_mul(j[a] << 2, M) << 1;  // 4 j (2^62) x 3 / (16 rho) = 3 u 2^60
+        if (a == FAX) E.u3[a] += c.shift;
+        E.sq[a] = fx_sq(E.u3[a] << 1);
+    }
+    E.base = (1ll << 61) - fx_mul(E.sq[0] + E.sq[1] + E.sq[2], third);
+    if (FAX < 3) {
+        const i64 k = fx_mul(rho, fx_split(c.B - fx_mul(E.u3[FAX < 3 ? FAX : 0], c.C)));
+        const i64 d = fx_mul(rho, c.Kf);
+        E.K1[0] = fx_split(k << 3), E.K1[1] = fx_split((k + d) << 3), E.K1[2] = fx_split((k - d) << 3);
+        E.K2[0] = fx_split(k << 2), E.K2[1] = fx_split((k + d) << 2), E.K2[2] = fx_split((k - d) << 2);
+    } else {
+        const i64 k = fx_mul(rho, fx_split(c.B));
+        E.K1[0] = E.K1[1] = E.K1[2] = fx_split(k << 3);
+        E.K2[0] = E.K2[1] = E.K2[2] = fx_split(k << 2);
+    }
+    return E;
+}
+
+// acc_p += K_p (polynomial at +-x) for the opposite pair (p, opp(p))
+template <int FAX>
+DG_FX void fx_pair(const FxEq &E, int p, i64 &accp, i64 &accq)
+{
+    const int ax = cx(p), ay = cy(p), az = cz(p);
+    i64 x = 0;
+    if (ax) x += ax > 0 ? E.u3[0] : -E.u3[0];
+    if (ay) x += ay > 0 ? E.u3[1] : -E.u3[1];
+    if (az) x += az > 0 ? E.u3[2] : -E.u3[2];
+    const i64 t = E.base + (p <= 6 ? (ax ? E.sq[0] : (ay ? E.sq[1] : E.sq[2])) : fx_sq(x << 1));
+    const int ca = FAX < 3 ? cc(FAX, p) : 0;
+    const int sp = ca == 0 ? 0 : (ca > 0 ? 1 : 2), sq = ca == 0 ? 0 : (ca > 0 ? 2 : 1);
+    accp = fx_mad(t + x, p <= 6 ? E.K1[sp] : E.K2[sp], accp);
+    accq = fx_mad(t - x, p <= 6 ? E.K1[sq] : E.K2[sq], accq);
+}
+
+// Density and momentum of 19 values.
+DG_FX void fx_moments(const i64 v[NPOP], i64 &r, i64 j[3])
+{
+    r = v[0];
+    j[0] = j[1] = j[2] = 0;
+DG_UNROLL
+    for (int p = 1; p < NPOP; ++p) {
+        r += v[p];
+DG_UNROLL
+        for (int a = 0; a < 3; ++a)
+            if (cc(a, p)) j[a] += cc(a, p) > 0 ? v[p] : -v[p];
+    }
+}
+
+// f-bar-plus of one cell from f-tilde: bw1 f + K feq-polynomial; the rest
+// population from the density (sum f-bar-plus = rho exactly).
+template <int FAX>
+DG_FX void fx_stage_a(const FxParams &P, const i64 v[NPOP], i64 ob[NPOP])
+{
+    i64 rho, j[3];
+    fx_moments(v, rho, j);
+    const FxEq E = fx_eq<FAX>(rho, j, P.cell, P.third);
+    i64 rest = rho;
+DG_UNROLL
+    for (int p = 1; p < NPOP; ++p) {
+        const int q = opp(p);
+        if (q < p) continue;
+        ob[p] = fx_mul(v[p] << 1, P.bw1);
+        ob[q] = fx_mul(v[q] << 1, P.bw1);
+        fx_pair<FAX>(E, p, ob[p], ob[q]);
+        rest -= ob[p] + ob[q];
+    }
+    ob[0] = rest;
+}
+
+// Face fluxes divided by fw1 2^esh, in place: v holds the 10 face values that
+// cross the face (flux_pop order), m the sums over the other 9 of their values
+// and of their tangential momenta.
+template <int AX, int FAX>
+DG_FX void fx_face_flux(const FxParams &P, i64 v[10], const i64 m[3])
+{
+    constexpr int T1 = AX == 0 ? 1 : 0, T2 = AX == 2 ? 1 : 2;
+    i64 rho = m[0], j[3];
+    j[AX] = 0;
+    j[T1] = m[1];
+    j[T2] = m[2];
+DG_UNROLL
+    for (int s = 0; s < 10; ++s) {
+        const int p = flux_pop(AX, s);
+        rho += v[s];
+DG_UNROLL
+        for (int a = 0; a < 3; ++a)
+            if (cc(a, p)) j[a] += cc(a, p) > 0 ? v[s] : -v[s];
+    }
+    const FxEq E = fx_eq<FAX>(rho, j, P.face, P.third);
+DG_UNROLL
+    for (int s = 0; s < 10; ++s) {
+        const int p = flux_pop(AX, s), q = opp(p), sq = flux_slot(AX, q);
+        if (q < p) continue;
+        i64 fp = v[s] >> P.esh, fq = v[sq] >> P.esh;
+        fx_pair<FAX>(E, p, fp, fq);
+        v[s] = fp;
+        v[sq] = fq;
+    }
+}
+
+#ifdef __CUDACC__
+
+// Outside the box of the range comment.  f-tilde as FP64: positive values compare
+// like their high words.
+__device__ __forceinline__ bool fx_bad_double(double x, int p)
+{
+    const double w = weight<double>(p);
+    const unsigned lo = unsigned(__double2hiint(w * FX_LO)) + 1, hi = unsigned(__double2hiint(w * FX_HI));
+    return unsigned(__double2hiint(x)) - lo >= hi - lo;
+}
+__device__ __forceinline__ bool fx_bad(i64 x, int p)
+{
+    const double w = weight<double>(p);
+    const unsigned lo = unsigned(w * FX_LO * 1073741824.0) + 1, hi = unsigned(w * FX_HI * 1073741824.0);
+    return unsigned(x >> 32) - lo >= hi - lo;
+}
+
+// Stage (a), one thread per cell, x ghost columns included.  xoff: cells shifted by
+// one thread when nx = 1 (mod 32), so that cells nx-2 and nx-1 share a warp.
+template <int FAX>
+__global__ void __launch_bounds__(128) fbar_fx_kernel(const double *__restrict__ f, i64 *__restrict__ fb,
+                                                      const FxParams P, int xoff, int *flag)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x - xoff;
+    const int j = blockIdx.y, k = blockIdx.z, nx = P.nx;
+    const bool in = i >= 0 && i < nx;
+    const int ic = in ? i : (i < 0 ? 0 : nx - 1);
+    const double *src = f + ((long long)k * P.ny + j) * P.pitch + ic;
+    i64 v[NPOP], ob[NPOP];
+    bool bad = false;
+#pragma unroll
+    for (int p = 0; p < NPOP; ++p) {
+        const double x = __ldg(src + p * P.ps);
+        bad |= fx_bad_double(x, p);
+        v[p] = fx_from_double(x);
+    }
+    fx_stage_a<FAX>(P, v, ob);
+    i64 *row = fb + ((long long)k * P.ny + j) * P.rs;
+    i64 *dst = row + fx_col(ic);
+#pragma unroll
+    for (int p = 0; p < NPOP; ++p) {
+        bad |= fx_bad(ob[p], p);
+        if (in) dst[p * 16] = ob[p];
+    }
+    const int w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31) - xoff;  // cell of lane 0
+    if (w0 <= 0) {  // the warp of cell 0: the ghost below it, or the image of cell 0 above cell nx-1
+        i64 *g = row + fx_col(P.periodic_x ? nx : nx + 1);
+#pragma unroll
+        for (int p = 0; p < NPOP; ++p) {
+            const i64 n = __shfl_down_sync(0xffffffffu, ob[p], 1);
+            const i64 e = P.periodic_x ? ob[p] : fx_mad(ob[p] - n, P.q0, ob[p] + (ob[p] - n));
+            if (i == 0) {
+                bad |= fx_bad(e, p);
+                g[p * 16] = e;
+            }
+        }
+    }
+    if (w0 <= nx - 1 && w0 + 31 >= nx - 1) {  // the warp of cell nx-1
+        i64 *g = row + fx_col(P.periodic_x ? nx + 1 : nx);
+#pragma unroll
+        for (int p = 0; p < NPOP; ++p) {
+            const i64 n = __shfl_up_sync(0xffffffffu, ob[p], 1);
+            const i64 e = P.periodic_x ? ob[p] : fx_mad(ob[p] - n, P.q1, ob[p] + (ob[p] - n));
+            if (i == nx - 1) {
+                bad |= fx_bad(e, p);
+                g[p * 16] = e;
+            }
+        }
+    }
+    if (bad && in) atomicOr(flag, 1);
+}
+
+// Where f-bar-plus is read around a cell: plane pointers k-1..k+1, row and column
+// offsets of the neighbours (periodic in y and z, ghosts stored in x).
+struct FxAt {
+    const i64 *pl[3];
+    int row[3], col[3];
+    __device__ __forceinline__ i64 operator()(int p, int dx, int dy, int dz) const
+    {
+        return __ldg(pl[dz + 1] + (row[dy + 1] + col[dx + 1]) + p * 16);
+    }
+};
+
+// Transverse interpolation of every population at one cell for the faces normal to
+// AX: g[0..9] the populations that cross such a face, g[10..12] the sums over the
+// others of their values and tangential momenta (their normal weights are equal, so
+// the face needs the sums only).  A face value is then one interpolation between
+// the two cells across it: each cell's transverse values are formed once per axis
+// and used by both of its faces.
+template <int AX>
+__device__ __forceinline__ i64 fx_interp(const FxParams &P, const FxAt &A, FxMul txp, FxMul txm, int p)
+{
+    const int ax = AX == 0 ? 0 : cx(p), ay = AX == 1 ? 0 : cy(p), az = AX == 2 ? 0 : cz(p);
+    const FxMul tx = ax > 0 ? txp : txm;
+    i64 a = A(p, 0, 0, 0);
+    if (ax) a = fx_lerp(a, A(p, -ax, 0, 0), tx);
+    if (ay) {
+        i64 b = A(p, 0, -ay, 0);
+        if (ax) b = fx_lerp(b, A(p, -ax, -ay, 0), tx);
+        a = fx_lerp(a, b, P.ty);
+    }
+    if (az) {
+        i64 b = A(p, 0, 0, -az);
+        if (ax) b = fx_lerp(b, A(p, -ax, 0, -az), tx);
+        if (ay) {
+            i64 c = A(p, 0, -ay, -az);
+            if (ax) c = fx_lerp(c, A(p, -ax, -ay, -az), tx);
+            b = fx_lerp(b, c, P.ty);
+        }
+        a = fx_lerp(a, b, P.tz);
+    }
+    return a;
+}
+
+constexpr int FXG = 13;
+
+template <int AX>
+__device__ __forceinline__ void fx_cell_values(const FxParams &P, const FxAt &A, FxMul txp, FxMul txm, i64 g[FXG])
+{
+    constexpr int T1 = AX == 0 ? 1 : 0, T2 = AX == 2 ? 1 : 2;
+#pragma unroll
+    for (int s = 0; s < 10; ++s) g[s] = fx_interp<AX>(P, A, txp, txm, flux_pop(AX, s));
+    g[10] = A(0, 0, 0, 0);
+    g[11] = g[12] = 0;
+#pragma unroll
+    for (int p = 1; p < NPOP; ++p) {
+        if (cc(AX, p)) continue;
+        const i64 x = fx_interp<AX>(P, A, txp, txm, p);
+        g[10] += x;
+        if (cc(T1, p)) g[11] += cc(T1, p) > 0 ? x : -x;
+        if (cc(T2, p)) g[12] += cc(T2, p) > 0 ? x : -x;
+    }
+}
+
+// face value of crossing population p between the lower cell's a and the upper cell's b
+template <int AX>
+__device__ __forceinline__ i64 fx_normal(int s, i64 a, i64 b, FxMul mp, FxMul mm)
+{
+    return cc(AX, flux_pop(AX, s)) > 0 ? fx_lerp(a, b, mp) : fx_lerp(b, a, mm);
+}
+
+template <int W>
+constexpr size_t flux_fx_smem_bytes()
+{
+    return sizeof(i64) * size_t((W - 1) * FXG * 34 + (W + 1) * FXG * 32 + W * 10 * 32 + (W - 1) * 10);
+}
+
+// Stages (b)-(e).  A CTA is W warps: warps 1..W-1 one row of 32 cells each (lane =
+// x), marching a chunk of z planes; warp 0 is the halo.  Per plane:
+//   1. every warp forms its cells' transverse values for x and y faces and
+//      publishes them in shared memory (gx, gy); the halo warp those of the rows
+//      below and above the tile and of the columns left and right of it;
+//   2. after a barrier every thread evaluates its +x, +z and +y faces, the halo
+//      warp the -y faces of the first row and the -x faces of the first column; y
+//      fluxes are published (ysh), the -x flux comes from lane-1;
+//   3. after a second barrier the cells are updated.
+// The transverse values and flux of the z faces are carried from plane to plane in
+// registers.
+template <int W, int MINB, int FAX>
+__global__ void __launch_bounds__(32 * W, MINB) flux_fx_kernel(const i64 *__restrict__ fb, const double *f_in,
+                                                               double *f_out, const FxParams P, int kchunk,
+                                                               const int *flag)
+{
+    constexpr int R = W - 1;
+    extern __shared__ __align__(16) i64 sm[];
+    i64(*gx)[FXG][34] = reinterpret_cast<i64(*)[FXG][34]>(sm);
+    i64(*gy)[FXG][32] = reinterpret_cast<i64(*)[FXG][32]>(sm + R * FXG * 34);
+    i64(*ysh)[10][32] = reinterpret_cast<i64(*)[10][32]>(sm + R * FXG * 34 + (R + 2) * FXG * 32);
+    i64(*xsh)[10] = reinterpret_cast<i64(*)[10]>(sm + R * FXG * 34 + (R + 2) * FXG * 32 + (R + 1) * 10 * 32);
+    if (*flag) return;  // a value out of range: the step is redone in FP64
+
+    const int lane = threadIdx.x, wr = threadIdx.y;
+    const int nx = P.nx, ny = P.ny, nz = P.nz, xs = nx + 2;
+    const int c0 = blockIdx.x * 32;            // first column of the tile (0-based cell)
+    const int j0 = blockIdx.y * R;             // first row
+    const int kb = blockIdx.z * kchunk, ke = min(kb + kchunk, nz);
+    if (kb >= ke) return;
+    const long long plane = (long long)ny * P.rs;
+    auto wrap = [](int a, int n) { return a < 0 ? a + n : (a >= n ? a - n : a); };
+    auto wrapc = [&](int a, int n) { a = wrap(a, n); return a < n ? a : n - 1; };  // rows past a ragged last tile: any valid row
+    auto rows = [&](FxAt &A, int j) {
+        A.row[0] = wrap(j - 1, ny) * P.rs;
+        A.row[1] = j * P.rs;
+        A.row[2] = wrap(j + 1, ny) * P.rs;
+    };
+    auto cols = [&](FxAt &A, int c) {  // c = -1 .. nx (ghost columns at nx + 1 and nx)
+        A.col[0] = fx_col(c <= 0 ? nx + 1 : c - 1);
+        A.col[1] = fx_col(c < 0 ? nx + 1 : c);
+        A.col[2] = fx_col(min(c + 1, nx));
+    };
+    auto planes = [&](FxAt &A, int k) {  // k = -1 .. nz
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            int q = k + d - 1;
+            q = wrap(wrap(q, nz), nz);
+            A.pl[d] = fb + q * plane;
+        }
+    };
+    auto at_x = [&](int I, int row) {
+        const int2 m = __ldg(reinterpret_cast<const int2 *>(P.tab) + row * xs + I);
+        return FxMul{m.x, m.y};
+    };
+
+    const int gc = c0 + lane, gj = j0 + wr - 1;
+    const bool cell = wr >= 1 && gc < nx && gj < ny;
+    const int cc1 = min(gc, nx - 1);
+    const FxMul txp = at_x(cc1 + 1, FXT_TXP), txm = at_x(cc1 + 1, FXT_TXM);
+    const int row = wr == 0 ? wrap(j0 - 1, ny) : wrapc(gj, ny);
+    // cell whose x-face values the thread forms: its own; in the halo warp, lane by
+    // lane, the column left of the tile (lanes 0..R-1) and the one right of it
+    const int hs = lane >= R, hr = hs ? lane - R : lane;
+    const int xcol = wr ? min(gc, nx) : (hs ? min(c0 + 32, nx) : c0 - 1);
+    const int xrow = wr ? row : wrapc(j0 + min(hr, R - 1), ny);
+    i64 *gxw = &gx[wr ? wr - 1 : min(hr, R - 1)][0][wr ? lane + 1 : (hs ? 33 : 0)];
+    const bool gxs = wr || lane < 2 * R;
+    // x face the thread evaluates: I (between 1-based columns I and I+1) of tile row
+    // xr; a lane past the last column takes that column's face, a valid one
+    const int I = wr ? min(gc + 1, nx) : c0, xr = wr ? wr - 1 : min(lane, R - 1);
+    FxAt A;
+    i64 gzA[FXG], fz[10];
+
+    // z face between the planes holding a (below) and the one whose values b are given
+    auto z_face = [&](const i64 a[FXG], const i64 b[FXG], i64 v[10]) {
+        i64 m[3];
+#pragma unroll
+        for (int s = 0; s < 10; ++s) v[s] = fx_normal<2>(s, a[s], b[s], P.mz, P.mz);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) m[s] = (a[10 + s] + b[10 + s]) >> 1;
+        fx_face_flux<2, FAX>(P, v, m);
+    };
+    auto y_face = [&](int r, i64 v[10]) {  // between tile rows r - 1 (gy[r]) and r
+        i64 m[3];
+#pragma unroll
+        for (int s = 0; s < 10; ++s) v[s] = fx_normal<1>(s, gy[r][s][lane], gy[r + 1][s][lane], P.my, P.my);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) m[s] = (gy[r][10 + s][lane] + gy[r + 1][10 + s][lane]) >> 1;
+        fx_face_flux<1, FAX>(P, v, m);
+    };
+    // x face I (between 1-based cells I and I+1) of tile row r, gx columns q and q + 1
+    auto x_face = [&](int I, int r, int q, const i64 *row, i64 v[10]) {
+        i64 m[3];
+        const FxMul mp = at_x(I, FXT_MP), mm = at_x(I, FXT_MM);
+#pragma unroll
+        for (int s = 0; s < 10; ++s) v[s] = fx_normal<0>(s, gx[r][s][q], gx[r][s][q + 1], mp, mm);
+        if (P.stretched) {
+            // weight 1/2 + d on the upper cell, except for the rest population (1/2)
+            const FxMul d = at_x(I, FXT_D0);
+            const i64 rest = __ldg(row + fx_col(I)) - __ldg(row + fx_col(I == 0 ? nx + 1 : I - 1));
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const i64 a = gx[r][10 + s][q], b = gx[r][10 + s][q + 1];
+                m[s] = fx_mad(b - a - (s == 0 ? rest : 0), d, (a + b) >> 1);
+            }
+        } else {
+#pragma unroll
+            for (int s = 0; s < 3; ++s) m[s] = (gx[r][10 + s][q] + gx[r][10 + s][q + 1]) >> 1;
+        }
+        if (!P.periodic_x) {
+            // bounce-back on the walls: populations entering the fluid take their opposites' values
+            if (I == 0) {
+                v[0] = v[1]; v[2] = v[5]; v[4] = v[3]; v[6] = v[9]; v[8] = v[7];
+            }
+            if (I == nx) {
+                v[1] = v[0]; v[5] = v[2]; v[3] = v[4]; v[9] = v[6]; v[7] = v[8];
+            }
+        }
+        fx_face_flux<0, FAX>(P, v, m);
+    };
+
+    // plane k's f-bar-plus rows of the tile and f-tilde into L2 (halo warp), two planes ahead of use
+    auto prefetch = [&](int k) {
+        const int q = wrap(k, nz);
+        if (lane < R + 2)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(fb + q * plane + wrapc(wrap(j0 - 1 + lane, ny), ny) * (long long)P.rs + fx_col(c0)),
+                         "r"(unsigned(min(2, (P.pitch_b - c0) >> 4) * NPOP * 16 * 8)));
+        if (k < ke)
+            for (int t = lane; t < NPOP * R * 2; t += 32) {
+                const int p = t / (2 * R), r = (t >> 1) % R;
+                const long long o = p * P.ps + ((long long)k * ny + min(j0 + r, ny - 1)) * P.pitch + min(c0 + 16 * (t & 1), nx - 1);
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(f_in + o));
+            }
+    };
+    // two rounds ahead of the first plane for the z values and flux below it
+    for (int k = kb - 2; k < ke; ++k) {
+        i64 fx[10], dz[10];
+        planes(A, k);
+        if (k >= kb) {
+            // 1. transverse values of the x and y faces
+            i64 g[FXG];
+            rows(A, xrow);
+            cols(A, xcol);
+            fx_cell_values<0>(P, A, txp, txm, g);
+            if (gxs) {
+#pragma unroll
+                for (int s = 0; s < FXG; ++s) gxw[s * 34] = g[s];
+            }
+            cols(A, cc1);
+#pragma unroll 1
+            for (int t = 0; t < (wr ? 1 : 2); ++t) {  // the halo warp: the rows below and above the tile
+                rows(A, t ? wrapc(j0 + R, ny) : row);
+                fx_cell_values<1>(P, A, txp, txm, g);
+                i64 *w = &gy[t ? R + 1 : wr][0][lane];
+#pragma unroll
+                for (int s = 0; s < FXG; ++s) w[s * 32] = g[s];
+            }
+            __syncthreads();
+            // 2. faces
+            x_face(I, xr, I - c0, A.pl[1] + (wr ? row : wrapc(j0 + xr, ny)) * P.rs, fx);
+            if (wr == 0 && lane < R) {
+#pragma unroll
+                for (int s = 0; s < 10; ++s) xsh[lane][s] = fx[s];
+            }
+            i64 v[10];
+            y_face(wr, v);
+#pragma unroll
+            for (int s = 0; s < 10; ++s) ysh[wr][s][lane] = v[s];
+        }
+        if (wr >= 1) {
+            i64 b[FXG], v[10];
+            planes(A, k + 1);
+            rows(A, row);
+            cols(A, cc1);
+            fx_cell_values<2>(P, A, txp, txm, b);
+            if (k >= kb - 1) {
+                z_face(gzA, b, v);
+#pragma unroll
+                for (int s = 0; s < 10; ++s) {
+                    dz[s] = cz(flux_pop(2, s)) > 0 ? fz[s] - v[s] : v[s] - fz[s];
+                    fz[s] = v[s];
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < FXG; ++s) gzA[s] = b[s];
+        } else if (k + 2 < ke + 1) {
+            prefetch(k + 2);
+        }
+        if (k < kb) continue;
+        __syncthreads();
+        // 3. update: f = 4/3 f-bar-plus - 1/3 f - sum of flux differences
+        if (wr >= 1) {
+            planes(A, k);
+            rows(A, row);
+            cols(A, cc1);
+            const FxMul cxm = at_x(cc1 + 1, FXT_CX);
+            const long long c = ((long long)k * ny + min(gj, ny - 1)) * P.pitch + cc1;
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) {
+                const i64 b = A(p, 0, 0, 0);
+                i64 a = fx_madr(b - fx_from_double(f_in[p * P.ps + c]), P.third, b);
+                if (cx(p)) {
+                    const int s = flux_slot(0, p);
+                    i64 l = __shfl_up_sync(0xffffffffu, fx[s], 1);
+                    if (lane == 0) l = xsh[wr - 1][s];
+                    a = fx_madr(cx(p) > 0 ? l - fx[s] : fx[s] - l, cxm, a);
+                }
+                if (cy(p)) {
+                    const int s = flux_slot(1, p);
+                    const i64 l = ysh[wr - 1][s][lane], u = ysh[wr][s][lane];
+                    a = fx_madr(cy(p) > 0 ? l - u : u - l, P.cy, a);
+                }
+                if (cz(p)) a = fx_madr(dz[flux_slot(2, p)], P.cz, a);
+                if (cell) f_out[p * P.ps + c] = fx_to_double(a);
+            }
+        }
+    }
+}
+
+#endif  // __CUDACC__
+
+}  // namespace dg

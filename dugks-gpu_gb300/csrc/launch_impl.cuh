@@ -28,7 +28,7 @@ cudaError_t Kern<T, S>::fbar(const S *f, S *fb, const StepParams<T, S> &P, cudaS
             // FP64 and periodic 16-bit storage: the fused ghost writes cost more issue in
             // stage (a) (FP64 pipe, 16-bit encode) than the separate pass saves
             fbar_kernel<T, S, 0><<<grid, bx, 0, st>>>(f, fb, P, 0);
-            const long long ghosts = 2LL * (P.ny + 2) * (P.nz + 2) + 2LL * P.nx * (P.nz + 2) + 2LL * P.nx * P.ny;
+            const long long ghosts = fb_ghosts(P.nx, P.ny, P.nz);
             fb_ghost_kernel<T, S><<<unsigned((ghosts + 255) / 256), 256, 0, st>>>(fb, P);
         }
     }
