@@ -851,10 +851,9 @@ int stats_form(dg_ctx *h, std::vector<double> &total)
     int rc = ensure_scratch(h, (part + size_t(h->nx) * NSTAT) * sizeof(double));
     if (rc) return rc;
     double *partial = h->scratch, *tot = h->scratch + part;
-    CK(K::stats_partials(static_cast<const S *>(h->f), params_for<T, S>(h, 0), h->hdt(), h->F, partial, nb,
-                                  h->stream),
-       "statistics launch");
-    CK(launch_stats_reduce(partial, nb, h->nx, tot, h->stream), "statistics reduce launch");
+    const StepParams<T, S> P = params_for<T, S>(h, 0);
+    CK(K::stats_partials(static_cast<const S *>(h->f), P, h->hdt(), h->F, partial, nb, h->stream), "statistics launch");
+    CK(launch_stats_reduce(partial, nb, h->nx, tot, K::stats_fp64_cells(P, h->hdt(), h->F), h->stream), "statistics reduce launch");
     total.assign(size_t(h->nx) * NSTAT, 0.0);
     CK(cudaMemcpyAsync(total.data(), tot, total.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
        "statistics copy");
@@ -877,9 +876,9 @@ int accumulate_form(dg_ctx *h)
         h->acc_count = 0;
     }
     double *partial = h->scratch, *tot = h->scratch + part;
-    CK(K::stats_partials(static_cast<const S *>(h->f), params_for<T, S>(h, 0), h->hdt(), h->F, partial, nb, h->stream),
-       "statistics launch");
-    CK(launch_stats_reduce(partial, nb, h->nx, tot, h->stream), "statistics reduce launch");
+    const StepParams<T, S> P = params_for<T, S>(h, 0);
+    CK(K::stats_partials(static_cast<const S *>(h->f), P, h->hdt(), h->F, partial, nb, h->stream), "statistics launch");
+    CK(launch_stats_reduce(partial, nb, h->nx, tot, K::stats_fp64_cells(P, h->hdt(), h->F), h->stream), "statistics reduce launch");
     stats_accumulate_kernel<<<(h->nx * 10 + 127) / 128, 128, 0, h->stream>>>(tot, h->nx, h->acc);
     CK(cudaGetLastError(), "accumulate launch");
     h->acc_count++;
@@ -1451,16 +1450,29 @@ std::string dirname_of(const std::string &p)
 namespace dg {
 __global__ void stats_reduce_kernel(const double *__restrict__ partial, int nblocks, int nx, double *__restrict__ total)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nx) return;
-    double acc[NSTAT];
-    stats_combine_blocks(partial, nblocks, nx, i, acc);
-    for (int s = 0; s < NSTAT; ++s) total[size_t(i) * NSTAT + s] = acc[s];
+    __shared__ double part[kStatsWarps][32];
+    const int lane = threadIdx.x, w = threadIdx.y, nw = blockDim.y;
+    const int i = blockIdx.x * 32 + lane, s = blockIdx.y;
+    const int per = (nblocks + nw - 1) / nw, b0 = w * per, b1 = min(b0 + per, nblocks);
+    if (i < nx && b0 < b1) part[w][lane] = stats_combine(partial, b0, b1, nx, i, s);
+    __syncthreads();
+    if (w || i >= nx) return;
+    double acc = part[0][lane];
+    for (int q = 1; q * per < nblocks; ++q) {
+        const double x = part[q][lane];
+        acc = s < 10 || s == 18 ? acc + x : (s < 14 ? fmin(acc, x) : fmax(acc, x));
+    }
+    total[size_t(i) * NSTAT + s] = acc;
 }
 
-cudaError_t launch_stats_reduce(const double *partial, int nblocks, int nx, double *total, cudaStream_t st)
+// The sums are chains of dependent FP64 additions, about 280 clocks each: over 608
+// blocks one chain per sum takes 90 us, sixteen of them side by side 13 us.  States
+// whose partials come from the FP64 cells (one_chain) keep the single chain, whose
+// rounding recorded outputs hold (kStatsFxCells).
+cudaError_t launch_stats_reduce(const double *partial, int nblocks, int nx, double *total, bool one_chain, cudaStream_t st)
 {
-    stats_reduce_kernel<<<(nx + 127) / 128, 128, 0, st>>>(partial, nblocks, nx, total);
+    stats_reduce_kernel<<<dim3((nx + 31) / 32, NSTAT), dim3(32, one_chain ? 1 : kStatsWarps), 0, st>>>(partial, nblocks, nx,
+                                                                                                        total);
     return cudaGetLastError();
 }
 

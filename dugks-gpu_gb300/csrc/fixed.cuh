@@ -116,16 +116,16 @@ DG_FX i64 fx_from_double(double x)
     return m << e;
 }
 
-// The FP64 value nearest to v / 2^62, any v: one conversion and an exponent
+// The FP64 value nearest to v / 2^s, any v: one conversion and an exponent
 // adjustment (zero has no exponent to adjust).
-DG_FX double fx_to_double(i64 v)
+DG_FX double fx_to_double(i64 v, int s = 62)
 {
 #ifdef __CUDA_ARCH__
     const double d = __ll2double_rn(v);
     const int hi = __double2hiint(d);
-    return __hiloint2double(v ? hi - (62 << 20) : 0, __double2loint(d));
+    return __hiloint2double(v ? hi - (s << 20) : 0, __double2loint(d));
 #else
-    return std::ldexp(double(v), -62);
+    return std::ldexp(double(v), -s);
 #endif
 }
 

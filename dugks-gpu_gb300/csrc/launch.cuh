@@ -59,6 +59,8 @@ struct Kern {
     static cudaError_t soa_to_aos(const S *src, double *dst, const StepParams<T, S> &P, cudaStream_t st);
     static cudaError_t stats_partials(const S *f, const StepParams<T, S> &P, double hdt, const double F[3],
                                       double *partial, int nblocks, cudaStream_t st);
+    // whether stats_partials forms density and velocity of the cells in FP64 (else in fixed point)
+    static bool stats_fp64_cells(const StepParams<T, S> &P, double hdt, const double F[3]);
     static cudaError_t moments_partials(const S *f, const StepParams<T, S> &P, double *partial, int nblocks,
                                         cudaStream_t st);
     // Adjoint of one step (adjoint_kernels.cuh): recomputes f-bar-plus of f_n into fb,
@@ -72,7 +74,7 @@ struct Kern {
     static int flux_kchunk(const StepParams<T, S> &P);
 };
 
-cudaError_t launch_stats_reduce(const double *partial, int nblocks, int nx, double *total, cudaStream_t st);
+cudaError_t launch_stats_reduce(const double *partial, int nblocks, int nx, double *total, bool one_chain, cudaStream_t st);
 
 // one thread waits `limit` polls on an mbarrier that nothing arrives at, then
 // raises *err (kern_fp64.cu); *polled_cycles = SM clock cycles spent waiting

@@ -31,7 +31,7 @@ constexpr int kBlocks = 64;                       // row blocks of the first pas
 constexpr size_t kPartial = size_t(kBlocks) * kMaxNx * dg::NSTAT;
 constexpr size_t kTotal = size_t(kMaxNx) * dg::NSTAT;
 
-// partial[kBlocks][nx][NSTAT] followed by total[nx][NSTAT]; every call writes
+// partial[kBlocks][NSTAT][nx] followed by total[nx][NSTAT]; every call writes
 // every entry it later reads, so nothing has to be cleared between calls.
 static __device__ __align__(256) double g_stats_scratch[kPartial + kTotal];
 
