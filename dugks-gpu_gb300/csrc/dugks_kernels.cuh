@@ -15,9 +15,12 @@
 //   fbar_kernel      stage (a), src/dugks.cu:1131-1196 (calc_fb1), with or without
 //                    the ghost writes
 //   fb_ghost_kernel  the ghost layer of f-bar-plus in a separate pass
-//   flux_kernel      stages (c) (d) (e), src/dugks.cu:715-959 (calc_fx_tri) or the
-//                    central-difference variant 421-649 (calc_fx); every face
-//                    evaluated once, z-marching warp rows
+//   flux_kernel      stages (c) (d) (e) in FP64, src/dugks.cu:715-959 (calc_fx_tri) or
+//                    the central-difference variant 421-649 (calc_fx); every face
+//                    evaluated once, z-marching warp rows (FP64 states near unit
+//                    density: fixed_kernels.cuh)
+//   flux_tma_kernel  the same in the float forms, trilinear reconstruction (central
+//                    differences: flux_shared.cuh)
 //   macro_kernel     src/dugks.cu:1021-1064 (calc_macro)
 //
 // Template parameters: T is the arithmetic type, S the storage type of f and
@@ -1478,17 +1481,10 @@ __device__ __forceinline__ void face_fluxes(const StepParams<T, S> &P, const RD 
     T v[NPOP];
     if constexpr (RECON == 0 && Fp64Form<T>::value)
         face_tri_cw<T, S, AX>(P, R, i, j, k, v);
-    else if constexpr (RECON == 0 && std::is_same<T, float>::value)
-        face_tri_x2<S, AX>(P, R, i, j, k, v);  // packed lerps: FP32, FP16, BF16
     else if constexpr (RECON == 0)
-        face_tri<T, S, AX>(P, R, i, j, k, v);
+        face_tri_x2<S, AX>(P, R, i, j, k, v);  // packed lerps: FP32, FP16, BF16
     else
-        face_grad<T, S, AX>(P, R, i, j, k, v);
-    if constexpr (RECON != 0 && Codec<T, S>::deviation) {
-        // the face values less their rest state, as the interpolating forms give them
-#pragma unroll
-        for (int p = 0; p < NPOP; ++p) v[p] -= P.codec.w[p];
-    }
+        face_grad<T, S, AX>(P, R, i, j, k, v);  // FP64 (float forms: flux_shared.cuh)
     if (AX == 0 && !P.periodic_x) bounce_back(v, i == 0, i == P.nx);
     face_flux<T, S, AX, FF>(P, v, out, FF ? face_field<T, S, AX>(P, i, j, k) : T(0));
 }
@@ -1657,7 +1653,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int lim
     return false;
 }
 
-template <class T, class S, int W, int RECON, int MINB, bool FF>
+template <class T, class S, int W, int MINB, bool FF>
 __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_constant__ CUtensorMap tmap,
                                                                  const S *f_in, S *f_out,
                                                                  const StepParams<T, S> P, int kchunk)
@@ -1763,7 +1759,7 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_con
         wall_ghosts(kb);
         __syncthreads();
     }
-    if (wr >= 1) face_fluxes<T, S, 2, RECON, FF>(P, R, ci, cj, kb - 1, fzd);
+    if (wr >= 1) face_fluxes<T, S, 2, 0, FF>(P, R, ci, cj, kb - 1, fzd);
     for (int k = kb; k < ke; ++k) {
         wait(k + 1);
         if (wall_tile) {
@@ -1771,9 +1767,9 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_con
             __syncthreads();
         }
         if (wr >= 1) {
-            face_fluxes<T, S, 0, RECON, FF>(P, R, ci, cj, k, fx);
-            face_fluxes<T, S, 1, RECON, FF>(P, R, ci, cj, k, fy);
-            face_fluxes<T, S, 2, RECON, FF>(P, R, ci, cj, k, fzu);
+            face_fluxes<T, S, 0, 0, FF>(P, R, ci, cj, k, fx);
+            face_fluxes<T, S, 1, 0, FF>(P, R, ci, cj, k, fy);
+            face_fluxes<T, S, 2, 0, FF>(P, R, ci, cj, k, fzu);
 #pragma unroll
             for (int s = 0; s < 10; ++s) ysh[buf][wr][s][lane] = fy[s];
             // the cell's f-tilde, loaded before the barrier so its latency overlaps the exchange
@@ -1783,12 +1779,12 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_con
                 for (int p = 0; p < NPOP; ++p) fo[p] = P.codec.raw(f_in, p * P.ps + c);
             }
         } else {
-            face_fluxes<T, S, 1, RECON, FF>(P, R, ci, j0 - 1, k, fy);
+            face_fluxes<T, S, 1, 0, FF>(P, R, ci, j0 - 1, k, fy);
 #pragma unroll
             for (int s = 0; s < 10; ++s) ysh[buf][0][s][lane] = fy[s];
             if (hx) {
                 T hxf[10];
-                face_fluxes<T, S, 0, RECON, FF>(P, R, i0 - 1, hj, k, hxf);
+                face_fluxes<T, S, 0, 0, FF>(P, R, i0 - 1, hj, k, hxf);
 #pragma unroll
                 for (int s = 0; s < 10; ++s) xsh[buf][lane + 1][s] = hxf[s];
             }

@@ -1145,7 +1145,7 @@ int make_tmap_form(dg_ctx *h)
     using K = Kern<T, S>;
     if (!K::uses_tma()) return DG_OK;
     const S *fb = static_cast<const S *>(h->fb);
-    int r = K::make_tmap(fb, h->nx, h->ny, h->nz, h->pitch_b, h->ps_b, TileCfg<T, S>::W + 1, &h->tmap);
+    int r = K::make_tmap(fb, h->nx, h->ny, h->nz, h->pitch_b, h->ps_b, K::flux_box_rows(h->recon), &h->tmap);
     if (!r) r = K::make_tmap(fb, h->nx, h->ny, h->nz, h->pitch_b, h->ps_b, AdjCfg<T, S>::W + 2, &h->tmap_adj);
     if (r) return h->fail(DG_ERR_CUDA, "cuTensorMapEncodeTiled failed for the f-bar-plus tensor map (" + std::to_string(r) + ")");
     h->have_tmap = true;

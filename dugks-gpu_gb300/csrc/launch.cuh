@@ -31,6 +31,19 @@ struct TileCfg<double, double> {
     static constexpr bool TMA = false;
 };
 
+// CTA of flux_sh_kernel (float forms, gradient reconstruction).  FP32 by (W, CTAs per SM),
+// ms per flux launch of a 256 x 128 x 128 channel, trilinear values in place of the
+// derivatives: (5, 3) 0.243, (7, 2) 0.265, (8, 2) 0.273, (4, 4) 0.29, (16, 1) 0.32; FP16:
+// (8, 2) 0.310, (6, 2) 0.32, (7, 2) 0.34, (16, 1) 0.35, (7, 3) 0.41.
+template <class S>
+struct GradCfg {
+    static constexpr int W = 8, MINB = 2;
+};
+template <>
+struct GradCfg<float> {
+    static constexpr int W = 5, MINB = 3;
+};
+
 // tile of the fused adjoint face kernel (TMA forms): W rows of 32 cells, box W+2 rows
 template <class T, class S>
 struct AdjCfg {
@@ -50,7 +63,7 @@ struct Kern {
     static bool uses_tma() { return TileCfg<T, S>::TMA; }
     // 4-D tensor map (x, y, z, population) over the ghosted f-bar-plus array,
     // box of TmaTile::BXT columns x box_rows rows x 1 plane x 19 populations
-    // (forward flux kernel: TileCfg::W + 1 rows; adjoint faces: AdjCfg::W + 2)
+    // (forward flux kernel: flux_box_rows; adjoint faces: AdjCfg::W + 2)
     static int make_tmap(const S *fb, int nx, int ny, int nz, int pitch_b, long long ps_b, int box_rows,
                          CUtensorMap *out);
     static cudaError_t macro(const S *f, const StepParams<T, S> &P, double hdt, const double F[3], double *rho,
@@ -71,7 +84,7 @@ struct Kern {
     static cudaError_t adjoint(const S *f_n, S *fb, const S *lam_next, S *lam_out, T *lamv,
                                const StepParams<T, S> &P, double *dphi, const CUtensorMap *tmap_adj,
                                cudaStream_t st);
-    static int flux_kchunk(const StepParams<T, S> &P);
+    static constexpr int flux_box_rows(int recon) { return (recon == 1 ? GradCfg<S>::W : TileCfg<T, S>::W) + 1; }
 };
 
 cudaError_t launch_stats_reduce(const double *partial, int nblocks, int nx, double *total, bool one_chain, cudaStream_t st);

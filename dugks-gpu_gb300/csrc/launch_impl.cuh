@@ -4,6 +4,7 @@
 #include <cmath>
 #include <type_traits>
 #include <cudaTypedefs.h>
+#include "flux_shared.cuh"
 #include "launch.cuh"
 
 namespace dg {
@@ -73,59 +74,69 @@ static int device_sms()
     return sms;
 }
 
-template <class T, class S>
-int Kern<T, S>::flux_kchunk(const StepParams<T, S> &P)
+// z chunk of a flux kernel whose CTAs are tiles of 32 x (W-1) cells
+template <class T, class S, class K>
+static int flux_kchunk(const StepParams<T, S> &P, K kern, int W, size_t smem)
 {
-    constexpr int W = TileCfg<T, S>::W, MB = TileCfg<T, S>::MINB;
-    const int sms = device_sms();
     int occ = 1;
-    if constexpr (TileCfg<T, S>::TMA)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, flux_tma_kernel<T, S, W, 0, MB, false>, 32 * W,
-                                                      flux_tma_smem_bytes<T, S, W>());
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, flux_kernel<T, S, W, 0, MB, false>, 32 * W, 0);
-    occ = std::max(occ, 1);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * W, smem);
     const long long cols = (long long)((P.nx + 31) / 32) * ((P.ny + W - 2) / (W - 1));
-    return choose_kchunk(P.nz, cols, (long long)sms * occ);
+    return choose_kchunk(P.nz, cols, (long long)device_sms() * std::max(occ, 1));
+}
+
+// one launch of a TMA-fed flux kernel of W warps
+template <int W, class T, class S, class K>
+static cudaError_t flux_tma_launch(K kern, size_t smem, bool *attr_set, const S *f_in, S *f_out,
+                                   const StepParams<T, S> &P, const CUtensorMap *tmap, cudaStream_t st)
+{
+    if (!*attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e != cudaSuccess) return e;
+        *attr_set = true;
+    }
+    if (!tmap) return cudaErrorInvalidValue;
+    const int kc = flux_kchunk(P, kern, W, smem);
+    const dim3 grid((P.nx + 31) / 32, (P.ny + W - 2) / (W - 1), (P.nz + kc - 1) / kc);
+    kern<<<grid, dim3(32, W), smem, st>>>(*tmap, f_in, f_out, P, kc);
+    return cudaGetLastError();
 }
 
 // one launch of the flux kernel variant <RECON, FF>
 template <class T, class S, int RECON, bool FF>
 static cudaError_t flux_launch(const S *fb, const S *f_in, S *f_out, const StepParams<T, S> &P,
-                               const CUtensorMap *tmap, int kchunk, cudaStream_t st)
+                               const CUtensorMap *tmap, cudaStream_t st)
 {
-    constexpr int W = TileCfg<T, S>::W, MB = TileCfg<T, S>::MINB;
-    dim3 grid((P.nx + 31) / 32, (P.ny + W - 2) / (W - 1), (P.nz + kchunk - 1) / kchunk);
-    dim3 block(32, W);
     if constexpr (TileCfg<T, S>::TMA) {
-        auto kern = flux_tma_kernel<T, S, W, RECON, MB, FF>;
-        const int bytes = int(flux_tma_smem_bytes<T, S, W>());
         static bool attr_set = false;
-        if (!attr_set) {
-            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-            if (e != cudaSuccess) return e;
-            attr_set = true;
+        if constexpr (RECON == 1) {
+            constexpr int W = GradCfg<S>::W;
+            return flux_tma_launch<W>(flux_sh_kernel<S, W, GradCfg<S>::MINB, FF>, flux_sh_smem_bytes<S, W>(), &attr_set,
+                                      f_in, f_out, P, tmap, st);
+        } else {
+            constexpr int W = TileCfg<T, S>::W;
+            return flux_tma_launch<W>(flux_tma_kernel<T, S, W, TileCfg<T, S>::MINB, FF>, flux_tma_smem_bytes<T, S, W>(),
+                                      &attr_set, f_in, f_out, P, tmap, st);
         }
-        if (!tmap) return cudaErrorInvalidValue;
-        kern<<<grid, block, bytes, st>>>(*tmap, f_in, f_out, P, kchunk);
     } else {
-        (void)tmap;
-        flux_kernel<T, S, W, RECON, MB, FF><<<grid, block, 0, st>>>(fb, f_in, f_out, P, kchunk);
+        constexpr int W = TileCfg<T, S>::W, MB = TileCfg<T, S>::MINB;
+        auto kern = flux_kernel<T, S, W, RECON, MB, FF>;
+        const int kc = flux_kchunk(P, kern, W, 0);
+        const dim3 grid((P.nx + 31) / 32, (P.ny + W - 2) / (W - 1), (P.nz + kc - 1) / kc);
+        kern<<<grid, dim3(32, W), 0, st>>>(fb, f_in, f_out, P, kc);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
 }
 
 template <class T, class S>
 cudaError_t Kern<T, S>::flux(const S *fb, const S *f_in, S *f_out, const StepParams<T, S> &P, int recon,
                              const CUtensorMap *tmap, cudaStream_t st)
 {
-    const int kchunk = flux_kchunk(P);
     const bool ff = P.ffield != nullptr;
     if (recon == 1)
-        return ff ? flux_launch<T, S, 1, true>(fb, f_in, f_out, P, tmap, kchunk, st)
-                  : flux_launch<T, S, 1, false>(fb, f_in, f_out, P, tmap, kchunk, st);
-    return ff ? flux_launch<T, S, 0, true>(fb, f_in, f_out, P, tmap, kchunk, st)
-              : flux_launch<T, S, 0, false>(fb, f_in, f_out, P, tmap, kchunk, st);
+        return ff ? flux_launch<T, S, 1, true>(fb, f_in, f_out, P, tmap, st)
+                  : flux_launch<T, S, 1, false>(fb, f_in, f_out, P, tmap, st);
+    return ff ? flux_launch<T, S, 0, true>(fb, f_in, f_out, P, tmap, st)
+              : flux_launch<T, S, 0, false>(fb, f_in, f_out, P, tmap, st);
 }
 
 template <class T, class S>
