@@ -8,12 +8,12 @@
 //                   extend_fb_x_wall / extend_fb_y kernels and the MPI z exchange
 //                   (src/dugks.cu:348-377, src/parallel.cu:185-234): written by
 //                   fb_ghost_kernel (FP64; 16-bit forms with periodic x), by
-//                   fbar_kernel itself (FP32; 16-bit forms between walls: the y / z
+//                   fbar_float_kernel itself (FP32; 16-bit forms between walls: the y / z
 //                   images, the wall columns formed by the flux kernel in shared memory).
 //
 // Kernels:
-//   fbar_kernel      stage (a), src/dugks.cu:1131-1196 (calc_fb1), with or without
-//                    the ghost writes
+//   fbar_kernel      stage (a), src/dugks.cu:1131-1196 (calc_fb1), in FP64
+//   fbar_float_kernel  the same in the float forms, with or without the ghost writes
 //   fb_ghost_kernel  the ghost layer of f-bar-plus in a separate pass
 //   flux_kernel      stages (c) (d) (e) in FP64, src/dugks.cu:715-959 (calc_fx_tri) or
 //                    the central-difference variant 421-649 (calc_fx); every face
@@ -388,21 +388,6 @@ __device__ __forceinline__ void copy_images(S *fb, long long ps_b, int I, int J,
     }
 }
 
-// Stage (a) for one cell.  GHOST = 0: the interior of f-bar-plus only
-// (fb_ghost_kernel fills the ghost layer).  GHOST = 2: the interior and its
-// periodic images in y and z only (the 16-bit forms between walls, whose flux
-// kernel forms the wall ghost columns itself).  GHOST = 1: the ghost layer is
-// written by the threads that hold its sources, in the same launch -- a cell
-// of the first/last row or plane also writes its periodic images in y and z
-// (src/dugks.cu:1256-1273, src/parallel.cu:192-199), the first/last cell of a
-// row writes the periodic x copy (src/dugks.cu:1212-1229), and between walls
-// each warp next to a wall forms the extrapolation g0 = q0 fb(1) + (1-q0) fb(2),
-// g_{nx+1} = q1 fb(nx) + (1-q1) fb(nx-1) of the stored values (src/dugks.cu:1234-1251;
-// stretched mesh src/fortran/channel/src/dugks.cuf:365-374), one population per
-// lane.  Warps away from walls, x ends and boundary rows/planes take the
-// plain path.  xoff shifts the cells by one thread when nx = 1 (mod 32) so
-// that cells nx-1 and nx share a warp.  The result equals the reference's
-// x -> y -> z fill order.
 // Stage (a) with a force along axis A only (FP64 form): f-bar-plus_p =
 // (B + K_p) feq_p + bw1 f_p with K_p in {0, +-Kb}, fused per opposite pair
 // (p, q): feq_{p,q} = w r (t +- eu), t = base + eu^2/2.  A pair with c_A = 0
@@ -444,38 +429,10 @@ __device__ __forceinline__ void fbar_one_axis(T r, T u, T vv, T w, T B, T Kb, T 
     pair(16, 17, w3 - v3, 2);
 }
 
-// One block of the grid, block (bx, j, k) of bdim threads; tid: the thread within it.
-template <class T, class S, int GHOST>
-__device__ __forceinline__ void fbar_block(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> &P,
-                                           int xoff, int tid, int bx, int bdim, int j, int k)
+// Stage (a) of one cell (column ic, row j, plane k): f-bar-plus ob from f-tilde v.
+template <class T, class S>
+__device__ __forceinline__ void fbar_cell(const StepParams<T, S> &P, int ic, int j, int k, const T v[NPOP], T ob[NPOP])
 {
-    const int i = bx * bdim + tid - xoff;
-    const int nx = P.nx, ny = P.ny, nz = P.nz;
-    const bool in = i >= 0 && i < nx;
-    const int wbase = bx * bdim + (tid & ~31) - xoff;  // cell of lane 0
-    const bool wall_warp =
-        GHOST == 1 && !P.periodic_x && ((wbase <= 1 && wbase + 31 >= 0) || (wbase <= nx - 1 && wbase + 31 >= nx - 2));
-    if (!in && !wall_warp) return;
-    const int ic = in ? i : (i < 0 ? 0 : nx - 1);  // lanes past the row read a valid cell and store nothing
-    const long long c = ((long long)k * ny + j) * P.pitch + ic;
-    const long long cb = ((long long)(k + 1) * (ny + 2) + (j + 1)) * P.pitch_b + ic + 1;
-
-    T v[NPOP];
-    if constexpr (Codec<T, S>::deviation) {
-        // decoded two populations at a time (pairs 2m-1, 2m)
-        v[0] = P.codec.load_nc(f, c, 0);
-#pragma unroll
-        for (int m = 1; m <= 9; ++m) {
-            const int p = 2 * m - 1, q = 2 * m;
-            const float2 x = P.codec.dec2(p, q, make_float2(P.codec.raw_nc(f, p * P.ps + c), P.codec.raw_nc(f, q * P.ps + c)));
-            v[p] = x.x;
-            v[q] = x.y;
-        }
-    } else {
-#pragma unroll
-        for (int p = 0; p < NPOP; ++p) v[p] = P.codec.load_nc(f, p * P.ps + c, p);
-    }
-
     // the 16-bit forms' moments two at a time; the FP32 form keeps the pair sums, whose
     // density, as the target of the moment correction below, measured a ten times smaller
     // mass drift (2e-7 against 2e-6 over 50,000 turbulent-channel steps)
@@ -511,8 +468,6 @@ __device__ __forceinline__ void fbar_block(const S *__restrict__ f, S *__restric
         B = fma(-P.bw0x3, fma(Fx, u, fma(Fy, vv, Fz * w)), P.bw2);
     }
 
-    const unsigned hc = P.codec.cell_hash(cb);
-    T ob[NPOP];
     if (one_axis) {
         if (P.fax == 0)
             fbar_one_axis<T, 0>(r, u, vv, w, B, P.Kba, P.bw1, v, ob);
@@ -590,91 +545,173 @@ __device__ __forceinline__ void fbar_block(const S *__restrict__ f, S *__restric
         const T c2 = (ob[9] + ob[10]) + (ob[11] + ob[12]), d = (ob[13] + ob[14]) + (ob[15] + ob[16]);
         ob[0] = r - ((((a + b) + (c2 + d)) + ob[17]) + ob[18]);
     }
+}
 
-    // periodic images of this row and plane (uniform over the warp): J = 1 -> ny+1,
-    // J = ny -> 0, likewise K, and the corner image
-    const long long rstep = P.pitch_b, pstep = (long long)(ny + 2) * P.pitch_b;
-    const long long dj = j == 0 ? ny * rstep : (j == ny - 1 ? -(long long)ny * rstep : 0);
-    const long long dk = k == 0 ? nz * pstep : (k == nz - 1 ? -(long long)nz * pstep : 0);
-    const bool small = ny == 1 || nz == 1;  // two images along one axis: copied at the end
-    const bool img = !small && (dj != 0 || dk != 0);
-    const bool xend = wbase <= 0 || wbase + 31 >= nx - 1;
-    S enc[NPOP];  // the stored values (16-bit forms: deviations of the pairs formed two at a time)
-    if constexpr (Codec<T, S>::deviation) {
-        enc[0] = P.codec.encode_h(0, ob[0], hc);
+// Stage (a) in FP64: the interior of f-bar-plus (fb_ghost_kernel fills the ghost
+// layer).  One block of the grid, block (bx, j, k) of bdim threads; tid: the thread
+// within it.
+template <class T, class S>
+__device__ __forceinline__ void fbar_block(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> &P,
+                                           int tid, int bx, int bdim, int j, int k)
+{
+    const int i = bx * bdim + tid;
+    if (i >= P.nx) return;
+    const long long c = ((long long)k * P.ny + j) * P.pitch + i;
+    const long long cb = ((long long)(k + 1) * (P.ny + 2) + (j + 1)) * P.pitch_b + i + 1;
+    T v[NPOP], ob[NPOP];
 #pragma unroll
-        for (int m = 1; m <= 9; ++m) {
-            const int p = 2 * m - 1, q = 2 * m;
-            const float2 d = P.codec.dev2(p, q, make_float2(ob[p], ob[q]));
-            enc[p] = P.codec.encode_dh(p, d.x, hc);
-            enc[q] = P.codec.encode_dh(q, d.y, hc);
+    for (int p = 0; p < NPOP; ++p) v[p] = P.codec.load_nc(f, p * P.ps + c, p);
+    fbar_cell(P, i, j, k, v, ob);
+#pragma unroll
+    for (int p = 0; p < NPOP; ++p) fb[p * P.ps_b + cb] = P.codec.encode_h(p, ob[p], 0u);
+}
+
+template <class T, class S>
+__global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> P)
+{
+    fbar_block<T, S>(f, fb, P, threadIdx.x, blockIdx.x, blockDim.x, blockIdx.y, blockIdx.z);
+}
+
+// Stage (a) of the float forms, one thread per cell.  GHOST = 0: the interior of
+// f-bar-plus only.  GHOST = 2: the interior and its periodic images in y and z (the
+// 16-bit forms between walls, whose flux kernel forms the wall ghost columns itself).
+// GHOST = 1 (FP32): the ghost layer is written by the threads that hold its sources --
+// a cell of the first/last row or plane also writes its periodic images in y and z
+// (src/dugks.cu:1256-1273, src/parallel.cu:192-199), the first/last cell of a row the
+// periodic x copy (src/dugks.cu:1212-1229), and between walls the warp next to a wall
+// forms the extrapolation g0 = q0 fb(1) + (1-q0) fb(2), g_{nx+1} = q1 fb(nx) +
+// (1-q1) fb(nx-1) of the stored values (src/dugks.cu:1234-1251; stretched mesh
+// src/fortran/channel/src/dugks.cuf:365-374), one population per lane.  xoff shifts the
+// cells by one thread when nx = 1 (mod 32) so that cells nx-1 and nx share a warp.  The
+// result equals the reference's x -> y -> z fill order.
+// Every cell takes the same 19 stores first; what the ghosts need comes behind them, so
+// that warps away from walls and boundary rows leave early and the others add 19
+// shared-memory stores (743 -> 588 instructions per cell in FP32); a block takes `rows`
+// rows and loads the next one while it computes.  Stage (a) of the 256 x 128 x 128
+// channel, FP32: 0.152 -> 0.143 ms (4.4 TB/s; bound by the latency of 38 population
+// streams: fewer registers, larger blocks and two cells per thread were no faster).
+template <class S, int GHOST>
+__global__ void __launch_bounds__(128) fbar_float_kernel(const S *__restrict__ f, S *__restrict__ fb,
+                                                         const StepParams<float, S> P, int xoff, int rows)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x - xoff;
+    const int k = blockIdx.z, nx = P.nx, ny = P.ny, nz = P.nz;
+    const int j0 = blockIdx.y * rows, j1 = min(j0 + rows, ny);
+    const bool in = i >= 0 && i < nx;
+    const int w0 = i - (threadIdx.x & 31);  // cell of lane 0
+    const bool lo = GHOST == 1 && !P.periodic_x && w0 <= 0, hi = GHOST == 1 && !P.periodic_x && w0 <= nx - 1 && w0 + 31 >= nx - 1;
+    if (!in && !lo && !hi) return;
+    const int ic = in ? i : (i < 0 ? 0 : nx - 1);  // lanes past the row read a valid cell and store nothing
+    const S *src = f + ((long long)k * ny + j0) * P.pitch;
+    S nv[NPOP];  // f-tilde as stored, of the next row
+#pragma unroll
+    for (int p = 0; p < NPOP; ++p) nv[p] = __ldg(src + p * P.ps + ic);
+#pragma unroll 1
+    for (int j = j0; j < j1; ++j) {
+        float v[NPOP], ob[NPOP];
+        if constexpr (Codec<float, S>::deviation) {
+            // decoded two populations at a time (pairs 2m-1, 2m)
+            v[0] = P.codec.dec(0, float(nv[0]));
+#pragma unroll
+            for (int m = 1; m <= 9; ++m) {
+                const int p = 2 * m - 1, q = 2 * m;
+                const float2 x = P.codec.dec2(p, q, make_float2(float(nv[p]), float(nv[q])));
+                v[p] = x.x;
+                v[q] = x.y;
+            }
+        } else {
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) v[p] = nv[p];
         }
-    } else {
+        src += P.pitch;
+        if (j + 1 < j1) {
 #pragma unroll
-        for (int p = 0; p < NPOP; ++p) enc[p] = P.codec.encode_h(p, ob[p], hc);
-    }
-    if (GHOST == 0 || (!wall_warp && !img && !small && !(P.periodic_x && xend))) {
+            for (int p = 0; p < NPOP; ++p) nv[p] = __ldg(src + p * P.ps + ic);
+        }
+        fbar_cell(P, ic, j, k, v, ob);
+        const long long rowb = ((long long)(k + 1) * (ny + 2) + (j + 1)) * P.pitch_b;
+        S *row = fb + rowb;
+        const unsigned hc = P.codec.cell_hash(rowb + ic + 1);
+        S enc[NPOP];  // the stored values (16-bit forms: deviations of the pairs formed two at a time)
+        if constexpr (Codec<float, S>::deviation) {
+            enc[0] = P.codec.encode_h(0, ob[0], hc);
 #pragma unroll
-        for (int p = 0; p < NPOP; ++p) fb[p * P.ps_b + cb] = enc[p];
-        return;
-    }
-    __shared__ T wv[4][4][NPOP];  // per warp: values of cells 1, 2, nx, nx-1 (blocks of at most 128 threads)
-    auto put = [&](S *q, S val) {  // a value and its images
-        q[0] = val;
-        if (img) {
+            for (int m = 1; m <= 9; ++m) {
+                const int p = 2 * m - 1, q = 2 * m;
+                const float2 d = P.codec.dev2(p, q, make_float2(ob[p], ob[q]));
+                enc[p] = P.codec.encode_dh(p, d.x, hc);
+                enc[q] = P.codec.encode_dh(q, d.y, hc);
+            }
+        } else {
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) enc[p] = P.codec.encode_h(p, ob[p], hc);
+        }
+        if (in) {
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) row[p * P.ps_b + ic + 1] = enc[p];
+        }
+        if (GHOST == 0) continue;
+
+        // periodic images of this row and plane (uniform over the block): J = 1 -> ny+1,
+        // J = ny -> 0, likewise K, and the corner image
+        const long long rstep = P.pitch_b, pstep = (long long)(ny + 2) * P.pitch_b;
+        const long long dj = j == 0 ? ny * rstep : (j == ny - 1 ? -(long long)ny * rstep : 0);
+        const long long dk = k == 0 ? nz * pstep : (k == nz - 1 ? -(long long)nz * pstep : 0);
+        const bool small = ny == 1 || nz == 1;  // two images along one axis: copied at the end
+        const bool img = !small && (dj != 0 || dk != 0);
+        auto images = [&](S *q, S val) {
             if (dj) q[dj] = val;
             if (dk) q[dk] = val;
             if (dj && dk) q[dj + dk] = val;
-        }
-    };
-    const long long rowb = cb - (ic + 1);  // stored column 0 of this row and plane
-    const int wl = tid >> 5;
+        };
+        if (img && in) {
 #pragma unroll
-    for (int p = 0; p < NPOP; ++p) {
-        const T out = ob[p];
-        S *pl = fb + p * P.ps_b + rowb;
-        const S e = enc[p];
-        if (in) {
-            put(pl + ic + 1, e);
-            if (P.periodic_x) {
-                if (ic == 0) put(pl + nx + 1, e);
-                if (ic == nx - 1) put(pl, e);
+            for (int p = 0; p < NPOP; ++p) images(row + p * P.ps_b + ic + 1, enc[p]);
+        }
+        if (GHOST == 1 && P.periodic_x && in && (ic == 0 || ic == nx - 1)) {
+            S *g = row + (ic == 0 ? nx + 1 : 0);
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) {
+                g[p * P.ps_b] = enc[p];
+                if (img) images(g + p * P.ps_b, enc[p]);
             }
         }
-        if (wall_warp) {
-            // the stored values of the two cells next to each wall
-            const T mine = Codec<T, S>::deviation ? P.codec.dec(p, T(e)) : out;
-            if (in && ic == 0) wv[wl][0][p] = mine;
-            if (in && ic == 1) wv[wl][1][p] = mine;
-            if (in && ic == nx - 1) wv[wl][2][p] = mine;
-            if (in && ic == nx - 2) wv[wl][3][p] = mine;
+        if (lo || hi) {
+            __shared__ float wv[4][4][NPOP];  // per warp: values of cells 1, 2, nx, nx-1
+            float(*mine)[NPOP] = wv[threadIdx.x >> 5];
+            if (lo && in && ic < 2) {
+#pragma unroll
+                for (int p = 0; p < NPOP; ++p) mine[ic][p] = ob[p];
+            }
+            if (hi && in && ic >= nx - 2) {
+#pragma unroll
+                for (int p = 0; p < NPOP; ++p) mine[2 + nx - 1 - ic][p] = ob[p];
+            }
+            __syncwarp();
+            const int p = threadIdx.x & 31;
+            if (p < NPOP) {
+                S *g = row + p * P.ps_b;
+                if (lo) {
+                    const S e = P.codec.encode_h(p, P.q0 * mine[0][p] + (1.0f - P.q0) * mine[1][p], hc);
+                    g[0] = e;
+                    if (img) images(g, e);
+                }
+                if (hi) {
+                    const S e = P.codec.encode_h(p, P.q1 * mine[2][p] + (1.0f - P.q1) * mine[3][p], hc);
+                    g[nx + 1] = e;
+                    if (img) images(g + nx + 1, e);
+                }
+            }
+            __syncwarp();
+        }
+        if (small && in) {
+            copy_images(fb, P.ps_b, ic + 1, j + 1, k + 1, ny, nz, P.pitch_b);
+            if (GHOST == 1 && ic == 0)
+                copy_images(fb, P.ps_b, P.periodic_x ? nx + 1 : 0, j + 1, k + 1, ny, nz, P.pitch_b);
+            if (GHOST == 1 && ic == nx - 1)
+                copy_images(fb, P.ps_b, P.periodic_x ? 0 : nx + 1, j + 1, k + 1, ny, nz, P.pitch_b);
         }
     }
-    if (wall_warp) {
-        __syncwarp();
-        const int lane = tid & 31;
-        if (lane < NPOP) {
-            const int p = lane;
-            S *pl = fb + p * P.ps_b + rowb;
-            if (wbase <= 0) put(pl, P.codec.encode_h(p, P.q0 * wv[wl][0][p] + (T(1) - P.q0) * wv[wl][1][p], hc));
-            if (wbase + 31 >= nx - 1)
-                put(pl + nx + 1, P.codec.encode_h(p, P.q1 * wv[wl][2][p] + (T(1) - P.q1) * wv[wl][3][p], hc));
-        }
-        __syncwarp();
-    }
-    if (small && in) {
-        copy_images(fb, P.ps_b, ic + 1, j + 1, k + 1, ny, nz, P.pitch_b);
-        if (GHOST == 1 && ic == 0) copy_images(fb, P.ps_b, P.periodic_x ? nx + 1 : 0, j + 1, k + 1, ny, nz, P.pitch_b);
-        if (GHOST == 1 && ic == nx - 1)
-            copy_images(fb, P.ps_b, P.periodic_x ? 0 : nx + 1, j + 1, k + 1, ny, nz, P.pitch_b);
-    }
-}
-
-template <class T, class S, int GHOST>
-__global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> P,
-                                                   int xoff)
-{
-    fbar_block<T, S, GHOST>(f, fb, P, xoff, threadIdx.x, blockIdx.x, blockDim.x, blockIdx.y, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------

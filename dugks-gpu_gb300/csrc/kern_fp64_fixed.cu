@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(32 * W, MINB) fp64_redo_kernel(const double *f
     const long long blocks = (long long)gx * P.ny * P.nz;
     for (long long b = blockIdx.x; b < blocks; b += nb) {
         const long long r = b / gx;
-        fbar_block<double, double, 0>(f_in, fb, P, 0, tid, int(b - r * gx), 32 * W, int(r % P.ny), int(r / P.ny));
+        fbar_block<double, double>(f_in, fb, P, tid, int(b - r * gx), 32 * W, int(r % P.ny), int(r / P.ny));
     }
     grid.sync();
     const long long ghosts = fb_ghosts(P.nx, P.ny, P.nz);

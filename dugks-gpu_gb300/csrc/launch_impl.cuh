@@ -12,27 +12,35 @@ namespace dg {
 template <class T, class S>
 cudaError_t Kern<T, S>::fbar(const S *f, S *fb, const StepParams<T, S> &P, cudaStream_t st)
 {
+    // 1-D blocks of whole warps over a row, at most 128 threads; cells nx-1 and nx must share a
+    // warp for FP32's wall extrapolation: shift by one when nx = 1 (mod 32)
+    const int xoff = (std::is_same<S, float>::value && !P.periodic_x && P.nx % 32 == 1) ? 1 : 0;
+    const int bx = P.nx + xoff >= 128 ? 128 : ((P.nx + xoff + 31) / 32) * 32;
+    // four rows per block where that leaves two waves of blocks (one row: 0.143 -> 0.164 ms on the
+    // 256 x 128 x 128 channel in FP32), one row on small grids, which need the blocks
+    const long long blocks = (long long)((P.nx + xoff + bx - 1) / bx) * P.ny * P.nz;
+    const int rows = blocks * bx >= 4LL * 2 * 152 * 1024 ? 4 : 1;
+    const dim3 grid((P.nx + xoff + bx - 1) / bx, (P.ny + rows - 1) / rows, P.nz);
+    bool ghosts = false;
     if constexpr (std::is_same<S, float>::value) {
-        // FP32: stage (a) writes the ghost layer itself (one launch); cells nx-1 and nx
-        // must share a warp for the wall extrapolation: shift by one when nx = 1 (mod 32)
-        const int xoff = (!P.periodic_x && P.nx % 32 == 1) ? 1 : 0;
-        const int bx = P.nx + xoff >= 128 ? 128 : ((P.nx + xoff + 31) / 32) * 32;
-        dim3 grid((P.nx + xoff + bx - 1) / bx, P.ny, P.nz);
-        fbar_kernel<T, S, 1><<<grid, bx, 0, st>>>(f, fb, P, xoff);
+        // FP32: stage (a) writes the ghost layer itself (one launch)
+        fbar_float_kernel<S, 1><<<grid, bx, 0, st>>>(f, fb, P, xoff, rows);
+    } else if constexpr (sizeof(S) == 2) {
+        // 16-bit storage between walls: stage (a) also writes the y / z images (the same encoded
+        // values); the flux kernel forms the wall ghost columns in shared memory.  Periodic: the
+        // fused ghost writes cost more issue in stage (a) (encode) than the separate pass saves
+        if (!P.periodic_x)
+            fbar_float_kernel<S, 2><<<grid, bx, 0, st>>>(f, fb, P, 0, rows);
+        else
+            fbar_float_kernel<S, 0><<<grid, bx, 0, st>>>(f, fb, P, 0, rows);
+        ghosts = P.periodic_x;
     } else {
-        const int bx = P.nx >= 128 ? 128 : ((P.nx + 31) / 32) * 32;
-        dim3 grid((P.nx + bx - 1) / bx, P.ny, P.nz);
-        if (sizeof(S) == 2 && !P.periodic_x) {
-            // 16-bit storage between walls: stage (a) also writes the y / z images (the same
-            // encoded values); the flux kernel forms the wall ghost columns in shared memory
-            fbar_kernel<T, S, 2><<<grid, bx, 0, st>>>(f, fb, P, 0);
-        } else {
-            // FP64 and periodic 16-bit storage: the fused ghost writes cost more issue in
-            // stage (a) (FP64 pipe, 16-bit encode) than the separate pass saves
-            fbar_kernel<T, S, 0><<<grid, bx, 0, st>>>(f, fb, P, 0);
-            const long long ghosts = fb_ghosts(P.nx, P.ny, P.nz);
-            fb_ghost_kernel<T, S><<<unsigned((ghosts + 255) / 256), 256, 0, st>>>(fb, P);
-        }
+        fbar_kernel<T, S><<<dim3((P.nx + bx - 1) / bx, P.ny, P.nz), bx, 0, st>>>(f, fb, P);
+        ghosts = true;
+    }
+    if (ghosts) {
+        const long long n = fb_ghosts(P.nx, P.ny, P.nz);
+        fb_ghost_kernel<T, S><<<unsigned((n + 255) / 256), 256, 0, st>>>(fb, P);
     }
     return cudaGetLastError();
 }
