@@ -1026,17 +1026,77 @@ __device__ __forceinline__ float2 lerp_first_x2(float2 om, float2 m, S ap, S aq,
     }
 }
 
+// The 10 populations that move along z, as the five pairs (5, 6), (11, 12), (13, 14),
+// (15, 16), (17, 18), interpolated within one plane at an x face I or a y face J: at plane
+// k where c_z > 0, at plane k+1 where c_z < 0.  An x or y face at plane k lies between
+// this at k and at k-1 (both populations of a stencil reach back one of the two), so the
+// march along z forms it once per plane and keeps the last one.
 template <class S, int AX, class RD>
-__device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const RD &R, int i, int j, int k,
-                                            float v[NPOP])
+__device__ __forceinline__ void zpairs_x2(const StepParams<float, S> &P, const RD &R, int i, int j, int k, float2 N[5])
 {
     using RI = decltype(R.rb(0, 0));
-    const int jm = j - 1, jp = j + 1, jc = j;
-    const int km = k - 1, kp = k + 1, kc = k;
+    const int xs = P.xws;
+    const float2 ty_o = make_float2(P.ty_om, P.ty_om), ty_m = make_float2(P.ty_m, P.ty_m);
+    // first lerp of populations p, q between (row ra, column ca) and (row rb, column cb) of each
+    auto L1 = [&](float2 om, float2 m, int p, int q, RI rap, int cap, RI raq, int caq, RI rbp, int cbp, RI rbq,
+                  int cbq) {
+        return lerp_first_x2<S>(om, m, R.bits(p, rap, cap), R.bits(q, raq, caq), R.bits(p, rbp, cbp),
+                                R.bits(q, rbq, cbq));
+    };
+#pragma unroll
+    for (int t = 0; t < 5; ++t) {
+        const int p = t == 0 ? 5 : 9 + 2 * t, q = p + 1;
+        const int kp = cz(p) > 0 ? k : k + 1, kq = cz(q) > 0 ? k : k + 1;
+        if (AX == 0) {
+            const int A = i == 0 ? 1 : i, B = i == 0 ? 0 : i + 1;
+            const float *xw = P.xw + i;
+            float2 om, m;
+            if (cx(p)) {
+                om = make_float2(__ldg(xw + 2 * xs), __ldg(xw + 4 * xs));
+                m = make_float2(__ldg(xw + 3 * xs), __ldg(xw + 5 * xs));
+            } else {
+                const float om3 = __ldg(xw + 6 * xs), m3 = __ldg(xw + 7 * xs);
+                om = make_float2(om3, om3);
+                m = make_float2(m3, m3);
+            }
+            const RI r0 = R.rb(j, kp), s0 = R.rb(j, kq);
+            N[t] = L1(om, m, p, q, r0, A, s0, A, r0, B, s0, B);
+            if (cy(p)) {
+                const RI r1 = R.rb(j - cy(p), kp), s1 = R.rb(j - cy(q), kq);
+                N[t] = lerp_x2(ty_o, ty_m, N[t], L1(om, m, p, q, r1, A, s1, A, r1, B, s1, B));
+            }
+        } else {
+            const float2 yo = make_float2(P.yn_om[p], P.yn_om[q]), ym = make_float2(P.yn_m[p], P.yn_m[q]);
+            const RI rA = R.rb(j, kp), sA = R.rb(j, kq), rB = R.rb(j + 1, kp), sB = R.rb(j + 1, kq);
+            if (cx(p)) {
+                const float *tw = P.txw + i;
+                const float2 tx_o = make_float2(__ldg(tw + 2 * xs), __ldg(tw + 4 * xs));
+                const float2 tx_m = make_float2(__ldg(tw + 3 * xs), __ldg(tw + 5 * xs));
+                const int ip = i - cx(p), iq = i - cx(q);
+                N[t] = lerp_x2(yo, ym, L1(tx_o, tx_m, p, q, rA, i, sA, i, rA, ip, sA, iq),
+                               L1(tx_o, tx_m, p, q, rB, i, sB, i, rB, ip, sB, iq));
+            } else {
+                N[t] = L1(yo, ym, p, q, rA, i, sA, i, rB, i, sB, i);
+            }
+        }
+    }
+}
+
+// 19 values of an x (AX = 0) or y (AX = 1) face; old: zpairs_x2 of plane k-1, becomes
+// that of plane k.
+template <class S, int AX, class RD>
+__device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const RD &R, int i, int j, int k,
+                                            float2 old[5], float v[NPOP])
+{
+    using RI = decltype(R.rb(0, 0));
     const int xs = P.xws;
     const float2 ty_o = make_float2(P.ty_om, P.ty_om), ty_m = make_float2(P.ty_m, P.ty_m);
     const float2 tz_o = make_float2(P.tz_om, P.tz_om), tz_m = make_float2(P.tz_m, P.tz_m);
-    // first lerp of populations p, q between (row ra, column ca) and (row rb, column cb) of each
+    auto put = [&](int p, float2 res) {
+        const float2 e = R.dec_e2(p, p + 1, res);
+        v[p] = e.x;
+        v[p + 1] = e.y;
+    };
     auto L1 = [&](float2 om, float2 m, int p, int q, RI rap, int cap, RI raq, int caq, RI rbp, int cbp, RI rbq,
                   int cbq) {
         return lerp_first_x2<S>(om, m, R.bits(p, rap, cap), R.bits(q, raq, caq), R.bits(p, rbp, cbp),
@@ -1049,41 +1109,23 @@ __device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const
         const float2 m12 = make_float2(__ldg(xw + 3 * xs), __ldg(xw + 5 * xs));
         const float om3 = __ldg(xw + 6 * xs), m3 = __ldg(xw + 7 * xs);
         const float2 om33 = make_float2(om3, om3), m33 = make_float2(m3, m3);
-        const RI r00 = R.rb(jc, kc);
+        const RI r00 = R.rb(j, k);
         v[0] = R.dec_e(0, 0.5f * (R.raw(0, r00, A) + R.raw(0, r00, B)));
 #pragma unroll
         for (int n = 0; n < 9; ++n) {
             const int p = pair_p(0, n), q = pair_q(0, n);
-            const bool ay = cy(p) != 0, az = cz(p) != 0;
+            if (cz(p)) continue;
             const float2 om = xrep(p) == 3 ? om33 : om12, m = xrep(p) == 3 ? m33 : m12;
-            const int jtp = cy(p) > 0 ? jm : (cy(p) < 0 ? jp : jc), jtq = cy(q) > 0 ? jm : (cy(q) < 0 ? jp : jc);
-            const int ktp = cz(p) > 0 ? km : (cz(p) < 0 ? kp : kc), ktq = cz(q) > 0 ? km : (cz(q) < 0 ? kp : kc);
-            const float2 x00 = L1(om, m, p, q, r00, A, r00, A, r00, B, r00, B);
-            float2 y00 = x00;
-            if (ay) {
-                const RI sp = R.rb(jtp, kc), sq = R.rb(jtq, kc);
-                const float2 x01 = L1(om, m, p, q, sp, A, sq, A, sp, B, sq, B);
-                y00 = lerp_x2(ty_o, ty_m, x00, x01);
+            float2 res = L1(om, m, p, q, r00, A, r00, A, r00, B, r00, B);
+            if (cy(p)) {
+                const RI sp = R.rb(j - cy(p), k), sq = R.rb(j - cy(q), k);
+                res = lerp_x2(ty_o, ty_m, res, L1(om, m, p, q, sp, A, sq, A, sp, B, sq, B));
             }
-            float2 res = y00;
-            if (az) {
-                const RI tp = R.rb(jc, ktp), tq = R.rb(jc, ktq);
-                const float2 x10 = L1(om, m, p, q, tp, A, tq, A, tp, B, tq, B);
-                float2 y11 = x10;
-                if (ay) {
-                    const RI up = R.rb(jtp, ktp), uq = R.rb(jtq, ktq);
-                    const float2 x11 = L1(om, m, p, q, up, A, uq, A, up, B, uq, B);
-                    y11 = lerp_x2(ty_o, ty_m, x10, x11);
-                }
-                res = lerp_x2(tz_o, tz_m, y00, y11);
-            }
-            const float2 e = R.dec_e2(p, q, res);
-            v[p] = e.x;
-            v[q] = e.y;
+            put(p, res);
         }
-    } else if (AX == 1) {
-        // rows j (A) and j+1 (B); transverse x to column i - cx, z to plane k - cz
-        const RI rA = R.rb(jc, kc), rB = R.rb(jp, kc);
+    } else {
+        // rows j (A) and j+1 (B); transverse x to column i - cx
+        const RI rA = R.rb(j, k), rB = R.rb(j + 1, k);
         v[0] = R.dec_e(0, 0.5f * (R.raw(0, rA, i) + R.raw(0, rB, i)));
         const float *tw = P.txw + i;
         const float2 tx_o = make_float2(__ldg(tw + 2 * xs), __ldg(tw + 4 * xs));
@@ -1091,71 +1133,85 @@ __device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const
 #pragma unroll
         for (int n = 0; n < 9; ++n) {
             const int p = pair_p(1, n), q = pair_q(1, n);
-            const bool ax = cx(p) != 0, az = cz(p) != 0;
-            const int iop = i - cx(p), ioq = i - cx(q);
-            const int ktp = cz(p) > 0 ? km : (cz(p) < 0 ? kp : kc), ktq = cz(q) > 0 ? km : (cz(q) < 0 ? kp : kc);
+            if (cz(p)) continue;
+            const int ip = i - cx(p), iq = i - cx(q);
             const float2 yo = make_float2(P.yn_om[p], P.yn_om[q]), ym = make_float2(P.yn_m[p], P.yn_m[q]);
-            // normal lerp between rows A and B of the values at column i, x-lerped first when c_x != 0
-            auto yl = [&](RI sAp, RI sAq, RI sBp, RI sBq) {
-                if (ax) {
-                    const float2 x0 = L1(tx_o, tx_m, p, q, sAp, i, sAq, i, sAp, iop, sAq, ioq);
-                    const float2 x1 = L1(tx_o, tx_m, p, q, sBp, i, sBq, i, sBp, iop, sBq, ioq);
-                    return lerp_x2(yo, ym, x0, x1);
-                }
-                return L1(yo, ym, p, q, sAp, i, sAq, i, sBp, i, sBq, i);
-            };
-            const float2 y00 = yl(rA, rA, rB, rB);
-            float2 res = y00;
-            if (az) {
-                const RI sAp = R.rb(jc, ktp), sBp = R.rb(jp, ktp), sAq = R.rb(jc, ktq), sBq = R.rb(jp, ktq);
-                res = lerp_x2(tz_o, tz_m, y00, yl(sAp, sAq, sBp, sBq));
-            }
-            const float2 e = R.dec_e2(p, q, res);
-            v[p] = e.x;
-            v[q] = e.y;
+            if (cx(p))
+                put(p, lerp_x2(yo, ym, L1(tx_o, tx_m, p, q, rA, i, rA, i, rA, ip, rA, iq),
+                               L1(tx_o, tx_m, p, q, rB, i, rB, i, rB, ip, rB, iq)));
+            else
+                put(p, L1(yo, ym, p, q, rA, i, rA, i, rB, i, rB, i));
         }
-    } else {
-        // planes k (A) and k+1 (B); transverse x to column i - cx, y to row j - cy
-        const RI rA = R.rb(jc, kc), rB = R.rb(jc, kp);
-        v[0] = R.dec_e(0, 0.5f * (R.raw(0, rA, i) + R.raw(0, rB, i)));
-        const float *tw = P.txw + i;
-        const float2 tx_o = make_float2(__ldg(tw + 2 * xs), __ldg(tw + 4 * xs));
-        const float2 tx_m = make_float2(__ldg(tw + 3 * xs), __ldg(tw + 5 * xs));
+    }
+    float2 N[5];
+    zpairs_x2<S, AX>(P, R, i, j, k, N);
 #pragma unroll
-        for (int n = 0; n < 9; ++n) {
-            const int p = pair_p(2, n), q = pair_q(2, n);
-            const bool ax = cx(p) != 0, ay = cy(p) != 0;
-            const int iop = i - cx(p), ioq = i - cx(q);
-            const int jtp = cy(p) > 0 ? jm : (cy(p) < 0 ? jp : jc), jtq = cy(q) > 0 ? jm : (cy(q) < 0 ? jp : jc);
-            const float2 zo = make_float2(P.zn_om[p], P.zn_om[q]), zm = make_float2(P.zn_m[p], P.zn_m[q]);
-            // value at column i of rows sp / sq, x-lerped when c_x != 0 (first lerps)
-            auto xl = [&](RI sp, RI sq) {
-                return L1(tx_o, tx_m, p, q, sp, i, sq, i, sp, iop, sq, ioq);
-            };
-            float2 res;
-            if (!ax && !ay) {
-                res = L1(zo, zm, p, q, rA, i, rA, i, rB, i, rB, i);
-            } else {
-                float2 y00, y11;
-                if (ay) {
-                    const RI sAp = R.rb(jtp, kc), sBp = R.rb(jtp, kp), sAq = R.rb(jtq, kc), sBq = R.rb(jtq, kp);
-                    if (ax) {
-                        y00 = lerp_x2(ty_o, ty_m, xl(rA, rA), xl(sAp, sAq));
-                        y11 = lerp_x2(ty_o, ty_m, xl(rB, rB), xl(sBp, sBq));
-                    } else {
-                        y00 = L1(ty_o, ty_m, p, q, rA, i, rA, i, sAp, i, sAq, i);
-                        y11 = L1(ty_o, ty_m, p, q, rB, i, rB, i, sBp, i, sBq, i);
-                    }
-                } else {
-                    y00 = xl(rA, rA);
-                    y11 = xl(rB, rB);
-                }
-                res = lerp_x2(zo, zm, y00, y11);
-            }
-            const float2 e = R.dec_e2(p, q, res);
-            v[p] = e.x;
-            v[q] = e.y;
-        }
+    for (int t = 0; t < 5; ++t) {
+        const int p = t == 0 ? 5 : 9 + 2 * t, q = p + 1;
+        // plane k, and plane k - c_z of each
+        const float2 a = make_float2(cz(p) > 0 ? N[t].x : old[t].x, cz(q) > 0 ? N[t].y : old[t].y);
+        const float2 b = make_float2(cz(p) > 0 ? old[t].x : N[t].x, cz(q) > 0 ? old[t].y : N[t].y);
+        put(p, lerp_x2(tz_o, tz_m, a, b));
+        old[t] = N[t];
+    }
+}
+
+// Plane k's part of the z faces below and above it: every population interpolated in x
+// and y at column i, row j.
+template <class S, class RD>
+__device__ __forceinline__ void plane_z_x2(const StepParams<float, S> &P, const RD &R, int i, int j, int k, float Y[NPOP])
+{
+    using RI = decltype(R.rb(0, 0));
+    const int xs = P.xws;
+    const float2 ty_o = make_float2(P.ty_om, P.ty_om), ty_m = make_float2(P.ty_m, P.ty_m);
+    const float *tw = P.txw + i;
+    const float2 tx_o = make_float2(__ldg(tw + 2 * xs), __ldg(tw + 4 * xs));
+    const float2 tx_m = make_float2(__ldg(tw + 3 * xs), __ldg(tw + 5 * xs));
+    const RI r = R.rb(j, k);
+    Y[0] = R.raw(0, r, i);
+#pragma unroll
+    for (int n = 0; n < 9; ++n) {
+        const int p = pair_p(2, n), q = pair_q(2, n);
+        const bool ax = cx(p) != 0, ay = cy(p) != 0;
+        const RI sp = R.rb(j - cy(p), k), sq = R.rb(j - cy(q), k);
+        // value at column i of rows rp / rq, x-lerped when c_x != 0 (first lerps)
+        auto xl = [&](RI rp, RI rq) {
+            return lerp_first_x2<S>(tx_o, tx_m, R.bits(p, rp, i), R.bits(q, rq, i), R.bits(p, rp, i - cx(p)),
+                                    R.bits(q, rq, i - cx(q)));
+        };
+        float2 y;
+        if (ax && ay)
+            y = lerp_x2(ty_o, ty_m, xl(r, r), xl(sp, sq));
+        else if (ax)
+            y = xl(r, r);
+        else if (ay)
+            y = lerp_first_x2<S>(ty_o, ty_m, R.bits(p, r, i), R.bits(q, r, i), R.bits(p, sp, i), R.bits(q, sq, i));
+        else
+            y = make_float2(R.raw(p, r, i), R.raw(q, r, i));
+        Y[p] = y.x;
+        Y[q] = y.y;
+    }
+}
+
+// 19 values of the z face between the planes with parts Y (below) and Z.
+template <class S, class RD>
+__device__ __forceinline__ void face_z_x2(const StepParams<float, S> &P, const RD &R, const float Y[NPOP],
+                                          const float Z[NPOP], float v[NPOP])
+{
+    v[0] = R.dec_e(0, 0.5f * (Y[0] + Z[0]));
+#pragma unroll
+    for (int n = 0; n < 9; ++n) {
+        const int p = pair_p(2, n), q = pair_q(2, n);
+        const float2 zo = make_float2(P.zn_om[p], P.zn_om[q]), zm = make_float2(P.zn_m[p], P.zn_m[q]);
+        const float2 a = make_float2(Y[p], Y[q]), b = make_float2(Z[p], Z[q]);
+        float2 res;
+        if (sizeof(S) == 2 && !cx(p) && !cy(p))  // its only lerp: as lerp_first_x2
+            res = __ffma2_rn(zm, make_float2(b.x - a.x, b.y - a.y), a);
+        else
+            res = lerp_x2(zo, zm, a, b);
+        const float2 e = R.dec_e2(p, q, res);
+        v[p] = e.x;
+        v[q] = e.y;
     }
 }
 
@@ -1511,17 +1567,15 @@ __device__ __forceinline__ void bounce_back(T v[NPOP], bool lo, bool hi)
     }
 }
 
-// Fluxes of one face: reconstruction + bounce-back + face equilibrium.
+// Fluxes of one face in FP64: reconstruction + bounce-back + face equilibrium.
 template <class T, class S, int AX, int RECON, bool FF, class RD>
 __device__ __forceinline__ void face_fluxes(const StepParams<T, S> &P, const RD &R, int i, int j, int k, T out[10])
 {
     T v[NPOP];
-    if constexpr (RECON == 0 && Fp64Form<T>::value)
+    if constexpr (RECON == 0)
         face_tri_cw<T, S, AX>(P, R, i, j, k, v);
-    else if constexpr (RECON == 0)
-        face_tri_x2<S, AX>(P, R, i, j, k, v);  // packed lerps: FP32, FP16, BF16
     else
-        face_grad<T, S, AX>(P, R, i, j, k, v);  // FP64 (float forms: flux_shared.cuh)
+        face_grad<T, S, AX>(P, R, i, j, k, v);
     if (AX == 0 && !P.periodic_x) bounce_back(v, i == 0, i == P.nx);
     face_flux<T, S, AX, FF>(P, v, out, FF ? face_field<T, S, AX>(P, i, j, k) : T(0));
 }
@@ -1690,6 +1744,11 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int lim
     return false;
 }
 
+// Float forms.  What the march along z already has is not formed again: the in-plane
+// part of the z-moving populations at x and y faces (zpairs_x2) and, in FP32, of every
+// population at z faces, 159 instead of 258 stencil reads and 141 instead of 201 lerps
+// per cell, each with its operations in the same order.  Flux kernel of the 256 x 128 x
+// 128 channel: FP32 0.301 -> 0.255 ms, FP16 0.335 -> 0.321 ms, BF16 0.327 -> 0.317 ms.
 template <class T, class S, int W, int MINB, bool FF>
 __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_constant__ CUtensorMap tmap,
                                                                  const S *f_in, S *f_out,
@@ -1785,6 +1844,17 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_con
     const int hj = j0 + lane;
     const bool hx = wr == 0 && lane < W - 1 && hj <= ny;
 
+    // the tile's f-tilde of plane k into L2 (halo warp), a plane ahead of its use
+    auto prefetch = [&](int k) {
+        const int seg = lane & 1 ? 128 / int(sizeof(S)) : 0;  // 32 cells lie in one or two lines
+        for (int t = lane >> 1; t < NPOP * (W - 1); t += 16) {
+            const int p = t / (W - 1), r = t - p * (W - 1);
+            if (seg < 32)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(f_in + p * P.ps +
+                                                              ((long long)(k - 1) * ny + min(j0 - 1 + r, ny - 1)) * P.pitch +
+                                                              min(i0 - 1 + seg, nx - 1)));
+        }
+    };
     for (int g = kb - 1; g <= kb + 2; ++g) issue(g);
     T fzd[10], fzu[10], fx[10], fy[10], fo[NPOP];
     int buf = 0;
@@ -1796,7 +1866,42 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_con
         wall_ghosts(kb);
         __syncthreads();
     }
-    if (wr >= 1) face_fluxes<T, S, 2, 0, FF>(P, R, ci, cj, kb - 1, fzd);
+    // FP32 also keeps plane k's part of the z faces (19 registers) and fetches f-tilde into
+    // L2 a plane ahead; in the 16-bit forms, which widen values as they read them and have
+    // no registers left, both measured slower (0.321 -> 0.322 ms, 0.335 -> 0.358 ms)
+    constexpr bool FP32 = sizeof(S) == 4;
+    // fluxes of an x or y face (old: see face_tri_x2) and of the z face above plane k
+    auto x_flux = [&](int i, int j, int k, float2 *old, T out[10]) {
+        T v[NPOP];
+        face_tri_x2<S, 0>(P, R, i, j, k, old, v);
+        if (!P.periodic_x) bounce_back(v, i == 0, i == nx);
+        face_flux<T, S, 0, FF>(P, v, out, FF ? face_field<T, S, 0>(P, i, j, k) : T(0));
+    };
+    auto y_flux = [&](int i, int j, int k, float2 *old, T out[10]) {
+        T v[NPOP];
+        face_tri_x2<S, 1>(P, R, i, j, k, old, v);
+        face_flux<T, S, 1, FF>(P, v, out, FF ? face_field<T, S, 1>(P, i, j, k) : T(0));
+    };
+    T Y[NPOP];  // plane k's part of the z faces
+    auto z_flux = [&](int k, T out[10]) {
+        T Z[NPOP], v[NPOP];
+        if (!FP32) plane_z_x2<S>(P, R, ci, cj, k, Y);
+        plane_z_x2<S>(P, R, ci, cj, k + 1, Z);
+        face_z_x2<S>(P, R, Y, Z, v);
+        face_flux<T, S, 2, FF>(P, v, out, FF ? face_field<T, S, 2>(P, ci, cj, k) : T(0));
+        if (FP32) {
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) Y[p] = Z[p];
+        }
+    };
+    float2 ox[5], oy[5];
+    const int xi = wr >= 1 ? ci : i0 - 1, xj = wr >= 1 ? cj : (hx ? hj : j0), yj = wr >= 1 ? cj : j0 - 1;
+    zpairs_x2<S, 0>(P, R, xi, xj, kb - 1, ox);
+    zpairs_x2<S, 1>(P, R, ci, yj, kb - 1, oy);
+    if (wr >= 1) {
+        if (FP32) plane_z_x2<S>(P, R, ci, cj, kb - 1, Y);
+        z_flux(kb - 1, fzd);
+    }
     for (int k = kb; k < ke; ++k) {
         wait(k + 1);
         if (wall_tile) {
@@ -1804,9 +1909,9 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_con
             __syncthreads();
         }
         if (wr >= 1) {
-            face_fluxes<T, S, 0, 0, FF>(P, R, ci, cj, k, fx);
-            face_fluxes<T, S, 1, 0, FF>(P, R, ci, cj, k, fy);
-            face_fluxes<T, S, 2, 0, FF>(P, R, ci, cj, k, fzu);
+            x_flux(ci, cj, k, ox, fx);
+            y_flux(ci, cj, k, oy, fy);
+            z_flux(k, fzu);
 #pragma unroll
             for (int s = 0; s < 10; ++s) ysh[buf][wr][s][lane] = fy[s];
             // the cell's f-tilde, loaded before the barrier so its latency overlaps the exchange
@@ -1816,15 +1921,16 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_tma_kernel(const __grid_con
                 for (int p = 0; p < NPOP; ++p) fo[p] = P.codec.raw(f_in, p * P.ps + c);
             }
         } else {
-            face_fluxes<T, S, 1, 0, FF>(P, R, ci, j0 - 1, k, fy);
+            y_flux(ci, j0 - 1, k, oy, fy);
 #pragma unroll
             for (int s = 0; s < 10; ++s) ysh[buf][0][s][lane] = fy[s];
             if (hx) {
                 T hxf[10];
-                face_fluxes<T, S, 0, 0, FF>(P, R, i0 - 1, hj, k, hxf);
+                x_flux(i0 - 1, hj, k, ox, hxf);
 #pragma unroll
                 for (int s = 0; s < 10; ++s) xsh[buf][lane + 1][s] = hxf[s];
             }
+            if (FP32 && k + 1 < ke) prefetch(k + 1);
         }
         __syncthreads();
         issue(k + 3);  // plane k-1 (same stage) is no longer read

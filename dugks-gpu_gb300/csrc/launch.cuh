@@ -15,12 +15,15 @@ namespace dg {
 template <class T, class S>
 struct TileCfg {
     static constexpr int W = 8;       // 7 rows of 32 cells
-    static constexpr int MINB = 2;    // two CTAs per SM (<= 128 registers)
+    static constexpr int MINB = 2;    // two CTAs per SM (<= 128 registers); (6, 2) 0.35, (7, 2) 0.37 ms against 0.32
     static constexpr bool TMA = true; // 4 x 13.7 KB planes per CTA for 16-bit storage
 };
 template <>
 struct TileCfg<float, float> {
-    static constexpr int W = 7;       // 6 rows: 4 x 21.9 KB planes, two CTAs per SM
+    // 5 rows: 4 x 19.2 KB planes, two CTAs per SM at up to 170 registers.  Flux kernel of the
+    // 256 x 128 x 128 channel by (W, CTAs per SM), ms: (6, 2) 0.255, (12, 1) 0.276, (4, 3)
+    // 0.28, (5, 2) 0.32, (7, 2) 0.36 (128 registers, spills)
+    static constexpr int W = 6;
     static constexpr int MINB = 2;
     static constexpr bool TMA = true;
 };
