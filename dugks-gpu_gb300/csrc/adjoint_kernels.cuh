@@ -9,8 +9,8 @@
 // Given lam' = dJ/df', the adjoint step returns lam = (dS/df)^T lam':
 //   lamF = -D^T lam'                    (per face, the two adjacent cells)
 //   lamv = B^T (dphi/dv')^T lamF        adj_face_kernel, one thread per face
-//   mu   = 4/3 lam' + G^T L^T lamv      adj_gather_kernel (gather form, deterministic)
-//   lam  = (dA/df)^T mu - 1/3 lam'      adj_gather_kernel
+//   mu   = 4/3 lam' + G^T L^T lamv      adj_cell_kernel (gather form, deterministic)
+//   lam  = (dA/df)^T mu - 1/3 lam'      adj_cell_kernel
 // For a face or a cell with density r, first moment j, u0 = j/r,
 // u = u0 + shift, coefficient c_p = fw2 + 3 fw0 (F.c_p - F.u) and
 // feq_p = w_p r (1 + 3 c_p.u + 4.5 (c_p.u)^2 - 1.5 u.u), the map
@@ -116,24 +116,29 @@ __host__ __device__ inline long long adj_cell(int i, int j, int k, int nx, int n
     return ((long long)(k - 1) * ny + (j - 1)) * nx + (i - 1);
 }
 
-// Per-face adjoint: reconstruct the face values (the forward's face_tri with
-// reader RD), take the flux adjoint from the two adjacent cells' lam', apply
-// (dphi/dv)^T and the bounce-back transpose.  F: the face's first index (x
-// faces: I = 0..nx, between columns I and I+1; y / z faces: the column i);
-// j, k: row and plane (1-based).  lv: the 19 adjoint face values; lf: dJ/dF
-// of the face force along the field axis (0 without a field).
-template <class T, class S, int AX, class RD>
-__device__ __forceinline__ void adj_face_values(const StepParams<T, S> &P, const RD &R,
-                                                const S *__restrict__ lam_next, int F, int j, int k, T lv[NPOP],
-                                                T &lf)
+// Layout of the adjoint face values LX, LY, LZ: per row (k, j) blocks of 32 columns with
+// the 19 populations of a block one after another, so that a population step is an
+// immediate of the load and a row's address serves all of them.  Column of the x face I,
+// 1 <= I <= nx, and of the y and z faces at i: adj_col; the x face 0 between walls: nx.
+__host__ __device__ constexpr int adj_col(int c) { return (c >> 5) * (NPOP * 32) + (c & 31); }
+__host__ __device__ inline int adj_xcol(int I, int nx) { return adj_col(I >= 1 ? I - 1 : nx); }
+__host__ __device__ inline int adj_rowlen(int nx) { return (nx + 32) / 32 * (NPOP * 32); }
+__host__ __device__ inline long long adj_row(int j, int k, int nx, int ny)
+{
+    return ((long long)(k - 1) * ny + (j - 1)) * adj_rowlen(nx);
+}
+
+// Per-face adjoint of the face values v: take the flux adjoint from the two adjacent
+// cells' lam', apply (dphi/dv)^T and the bounce-back transpose.  F: the face's first index
+// (x faces: I = 0..nx, between columns I and I+1; y / z faces: the column i); j, k: row and
+// plane (1-based).  lv: the 19 adjoint face values; lf: dJ/dF of the face force along the
+// field axis (0 without a field).
+template <class T, class S, int AX>
+__device__ __forceinline__ void adj_face_flux(const StepParams<T, S> &P, T v[NPOP], const S *__restrict__ lam_next,
+                                              int F, int j, int k, T lv[NPOP], T &lf)
 {
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const int I = AX == 0 ? F : 0, i = AX == 0 ? 1 : F;
-    T v[NPOP];
-    if (Fp64Form<T>::value)
-        face_tri_cw<T, S, AX>(P, R, F, j, k, v);  // the forward's own face values
-    else
-        face_tri<T, S, AX>(P, R, F, j, k, v);
     const bool lo = AX == 0 && !P.periodic_x && I == 0;
     const bool hi = AX == 0 && !P.periodic_x && I == nx;
     bounce_back(v, lo, hi);
@@ -238,7 +243,7 @@ __device__ __forceinline__ void adj_face_values(const StepParams<T, S> &P, const
 }
 
 // One thread per face of orientation AX (f-bar-plus through L1), storing
-// lamv[19] of the face (population-major, stride nface) and dJ/dF.
+// lamv[19] of the face and dJ/dF.
 // only_x0: x faces I = 0 only (one thread per row and plane).
 template <class T, class S, int AX>
 __global__ void __launch_bounds__(128) adj_face_kernel(const S *__restrict__ fb, const S *__restrict__ lam_next,
@@ -262,8 +267,7 @@ __global__ void __launch_bounds__(128) adj_face_kernel(const S *__restrict__ fb,
         const long long r = q / (nx + 1);
         j = int(r % ny) + 1;
         k = int(r / ny) + 1;
-        if (P.periodic_x && F == 0) {
-            for (int p = 0; p < NPOP; ++p) lamv[p * nface + q] = T(0);  // periodic: face 0 is face nx
+        if (P.periodic_x && F == 0) {  // face 0 is face nx
             if (lamF_face) lamF_face[q] = T(0);
             return;
         }
@@ -276,18 +280,26 @@ __global__ void __launch_bounds__(128) adj_face_kernel(const S *__restrict__ fb,
         k = int(r / ny) + 1;
     }
     const FbRead<T, S> R{fb, P.ps_b, P.pitch_b, ny, nz, P.codec};
-    T lv[NPOP], lf;
-    adj_face_values<T, S, AX>(P, R, lam_next, F, j, k, lv, lf);
+    T v[NPOP], lv[NPOP], lf;
+    if (Fp64Form<T>::value)
+        face_tri_cw<T, S, AX>(P, R, F, j, k, v);  // the forward's own face values
+    else
+        face_tri<T, S, AX>(P, R, F, j, k, v);
+    adj_face_flux<T, S, AX>(P, v, lam_next, F, j, k, lv, lf);
     if (lamF_face) lamF_face[q] = lf;
+    T *o = lamv + adj_row(j, k, nx, ny) + (AX == 0 ? adj_xcol(F, nx) : adj_col(F - 1));
 #pragma unroll
-    for (int p = 0; p < NPOP; ++p) lamv[p * nface + q] = lv[p];
+    for (int p = 0; p < NPOP; ++p) o[p * 32] = lv[p];
 }
 
 // The three faces +x (I = i), +y (J = j) and +z (K = k) of every cell, with
 // f-bar-plus staged through the same 4-plane TMA ring as the forward flux
-// kernel: W warps, one row of 32 cells each, marching a chunk of z planes.
+// kernel: W warps, one row of 32 cells each, marching a chunk of z planes, and with its
+// reuse along the march (zpairs_x2, plane_z_x2).
 // The box holds rows j0-1 .. j0+W (the stencil's transverse and +y rows).
 // x faces I = 0 are left to adj_face_kernel (only_x0).
+// FP32, 128 x 96 x 96 channel: 159 us with seven warps and face_tri, 149 us with the
+// reuse, 145 us with eight warps (two CTAs per SM; four and six warps +1 %).
 template <class T, class S, int W>
 constexpr size_t adj_faces_tma_smem_bytes()
 {
@@ -348,27 +360,42 @@ __global__ void __launch_bounds__(32 * W, MINB) adj_faces_tma_kernel(const __gri
 
     const int gi = i0 + lane, gj = j0 + wr;
     const bool cell = gi <= nx && gj <= ny;
-    const long long nfx = adj_nface(0, nx, ny, nz), nfc = adj_nface(1, nx, ny, nz);
     for (int g = kb - 1; g <= kb + 2; ++g) issue(g);
     wait(kb - 1);
     wait(kb);
+    float2 ox[5], oy[5];
+    T Y[NPOP];
+    if (cell) {
+        zpairs_x2<S, 0, true>(P, R, gi, gj, kb - 1, ox);
+        zpairs_x2<S, 1, true>(P, R, gi, gj, kb - 1, oy);
+        plane_z_x2<S, true>(P, R, gi, gj, kb, Y);
+    }
     for (int k = kb; k < ke; ++k) {
         wait(k + 1);
         if (cell) {
-            T lv[NPOP], lf;
+            T v[NPOP], lv[NPOP], lf;
             const long long qx = adj_xface(gi, gj, k, nx, ny), qc = adj_cell(gi, gj, k, nx, ny);
-            adj_face_values<T, S, 0>(P, R, lam_next, gi, gj, k, lv, lf);
+            const long long o = adj_row(gj, k, nx, ny) + adj_col(gi - 1);
+            face_tri_x2<S, 0, true>(P, R, gi, gj, k, ox, v);
+            adj_face_flux<T, S, 0>(P, v, lam_next, gi, gj, k, lv, lf);
             LFX[qx] = lf;
 #pragma unroll
-            for (int p = 0; p < NPOP; ++p) LX[p * nfx + qx] = lv[p];
-            adj_face_values<T, S, 1>(P, R, lam_next, gi, gj, k, lv, lf);
+            for (int p = 0; p < NPOP; ++p) LX[o + p * 32] = lv[p];
+            face_tri_x2<S, 1, true>(P, R, gi, gj, k, oy, v);
+            adj_face_flux<T, S, 1>(P, v, lam_next, gi, gj, k, lv, lf);
             LFY[qc] = lf;
 #pragma unroll
-            for (int p = 0; p < NPOP; ++p) LY[p * nfc + qc] = lv[p];
-            adj_face_values<T, S, 2>(P, R, lam_next, gi, gj, k, lv, lf);
+            for (int p = 0; p < NPOP; ++p) LY[o + p * 32] = lv[p];
+            T Z[NPOP];
+            plane_z_x2<S, true>(P, R, gi, gj, k + 1, Z);
+            face_z_x2<S, true>(P, R, Y, Z, v);
+            adj_face_flux<T, S, 2>(P, v, lam_next, gi, gj, k, lv, lf);
             LFZ[qc] = lf;
 #pragma unroll
-            for (int p = 0; p < NPOP; ++p) LZ[p * nfc + qc] = lv[p];
+            for (int p = 0; p < NPOP; ++p) {
+                LZ[o + p * 32] = lv[p];
+                Y[p] = Z[p];
+            }
         }
         __syncthreads();
         issue(k + 3);  // plane k-1 (same stage) is no longer read
@@ -376,204 +403,139 @@ __global__ void __launch_bounds__(32 * W, MINB) adj_faces_tma_kernel(const __gri
     // every plane issued (g <= ke) has been waited for: no bulk copy is left in flight
 }
 
-// Row / plane offsets of the face arrays around one interior cell (the
-// periodic images in y and z folded in): x faces ((k-1)*ny + (j-1))*(nx+1),
-// y / z faces ((k-1)*ny + (j-1))*nx, for j-1..j+1 and k-1..k+1.
-struct AdjRows {
-    int kx[3], jx[3];  // x faces: plane part ((k'-1)*ny)*(nx+1) and row part (j'-1)*(nx+1), k' = k-1..k+1
-    int kc[3], jc[3];  // y / z faces: the same with nx
-    __device__ __forceinline__ int x(int dk, int dj) const { return kx[dk] + jx[dj]; }  // [dk+1][dj+1]
-    __device__ __forceinline__ int c(int dk, int dj) const { return kc[dk] + jc[dj]; }
+// Where the transposed stencil of one cell reads: population 0 of the face rows around
+// row j, plane k, [dk+1][dj+1] (y faces: dj = -1, 0; z faces: dk = -1, 0; the periodic
+// images in y and z folded in), x faces at stored column cf, y and z faces at cc.
+template <class T>
+struct AdjAt {
+    const T *x[3][3], *y[3][2], *z[2][3];
 };
 
-__device__ __forceinline__ AdjRows adj_rows(int j, int k, int nx, int ny, int nz)
+template <class T>
+__device__ __forceinline__ AdjAt<T> adj_at(const T *LX, const T *LY, const T *LZ, int j, int k, int cf, int cc, int nx,
+                                           int ny, int nz)
 {
-    AdjRows R;
+    AdjAt<T> A;
     const int js[3] = {j == 1 ? ny : j - 1, j, j == ny ? 1 : j + 1};
     const int ks[3] = {k == 1 ? nz : k - 1, k, k == nz ? 1 : k + 1};
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        R.kx[a] = (ks[a] - 1) * ny * (nx + 1);
-        R.jx[a] = (js[a] - 1) * (nx + 1);
-        R.kc[a] = (ks[a] - 1) * ny * nx;
-        R.jc[a] = (js[a] - 1) * nx;
-    }
-    return R;
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const long long o = adj_row(js[b], ks[a], nx, ny);
+            A.x[a][b] = LX + o + cf;
+            if (b < 2) A.y[a][b] = LY + o + cc;
+            if (a < 2) A.z[a][b] = LZ + o + cc;
+        }
+    return A;
 }
 
-// Transposed-stencil sums of one population p (a compile-time constant)
-// around row j, plane k: the adjoint that an f-bar-plus value at column gi
-// receives from the x faces I (xsum) and from the y and z faces at column i
-// (colsum), with the stencil offsets resolved at compile time.
+// Transposed-stencil sums of one population p (a compile-time constant): the adjoint
+// that an f-bar-plus value receives from the x faces at A's face column (xsum) and from
+// the y and z faces at its column (colsum).
 template <int p, class T, class S>
 struct AdjPop {
-    const T *__restrict__ LX;
-    const T *__restrict__ LY;
-    const T *__restrict__ LZ;
+    const AdjAt<T> &A;
     const StepParams<T, S> &P;
-    const AdjRows &R;
-    long long nfx, nfc;
     static constexpr int ax = cx(p), ay = cy(p), az = cz(p), rp = xrep(p);
 
-    __device__ __forceinline__ T xsum(int I) const
+    __device__ __forceinline__ T X(int dk, int dj) const { return __ldg(A.x[dk + 1][dj + 1] + p * 32); }
+    __device__ __forceinline__ T Y(int dk, int dj) const { return __ldg(A.y[dk + 1][dj + 1] + p * 32); }
+    __device__ __forceinline__ T Z(int dk, int dj) const { return __ldg(A.z[dk + 1][dj + 1] + p * 32); }
+    __device__ __forceinline__ T xsum() const
     {
         const T tyo = p == 0 ? T(1) : P.ty_om, tym = P.ty_m, tzo = p == 0 ? T(1) : P.tz_om, tzm = P.tz_m;
-        const T *base = LX + (long long)p * nfx;
-        T s = (ay ? tyo : T(1)) * (az ? tzo : T(1)) * base[R.x(1, 1) + I];
-        if (ay) s += tym * (az ? tzo : T(1)) * base[R.x(1, 1 + ay) + I];
-        if (az) s += (ay ? tyo : T(1)) * tzm * base[R.x(1 + az, 1) + I];
-        if (ay && az) s += tym * tzm * base[R.x(1 + az, 1 + ay) + I];
+        T s = (ay ? tyo : T(1)) * (az ? tzo : T(1)) * X(0, 0);
+        if (ay) s += tym * (az ? tzo : T(1)) * X(0, ay);
+        if (az) s += (ay ? tyo : T(1)) * tzm * X(az, 0);
+        if (ay && az) s += tym * tzm * X(az, ay);
         return s;
     }
-    // x weight of face I: anchor (which = 0) or other column (which = 1)
-    __device__ __forceinline__ T xw(int I, int which) const
-    {
-        return p == 0 ? T(0.5) : __ldg(P.xw + (2 * rp + which) * P.xws + I);
-    }
-    // transverse x weight of the y / z faces at column i: own column (0) or column i - cx (1)
-    __device__ __forceinline__ T tw(int i, int which) const { return __ldg(P.txw + (2 * rp + which) * P.xws + i); }
-    __device__ __forceinline__ T colsum(int i) const
+    __device__ __forceinline__ T colsum() const
     {
         const T tyo = p == 0 ? T(1) : P.ty_om, tym = P.ty_m, tzo = p == 0 ? T(1) : P.tz_om, tzm = P.tz_m;
-        const int c = i - 1;
         T sy, sz;
         {
-            const T *base = LY + (long long)p * nfc;
             const T yo = p == 0 ? T(0.5) : P.yn_om[p], ym = p == 0 ? T(0.5) : P.yn_m[p];
-            sy = yo * base[R.c(1, 1) + c] + ym * base[R.c(1, 0) + c];
+            sy = yo * Y(0, 0) + ym * Y(0, -1);
             if (az) {
                 sy = tzo * sy;
-                sy += tzm * (yo * base[R.c(1 + az, 1) + c] + ym * base[R.c(1 + az, 0) + c]);
+                sy += tzm * (yo * Y(az, 0) + ym * Y(az, -1));
             }
         }
         {
-            const T *base = LZ + (long long)p * nfc;
             const T zo = p == 0 ? T(0.5) : P.zn_om[p], zm = p == 0 ? T(0.5) : P.zn_m[p];
-            sz = zo * base[R.c(1, 1) + c] + zm * base[R.c(0, 1) + c];
+            sz = zo * Z(0, 0) + zm * Z(-1, 0);
             if (ay) {
                 sz = tyo * sz;
-                sz += tym * (zo * base[R.c(1, 1 + ay) + c] + zm * base[R.c(0, 1 + ay) + c]);
+                sz += tym * (zo * Z(0, ay) + zm * Z(-1, ay));
             }
         }
         return sy + sz;
     }
-    // interior column gi (1..nx); Ix2 / x2_anchor: the second x face holding the
-    // column (face gi-1 as "other", face 0 as anchor for gi = 1 between walls,
-    // face nx as "other" for gi = 1 when periodic); i2: the column i with
-    // i - cx = gi of the y / z faces, 0 if none
-    __device__ __forceinline__ T interior(int gi, int Ix2, bool x2_anchor, int i2) const
-    {
-        T acc = xw(gi, 0) * xsum(gi) + xw(Ix2, x2_anchor ? 0 : 1) * xsum(Ix2);
-        if (ax) {
-            acc += tw(gi, 0) * colsum(gi);
-            if (i2 >= 1) acc += tw(i2, 1) * colsum(i2);
-        } else {
-            acc += colsum(gi);
-        }
-        return acc;
-    }
-    // wall ghost column 0 (side 0) or nx+1 (side 1): the other column of x face
-    // 0 / nx, and the y / z faces at column 1 (cx > 0) / nx (cx < 0)
-    __device__ __forceinline__ T ghost(int side) const
-    {
-        const int nx = P.nx;
-        const int I = side ? nx : 0;
-        T acc = xw(I, 1) * xsum(I);
-        if (!side && ax > 0) acc += tw(1, 1) * colsum(1);
-        if (side && ax < 0) acc += tw(nx, 1) * colsum(nx);
-        return acc;
-    }
 };
 
-// Adjoint received by the wall ghost columns (0 and nx+1) of f-bar-plus, per
-// population, row and plane: GH[(side*19 + p) * ny*nz + (k-1)*ny + (j-1)].
-// The gather folds it into columns 1, 2 and nx-1, nx with the extrapolation
-// weights.
+// x weight of face I (which = 0: anchor, 1: other column) and transverse x weight of the y
+// and z faces at column i (0: own column, 1: column i - cx), for the class of population p
+template <class T, class S>
+__device__ __forceinline__ T adj_xw(const StepParams<T, S> &P, int p, int I, int which)
+{
+    return p == 0 ? T(0.5) : __ldg(P.xw + (2 * xrep(p) + which) * P.xws + I);
+}
+template <class T, class S>
+__device__ __forceinline__ T adj_tw(const StepParams<T, S> &P, int p, int i, int which)
+{
+    return __ldg(P.txw + (2 * xrep(p) + which) * P.xws + i);
+}
+
+// x weights of an interior column i by class of c_x (+, -, 0): face i and the second x
+// face holding the column (face i-1 as "other", face 0 as anchor for i = 1 between walls,
+// face nx as "other" for i = 1 when periodic), transverse weights of its own column and of
+// the column i + c_x (zero past a wall)
+template <class T>
+struct AdjXw {
+    T f[3], g[3], t[2], n[2];
+};
+
+// Transposed interpolation stencil of the populations p and up at column i (the part of
+// mu that comes from the faces).  The lanes of a warp hold consecutive columns and each
+// forms the face sums of its own x face and column only: the face on the other side and
+// the column i + c_x come from the neighbouring lane.  wall: the warp holds columns next
+// to a wall, which also take the adjoint of the wall's ghost column: formed by the lane of
+// column 1 or nx, the next lane inside gets its share.
 template <class T, class S, int p = 0>
-__device__ __forceinline__ void adj_ghost_pops(const T *LX, const T *LY, const T *LZ, const StepParams<T, S> &P,
-                                               const AdjRows &R, long long nfx, long long nfc, int side,
-                                               T *__restrict__ GH, long long o)
+__device__ __forceinline__ void adj_stencil(const AdjAt<T> &A, const StepParams<T, S> &P, const AdjXw<T> &X, int i,
+                                            bool wall, T *mu)
 {
-    const AdjPop<p, T, S> A{LX, LY, LZ, P, R, nfx, nfc};
-    GH[(long long)(side * NPOP + p) * P.ny * P.nz + o] = A.ghost(side);
-    if constexpr (p + 1 < NPOP) adj_ghost_pops<T, S, p + 1>(LX, LY, LZ, P, R, nfx, nfc, side, GH, o);
-}
-
-template <class T, class S>
-__global__ void __launch_bounds__(128) adj_ghost_kernel(const T *__restrict__ LX, const T *__restrict__ LY,
-                                                        const T *__restrict__ LZ, T *__restrict__ GH,
-                                                        const StepParams<T, S> P)
-{
-    const long long nyz = (long long)P.ny * P.nz;
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= 2 * nyz) return;
-    const int side = int(q / nyz);
-    const long long o = q % nyz;
-    const int j = int(o % P.ny) + 1, k = int(o / P.ny) + 1;
-    const AdjRows R = adj_rows(j, k, P.nx, P.ny, P.nz);
-    adj_ghost_pops<T, S>(LX, LY, LZ, P, R, adj_nface(0, P.nx, P.ny, P.nz), adj_nface(1, P.nx, P.ny, P.nz), side,
-                         GH, o);
-}
-
-// Transposed interpolation stencil of every population at one cell (the
-// part of mu that comes from the faces), stored population by population:
-// MU[p * ncell + cell], cell = ((k-1)*ny + (j-1))*nx + (i-1).
-template <class T, class S, int p, int pend>
-__device__ __forceinline__ void adj_stencil_pops(const T *__restrict__ LX, const T *__restrict__ LY,
-                                                 const T *__restrict__ LZ, const T *__restrict__ GH,
-                                                 const StepParams<T, S> &P, const AdjRows &R, int i, long long o,
-                                                 int Ix2, bool x2_anchor, long long nfx, long long nfc,
-                                                 T *__restrict__ MU, long long cc)
-{
-    constexpr int ax = cx(p);
-    // second column of the y / z faces: i + cx (periodic image, or none past a wall)
-    int i2 = 0;
+    constexpr int ax = cx(p), c = xrep(p) - 1;
+    const int nx = P.nx;
+    const AdjPop<p, T, S> a{A, P};
+    const T xs = a.xsum(), cs = a.colsum();
+    const T xl = __shfl_up_sync(0xffffffffu, xs, 1);
+    T m = (p == 0 ? T(0.5) : X.f[c]) * xs + (p == 0 ? T(0.5) : X.g[c]) * xl;
     if (ax) {
-        i2 = i + ax;
-        if (P.periodic_x) i2 = i2 < 1 ? P.nx : (i2 > P.nx ? 1 : i2);
-        else if (i2 < 1 || i2 > P.nx) i2 = 0;
+        const T cn = ax > 0 ? __shfl_down_sync(0xffffffffu, cs, 1) : __shfl_up_sync(0xffffffffu, cs, 1);
+        m += X.t[c < 2 ? c : 0] * cs;
+        // i + c_x is the periodic image, or past a wall, where there is none
+        if (P.periodic_x || (ax > 0 ? i < nx : i > 1)) m += X.n[c < 2 ? c : 0] * cn;
+    } else {
+        m += cs;
     }
-    const AdjPop<p, T, S> A{LX, LY, LZ, P, R, nfx, nfc};
-    T m = A.interior(i, Ix2, x2_anchor, i2);
-    if (!P.periodic_x && (i <= 2 || i >= P.nx - 1)) {
-        // wall ghosts: g0 = q0 fb1 + (1-q0) fb2, g_{nx+1} = q1 fb_nx + (1-q1) fb_{nx-1}
-        const long long nyz = (long long)P.ny * P.nz;
-        const T g0 = GH[(long long)p * nyz + o], g1 = GH[(long long)(NPOP + p) * nyz + o];
+    if (wall) {
+        // the ghost columns: the other column of the x faces 0 and nx, and of the y and z
+        // faces at column 1 (c_x > 0) and nx (c_x < 0)
+        T g0 = adj_xw(P, p, 0, 1) * xl, g1 = adj_xw(P, p, nx, 1) * xs;
+        if (ax > 0) g0 += adj_tw(P, p, 1, 1) * cs;
+        if (ax < 0) g1 += adj_tw(P, p, nx, 1) * cs;
+        const T g0n = __shfl_up_sync(0xffffffffu, g0, 1), g1n = __shfl_down_sync(0xffffffffu, g1, 1);
+        // g0 = q0 fb1 + (1-q0) fb2, g_{nx+1} = q1 fb_nx + (1-q1) fb_{nx-1}
         if (i == 1) m += P.q0 * g0;
-        if (i == 2) m += (T(1) - P.q0) * g0;
-        if (i == P.nx) m += P.q1 * g1;
-        if (i == P.nx - 1) m += (T(1) - P.q1) * g1;
+        if (i == 2) m += (T(1) - P.q0) * g0n;
+        if (i == nx) m += P.q1 * g1;
+        if (i == nx - 1) m += (T(1) - P.q1) * g1n;
     }
-    MU[(long long)p * nfc + cc] = m;
-    if constexpr (p + 1 < pend)
-        adj_stencil_pops<T, S, p + 1, pend>(LX, LY, LZ, GH, P, R, i, o, Ix2, x2_anchor, nfx, nfc, MU, cc);
-}
-
-// Transposed stencil pass of the gather, split from the stage-(a) transpose so
-// that it runs with few registers and many warps in flight (it is bound by
-// the latency of its ~250 scattered loads per cell).  The populations are
-// split into four groups, one per block (blockIdx.z = plane * 4 + group), so
-// that each thread carries a quarter of the loads.
-template <class T, class S>
-__global__ void __launch_bounds__(128, 12) adj_stencil_kernel(const T *__restrict__ LX, const T *__restrict__ LY,
-                                                             const T *__restrict__ LZ, const T *__restrict__ GH,
-                                                             T *__restrict__ MU, const StepParams<T, S> P)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z / 4 + 1, grp = blockIdx.z % 4;
-    if (i > P.nx || j > P.ny) return;
-    const AdjRows R = adj_rows(j, k, P.nx, P.ny, P.nz);
-    const long long nfx = adj_nface(0, P.nx, P.ny, P.nz), nfc = adj_nface(1, P.nx, P.ny, P.nz);
-    // second x face holding column i: face i-1 ("other" column), face 0 (anchor) at a wall,
-    // face nx ("other") for i = 1 when periodic
-    const bool wall1 = !P.periodic_x && i == 1;
-    const int Ix2 = i == 1 ? (P.periodic_x ? P.nx : 0) : i - 1;
-    const long long o = (long long)(k - 1) * P.ny + (j - 1);
-    const long long cc = adj_cell(i, j, k, P.nx, P.ny);
-    if (grp == 0) adj_stencil_pops<T, S, 0, 5>(LX, LY, LZ, GH, P, R, i, o, Ix2, wall1, nfx, nfc, MU, cc);
-    else if (grp == 1) adj_stencil_pops<T, S, 5, 10>(LX, LY, LZ, GH, P, R, i, o, Ix2, wall1, nfx, nfc, MU, cc);
-    else if (grp == 2) adj_stencil_pops<T, S, 10, 15>(LX, LY, LZ, GH, P, R, i, o, Ix2, wall1, nfx, nfc, MU, cc);
-    else adj_stencil_pops<T, S, 15, NPOP>(LX, LY, LZ, GH, P, R, i, o, Ix2, wall1, nfx, nfc, MU, cc);
+    mu[p] = m;
+    if constexpr (p + 1 < NPOP) adj_stencil<T, S, p + 1>(A, P, X, i, wall, mu);
 }
 
 // mu = 4/3 lam' + (G^T L^T lamv); lam = (dA/df)^T mu - 1/3 lam'.
@@ -586,24 +548,59 @@ __device__ __forceinline__ T xface_share(const StepParams<T, S> &P, int I, int g
     return T(0.5) * (T(i1 == gi) + T(i2 == gi));
 }
 
+// The transposed stencil, the stage-(a) transpose and dJ/dphi of a cell.  A warp takes
+// the columns of one row, run on into the rows below it (so that a row length that is no
+// multiple of a warp leaves no lanes idle); the outermost lanes only form the sums their
+// neighbours need.
+// Bound by the latency of the face values' loads (128 registers: 16 warps per SM).  FP32,
+// 128 x 96 x 96 channel: 199 us, and 15 us less without a kernel for the wall ghosts; as two
+// kernels that formed the neighbours' sums again and handed the 19 sums over in memory
+// 221 us.  A row per warp beats the populations of a row over four warps (240 us: the row
+// addresses formed four times), 16 warps per SM beat 12 and 20, adjacent rows in a CTA
+// beat one row (they share the rows between them in L1).
+constexpr int kAdjRows = 4;                                                      // warps, on adjacent rows, of a CTA
+__host__ __device__ inline int adj_halo(int periodic_x) { return periodic_x ? 1 : 2; }  // lanes below the first cell
+__host__ __device__ inline int adj_cols(int periodic_x) { return 31 - adj_halo(periodic_x); }
+
 template <class T, class S>
-__global__ void __launch_bounds__(128) adj_gather_kernel(const S *__restrict__ f, const S *__restrict__ lam_next,
-                                                         const T *__restrict__ LX, const T *__restrict__ LY,
-                                                         const T *__restrict__ LZ, S *__restrict__ lam_out,
-                                                         const T *__restrict__ LFX, const T *__restrict__ LFY,
-                                                         const T *__restrict__ LFZ, double *__restrict__ dphi,
-                                                         const T *__restrict__ MU, const StepParams<T, S> P)
+__global__ void __launch_bounds__(32 * kAdjRows, 4)
+    adj_cell_kernel(const S *__restrict__ f, const S *__restrict__ lam_next, const T *__restrict__ LX,
+                    const T *__restrict__ LY, const T *__restrict__ LZ, S *lam_out,
+                    const T *__restrict__ LFX, const T *__restrict__ LFY, const T *__restrict__ LFZ,
+                    double *__restrict__ dphi, const StepParams<T, S> P)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z + 1;
-    if (i > P.nx || j > P.ny) return;
-    const long long c = ((long long)(k - 1) * P.ny + (j - 1)) * P.pitch + (i - 1);
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, k = blockIdx.y + 1;
+    // position of the lane in the sequence of the rows wp + 1, wp + 1 + kAdjRows, ..., each
+    // of nx + 2 columns
+    const int lo = adj_halo(P.periodic_x);
+    const int s = max(int(blockIdx.x) * adj_cols(P.periodic_x) + lane - (lo - 1), 0), m = s / (P.nx + 2), i = s - m * (P.nx + 2);
+    const int jr = m * kAdjRows + wp + 1, j = min(jr, P.ny);
+    const bool out = lane >= lo && lane < 31 && i >= 1 && i <= P.nx && jr <= P.ny;
+    const long long c = ((long long)(k - 1) * P.ny + (j - 1)) * P.pitch + (min(max(i, 1), P.nx) - 1);
     T mu[NPOP];
     {
-        const long long nfc = adj_nface(1, P.nx, P.ny, P.nz), cc = adj_cell(i, j, k, P.nx, P.ny);
+        // x face and column whose sums the lane forms: its own, or the periodic image at the ends
+        const int nx = P.nx, per = P.periodic_x;
+        const int cf = adj_xcol(i == 0 ? (per ? nx : 0) : min(i, nx), nx);
+        const int cc = adj_col((i == 0 ? (per ? nx : 1) : (i == nx + 1 && per ? 1 : min(i, nx))) - 1);
+        const int ic = min(max(i, 1), nx);
+        AdjXw<T> X;
 #pragma unroll
-        for (int p = 0; p < NPOP; ++p) mu[p] = T(4.0 / 3.0) * T(lam_next[p * P.ps + c]) + MU[p * nfc + cc];
+        for (int c = 0; c < 3; ++c) {
+            X.f[c] = adj_xw(P, c + 1, ic, 0);
+            X.g[c] = adj_xw(P, c + 1, ic == 1 ? (per ? nx : 0) : ic - 1, !per && ic == 1 ? 0 : 1);
+        }
+        X.t[0] = adj_tw(P, 1, ic, 0);
+        X.t[1] = adj_tw(P, 2, ic, 0);
+        X.n[0] = adj_tw(P, 1, ic == nx ? (per ? 1 : nx) : ic + 1, 1);
+        X.n[1] = adj_tw(P, 2, ic == 1 ? (per ? nx : 1) : ic - 1, 1);
+        const AdjAt<T> A = adj_at(LX, LY, LZ, j, k, cf, cc, nx, P.ny, P.nz);
+        const bool wall = !per && __any_sync(0xffffffffu, i <= 2 || i >= nx - 1);
+        adj_stencil<T, S>(A, P, X, i, wall, mu);
     }
+    if (!out) return;
+#pragma unroll
+    for (int p = 0; p < NPOP; ++p) mu[p] = T(4.0 / 3.0) * T(lam_next[p * P.ps + c]) + mu[p];
     // stage (a) transpose at this cell
     T v[NPOP];
 #pragma unroll

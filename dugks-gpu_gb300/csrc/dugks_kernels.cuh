@@ -987,9 +987,12 @@ __host__ __device__ constexpr bool face_pairs_ok()
 }
 static_assert(face_pairs_ok(), "face population pairs of face_tri_x2 must share their stencil shape");
 
+// om a + m b.  OF: the product om a is the one inside the fused operation, as the compiler
+// contracts face_tri's scalar lerps (the adjoint's face values), else m b (the forward's).
+template <bool OF = false>
 __device__ __forceinline__ float2 lerp_x2(float2 om, float2 m, float2 a, float2 b)
 {
-    return __ffma2_rn(m, b, __fmul2_rn(om, a));
+    return OF ? __ffma2_rn(om, a, __fmul2_rn(m, b)) : __ffma2_rn(m, b, __fmul2_rn(om, a));
 }
 
 // b - a for a stored 16-bit value b and a float a, in one mixed-precision
@@ -1014,7 +1017,7 @@ __device__ __forceinline__ float sub_stored(__nv_bfloat16 b, float a)
 // instructions per pair of values instead of four widenings and two packed
 // products); this uses om = 1 - m, which the weight tables hold to the last
 // bit of FP32.
-template <class S>
+template <class S, bool OF>
 __device__ __forceinline__ float2 lerp_first_x2(float2 om, float2 m, S ap, S aq, S bp, S bq)
 {
     if constexpr (sizeof(S) == 2) {
@@ -1022,7 +1025,7 @@ __device__ __forceinline__ float2 lerp_first_x2(float2 om, float2 m, S ap, S aq,
         return __ffma2_rn(m, make_float2(sub_stored(bp, af.x), sub_stored(bq, af.y)), af);
     } else {
         (void)om;
-        return lerp_x2(om, m, make_float2(ap, aq), make_float2(bp, bq));
+        return lerp_x2<OF>(om, m, make_float2(ap, aq), make_float2(bp, bq));
     }
 }
 
@@ -1031,7 +1034,7 @@ __device__ __forceinline__ float2 lerp_first_x2(float2 om, float2 m, S ap, S aq,
 // k where c_z > 0, at plane k+1 where c_z < 0.  An x or y face at plane k lies between
 // this at k and at k-1 (both populations of a stencil reach back one of the two), so the
 // march along z forms it once per plane and keeps the last one.
-template <class S, int AX, class RD>
+template <class S, int AX, bool OF = false, class RD>
 __device__ __forceinline__ void zpairs_x2(const StepParams<float, S> &P, const RD &R, int i, int j, int k, float2 N[5])
 {
     using RI = decltype(R.rb(0, 0));
@@ -1040,7 +1043,7 @@ __device__ __forceinline__ void zpairs_x2(const StepParams<float, S> &P, const R
     // first lerp of populations p, q between (row ra, column ca) and (row rb, column cb) of each
     auto L1 = [&](float2 om, float2 m, int p, int q, RI rap, int cap, RI raq, int caq, RI rbp, int cbp, RI rbq,
                   int cbq) {
-        return lerp_first_x2<S>(om, m, R.bits(p, rap, cap), R.bits(q, raq, caq), R.bits(p, rbp, cbp),
+        return lerp_first_x2<S, OF>(om, m, R.bits(p, rap, cap), R.bits(q, raq, caq), R.bits(p, rbp, cbp),
                                 R.bits(q, rbq, cbq));
     };
 #pragma unroll
@@ -1063,7 +1066,7 @@ __device__ __forceinline__ void zpairs_x2(const StepParams<float, S> &P, const R
             N[t] = L1(om, m, p, q, r0, A, s0, A, r0, B, s0, B);
             if (cy(p)) {
                 const RI r1 = R.rb(j - cy(p), kp), s1 = R.rb(j - cy(q), kq);
-                N[t] = lerp_x2(ty_o, ty_m, N[t], L1(om, m, p, q, r1, A, s1, A, r1, B, s1, B));
+                N[t] = lerp_x2<OF>(ty_o, ty_m, N[t], L1(om, m, p, q, r1, A, s1, A, r1, B, s1, B));
             }
         } else {
             const float2 yo = make_float2(P.yn_om[p], P.yn_om[q]), ym = make_float2(P.yn_m[p], P.yn_m[q]);
@@ -1073,7 +1076,7 @@ __device__ __forceinline__ void zpairs_x2(const StepParams<float, S> &P, const R
                 const float2 tx_o = make_float2(__ldg(tw + 2 * xs), __ldg(tw + 4 * xs));
                 const float2 tx_m = make_float2(__ldg(tw + 3 * xs), __ldg(tw + 5 * xs));
                 const int ip = i - cx(p), iq = i - cx(q);
-                N[t] = lerp_x2(yo, ym, L1(tx_o, tx_m, p, q, rA, i, sA, i, rA, ip, sA, iq),
+                N[t] = lerp_x2<OF>(yo, ym, L1(tx_o, tx_m, p, q, rA, i, sA, i, rA, ip, sA, iq),
                                L1(tx_o, tx_m, p, q, rB, i, sB, i, rB, ip, sB, iq));
             } else {
                 N[t] = L1(yo, ym, p, q, rA, i, sA, i, rB, i, sB, i);
@@ -1084,7 +1087,7 @@ __device__ __forceinline__ void zpairs_x2(const StepParams<float, S> &P, const R
 
 // 19 values of an x (AX = 0) or y (AX = 1) face; old: zpairs_x2 of plane k-1, becomes
 // that of plane k.
-template <class S, int AX, class RD>
+template <class S, int AX, bool OF = false, class RD>
 __device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const RD &R, int i, int j, int k,
                                             float2 old[5], float v[NPOP])
 {
@@ -1099,7 +1102,7 @@ __device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const
     };
     auto L1 = [&](float2 om, float2 m, int p, int q, RI rap, int cap, RI raq, int caq, RI rbp, int cbp, RI rbq,
                   int cbq) {
-        return lerp_first_x2<S>(om, m, R.bits(p, rap, cap), R.bits(q, raq, caq), R.bits(p, rbp, cbp),
+        return lerp_first_x2<S, OF>(om, m, R.bits(p, rap, cap), R.bits(q, raq, caq), R.bits(p, rbp, cbp),
                                 R.bits(q, rbq, cbq));
     };
     if (AX == 0) {
@@ -1119,7 +1122,7 @@ __device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const
             float2 res = L1(om, m, p, q, r00, A, r00, A, r00, B, r00, B);
             if (cy(p)) {
                 const RI sp = R.rb(j - cy(p), k), sq = R.rb(j - cy(q), k);
-                res = lerp_x2(ty_o, ty_m, res, L1(om, m, p, q, sp, A, sq, A, sp, B, sq, B));
+                res = lerp_x2<OF>(ty_o, ty_m, res, L1(om, m, p, q, sp, A, sq, A, sp, B, sq, B));
             }
             put(p, res);
         }
@@ -1137,28 +1140,28 @@ __device__ __forceinline__ void face_tri_x2(const StepParams<float, S> &P, const
             const int ip = i - cx(p), iq = i - cx(q);
             const float2 yo = make_float2(P.yn_om[p], P.yn_om[q]), ym = make_float2(P.yn_m[p], P.yn_m[q]);
             if (cx(p))
-                put(p, lerp_x2(yo, ym, L1(tx_o, tx_m, p, q, rA, i, rA, i, rA, ip, rA, iq),
+                put(p, lerp_x2<OF>(yo, ym, L1(tx_o, tx_m, p, q, rA, i, rA, i, rA, ip, rA, iq),
                                L1(tx_o, tx_m, p, q, rB, i, rB, i, rB, ip, rB, iq)));
             else
                 put(p, L1(yo, ym, p, q, rA, i, rA, i, rB, i, rB, i));
         }
     }
     float2 N[5];
-    zpairs_x2<S, AX>(P, R, i, j, k, N);
+    zpairs_x2<S, AX, OF>(P, R, i, j, k, N);
 #pragma unroll
     for (int t = 0; t < 5; ++t) {
         const int p = t == 0 ? 5 : 9 + 2 * t, q = p + 1;
         // plane k, and plane k - c_z of each
         const float2 a = make_float2(cz(p) > 0 ? N[t].x : old[t].x, cz(q) > 0 ? N[t].y : old[t].y);
         const float2 b = make_float2(cz(p) > 0 ? old[t].x : N[t].x, cz(q) > 0 ? old[t].y : N[t].y);
-        put(p, lerp_x2(tz_o, tz_m, a, b));
+        put(p, lerp_x2<OF>(tz_o, tz_m, a, b));
         old[t] = N[t];
     }
 }
 
 // Plane k's part of the z faces below and above it: every population interpolated in x
 // and y at column i, row j.
-template <class S, class RD>
+template <class S, bool OF = false, class RD>
 __device__ __forceinline__ void plane_z_x2(const StepParams<float, S> &P, const RD &R, int i, int j, int k, float Y[NPOP])
 {
     using RI = decltype(R.rb(0, 0));
@@ -1176,16 +1179,16 @@ __device__ __forceinline__ void plane_z_x2(const StepParams<float, S> &P, const 
         const RI sp = R.rb(j - cy(p), k), sq = R.rb(j - cy(q), k);
         // value at column i of rows rp / rq, x-lerped when c_x != 0 (first lerps)
         auto xl = [&](RI rp, RI rq) {
-            return lerp_first_x2<S>(tx_o, tx_m, R.bits(p, rp, i), R.bits(q, rq, i), R.bits(p, rp, i - cx(p)),
+            return lerp_first_x2<S, OF>(tx_o, tx_m, R.bits(p, rp, i), R.bits(q, rq, i), R.bits(p, rp, i - cx(p)),
                                     R.bits(q, rq, i - cx(q)));
         };
         float2 y;
         if (ax && ay)
-            y = lerp_x2(ty_o, ty_m, xl(r, r), xl(sp, sq));
+            y = lerp_x2<OF>(ty_o, ty_m, xl(r, r), xl(sp, sq));
         else if (ax)
             y = xl(r, r);
         else if (ay)
-            y = lerp_first_x2<S>(ty_o, ty_m, R.bits(p, r, i), R.bits(q, r, i), R.bits(p, sp, i), R.bits(q, sq, i));
+            y = lerp_first_x2<S, OF>(ty_o, ty_m, R.bits(p, r, i), R.bits(q, r, i), R.bits(p, sp, i), R.bits(q, sq, i));
         else
             y = make_float2(R.raw(p, r, i), R.raw(q, r, i));
         Y[p] = y.x;
@@ -1194,7 +1197,7 @@ __device__ __forceinline__ void plane_z_x2(const StepParams<float, S> &P, const 
 }
 
 // 19 values of the z face between the planes with parts Y (below) and Z.
-template <class S, class RD>
+template <class S, bool OF = false, class RD>
 __device__ __forceinline__ void face_z_x2(const StepParams<float, S> &P, const RD &R, const float Y[NPOP],
                                           const float Z[NPOP], float v[NPOP])
 {
@@ -1208,7 +1211,7 @@ __device__ __forceinline__ void face_z_x2(const StepParams<float, S> &P, const R
         if (sizeof(S) == 2 && !cx(p) && !cy(p))  // its only lerp: as lerp_first_x2
             res = __ffma2_rn(zm, make_float2(b.x - a.x, b.y - a.y), a);
         else
-            res = lerp_x2(zo, zm, a, b);
+            res = lerp_x2<OF>(zo, zm, a, b);
         const float2 e = R.dec_e2(p, q, res);
         v[p] = e.x;
         v[q] = e.y;

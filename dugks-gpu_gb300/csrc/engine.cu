@@ -911,13 +911,10 @@ int adjoint_form(dg_ctx *h, int istep, const void *f_n, const void *lam_next, vo
     if (!std::is_same<T, S>::value) return h->fail(DG_ERR_UNSUPPORTED, "the adjoint exists for the fp64 and fp32 forms");
     if (h->recon != 0) return h->fail(DG_ERR_UNSUPPORTED, "the adjoint exists for the trilinear reconstruction");
     if (!h->adj) {
-        // 19 adjoint values and one dJ/dF (force-field face term) per face, the
-        // wall-ghost sums (2 * 19 per row and plane) and the transposed-stencil
-        // sums (19 per cell)
+        // 19 adjoint values and one dJ/dF (force-field face term) per face
         const long long n = adj_nface(0, h->nx, h->ny, h->nz) + 2 * adj_nface(1, h->nx, h->ny, h->nz);
-        const long long ng = 2LL * NPOP * h->ny * h->nz;
-        const long long nm = (long long)NPOP * h->ncell();
-        CK(cudaMalloc(&h->adj, (size_t(n) * (NPOP + 1) + size_t(ng) + size_t(nm)) * sizeof(T)),
+        const long long nl = adj_row(1, h->nz + 1, h->nx, h->ny);
+        CK(cudaMalloc(&h->adj, (3 * size_t(nl) + size_t(n)) * sizeof(T)),
            "cudaMalloc (adjoint scratch)");
     }
     if (h->ffield && !h->dphi) {

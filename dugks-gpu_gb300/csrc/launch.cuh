@@ -50,7 +50,7 @@ struct GradCfg<float> {
 // tile of the fused adjoint face kernel (TMA forms): W rows of 32 cells, box W+2 rows
 template <class T, class S>
 struct AdjCfg {
-    static constexpr int W = 7;       // 4 x 24.6 KB planes (FP32), two CTAs per SM
+    static constexpr int W = 8;       // 4 x 27.4 KB planes (FP32), two CTAs per SM
     static constexpr int MINB = 2;
 };
 
@@ -80,7 +80,7 @@ struct Kern {
     static cudaError_t moments_partials(const S *f, const StepParams<T, S> &P, double *partial, int nblocks,
                                         cudaStream_t st);
     // Adjoint of one step (adjoint_kernels.cuh): recomputes f-bar-plus of f_n into fb,
-    // per-face adjoints into lamv (T-typed scratch, adj_nface(0)+2*adj_nface(1) faces x 19),
+    // per-face adjoints into lamv (T-typed scratch: three face arrays of adj_row(1, nz + 1), then dJ/dF per face),
     // then lam_out = (dS/df)^T lam_next.  FP64 and FP32 forms only.
     // dphi (optional, FP64, dump order [k][j][i]): += dJ/dphi of this step when a force field is set;
     // tmap_adj: f-bar-plus tensor map with AdjCfg::W + 2 rows (TMA forms)

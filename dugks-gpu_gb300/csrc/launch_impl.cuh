@@ -226,8 +226,9 @@ cudaError_t Kern<T, S>::adjoint(const S *f_n, S *fb, const S *lam_next, S *lam_o
         cudaError_t e = fbar(f_n, fb, P, st);
         if (e != cudaSuccess) return e;
         const long long nfx = adj_nface(0, P.nx, P.ny, P.nz), nfc = adj_nface(1, P.nx, P.ny, P.nz);
-        T *LX = lamv, *LY = lamv + NPOP * nfx, *LZ = LY + NPOP * nfc;
-        T *LFX = LZ + NPOP * nfc, *LFY = LFX + nfx, *LFZ = LFY + nfc;  // per-face dJ/dF (force field)
+        const long long nl = adj_row(1, P.nz + 1, P.nx, P.ny);  // values of one face array
+        T *LX = lamv, *LY = lamv + nl, *LZ = LY + nl;
+        T *LFX = LZ + nl, *LFY = LFX + nfx, *LFZ = LFY + nfc;  // per-face dJ/dF (force field)
         if constexpr (TileCfg<T, S>::TMA) {
             // +x, +y, +z faces of every cell from the TMA-staged tile; x faces I = 0 apart
             if (!tmap_adj) return cudaErrorInvalidValue;
@@ -246,9 +247,10 @@ cudaError_t Kern<T, S>::adjoint(const S *f_n, S *fb, const S *lam_next, S *lam_o
             const int kchunk = choose_kchunk(P.nz, cols, (long long)device_sms() * std::max(occ, 1));
             dim3 grid((P.nx + 31) / 32, (P.ny + W - 1) / W, (P.nz + kchunk - 1) / kchunk);
             kern<<<grid, dim3(32, W), smem, st>>>(*tmap_adj, lam_next, LX, LY, LZ, LFX, LFY, LFZ, P, kchunk);
-            // one warp per block: the few wall faces spread over every SM
+            // between walls; one warp per block: the few wall faces spread over every SM
             const long long n0 = (long long)P.ny * P.nz;
-            adj_face_kernel<T, S, 0><<<unsigned((n0 + 31) / 32), 32, 0, st>>>(fb, lam_next, LX, LFX, P, 1);
+            if (!P.periodic_x)
+                adj_face_kernel<T, S, 0><<<unsigned((n0 + 31) / 32), 32, 0, st>>>(fb, lam_next, LX, LFX, P, 1);
         } else {
             adj_face_kernel<T, S, 0><<<unsigned((nfx + 127) / 128), 128, 0, st>>>(fb, lam_next, LX, LFX, P, 0);
             adj_face_kernel<T, S, 1><<<unsigned((nfc + 127) / 128), 128, 0, st>>>(fb, lam_next, LY, LFY, P, 0);
@@ -256,18 +258,9 @@ cudaError_t Kern<T, S>::adjoint(const S *f_n, S *fb, const S *lam_next, S *lam_o
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        T *GH = LFZ + nfc;  // wall-ghost sums, 2 * 19 * ny * nz
-        if (!P.periodic_x) {
-            const long long ng = 2LL * P.ny * P.nz;
-            adj_ghost_kernel<T, S><<<unsigned((ng + 31) / 32), 32, 0, st>>>(LX, LY, LZ, GH, P);
-        }
-        T *MU = GH + 2LL * NPOP * P.ny * P.nz;  // transposed-stencil sums, 19 * nx * ny * nz
-        // 128-thread blocks of whole warps over x (one to four rows when nx < 128), so
-        // that narrow grids leave no lanes idle
-        const int bx = P.nx >= 128 ? 128 : (P.nx + 31) / 32 * 32, by = 128 / bx;
-        const dim3 blk(bx, by), grid((P.nx + bx - 1) / bx, (P.ny + by - 1) / by, P.nz);
-        adj_stencil_kernel<T, S><<<dim3(grid.x, grid.y, 4 * P.nz), blk, 0, st>>>(LX, LY, LZ, GH, MU, P);
-        adj_gather_kernel<T, S><<<grid, blk, 0, st>>>(f_n, lam_next, LX, LY, LZ, lam_out, LFX, LFY, LFZ, dphi, MU, P);
+        const long long seq = (long long)((P.ny + kAdjRows - 1) / kAdjRows) * (P.nx + 2);
+        const dim3 grid(unsigned((seq - 2 + adj_cols(P.periodic_x) - 1) / adj_cols(P.periodic_x)), P.nz);
+        adj_cell_kernel<T, S><<<grid, 32 * kAdjRows, 0, st>>>(f_n, lam_next, LX, LY, LZ, lam_out, LFX, LFY, LFZ, dphi, P);
         return cudaGetLastError();
     }
 }
