@@ -7,8 +7,8 @@
 // exactly (its values have fewer bits than the fixed point) and rounded once when
 // written.  f-bar-plus, written and read by these two kernels only, is held in
 // fixed point.  Step of the 256 x 128 x 128 channel: 6.65 ms with the FP64 kernels,
-// 1.65 ms here (stage (a) 0.21, flux 1.45); 64^3 box 0.63 -> 0.18 ms, 64 x 32 x 32
-// channel 0.229 -> 0.078 ms.
+// 1.27 ms here (stage (a) 0.21, flux 1.06); 64^3 box 0.63 -> 0.104 ms, 64 x 32 x 32
+// channel 0.229 -> 0.037 ms.
 //
 // Error of the state against an 80-bit run of the same scheme (relative 2-norm):
 // 5e-17 after one step, the rounding of the stored values (FP64 kernels 2.4e-16 to
@@ -278,55 +278,69 @@ struct FxAt {
     }
 };
 
-// Transverse interpolation of every population at one cell for the faces normal to
-// AX: g[0..9] the populations that cross such a face, g[10..12] the sums over the
-// others of their values and tangential momenta (their normal weights are equal, so
-// the face needs the sums only).  A face value is then one interpolation between
-// the two cells across it: each cell's transverse values are formed once per axis
-// and used by both of its faces.
+// Population p interpolated within plane dz of A, transversely to the faces normal to AX.
 template <int AX>
-__device__ __forceinline__ i64 fx_interp(const FxParams &P, const FxAt &A, FxMul txp, FxMul txm, int p)
+__device__ __forceinline__ i64 fx_inplane(const FxParams &P, const FxAt &A, FxMul txp, FxMul txm, int p, int dz)
 {
-    const int ax = AX == 0 ? 0 : cx(p), ay = AX == 1 ? 0 : cy(p), az = AX == 2 ? 0 : cz(p);
+    const int ax = AX == 0 ? 0 : cx(p), ay = AX == 1 ? 0 : cy(p);
     const FxMul tx = ax > 0 ? txp : txm;
-    i64 a = A(p, 0, 0, 0);
-    if (ax) a = fx_lerp(a, A(p, -ax, 0, 0), tx);
+    i64 a = A(p, 0, 0, dz);
+    if (ax) a = fx_lerp(a, A(p, -ax, 0, dz), tx);
     if (ay) {
-        i64 b = A(p, 0, -ay, 0);
-        if (ax) b = fx_lerp(b, A(p, -ax, -ay, 0), tx);
+        i64 b = A(p, 0, -ay, dz);
+        if (ax) b = fx_lerp(b, A(p, -ax, -ay, dz), tx);
         a = fx_lerp(a, b, P.ty);
-    }
-    if (az) {
-        i64 b = A(p, 0, 0, -az);
-        if (ax) b = fx_lerp(b, A(p, -ax, 0, -az), tx);
-        if (ay) {
-            i64 c = A(p, 0, -ay, -az);
-            if (ax) c = fx_lerp(c, A(p, -ax, -ay, -az), tx);
-            b = fx_lerp(b, c, P.ty);
-        }
-        a = fx_lerp(a, b, P.tz);
     }
     return a;
 }
 
+// In-plane part of the z-moving populations at plane k (A's middle plane) where c_z > 0,
+// at k + 1 where c_z < 0.  A transverse value at plane k lies between this at k and at
+// k - 1 (both kinds reach back one of the two), so the march along z forms it once per
+// plane and keeps the last one.
+template <int AX>
+__device__ __forceinline__ void fx_zparts(const FxParams &P, const FxAt &A, FxMul txp, FxMul txm, i64 old[10])
+{
+#pragma unroll
+    for (int s = 0; s < 10; ++s) {
+        const int p = flux_pop(2, s);
+        old[s] = fx_inplane<AX>(P, A, txp, txm, p, cz(p) > 0 ? 0 : 1);
+    }
+}
+
 constexpr int FXG = 13;
 
-template <int AX>
-__device__ __forceinline__ void fx_cell_values(const FxParams &P, const FxAt &A, FxMul txp, FxMul txm, i64 g[FXG])
+// Transverse interpolation of every population at one cell for the faces normal to
+// AX: put(n, x), n = 0..9 the populations that cross such a face, n = 10..12 the sums over
+// the others of their values and tangential momenta (their normal weights are equal, so
+// the face needs the sums only).  A face value is then one interpolation between
+// the two cells across it: each cell's transverse values are formed once per axis
+// and used by both of its faces.  AX < 2, old: fx_zparts of plane k - 1, becomes that of k.
+template <int AX, class Put>
+__device__ __forceinline__ void fx_cell_values(const FxParams &P, const FxAt &A, FxMul txp, FxMul txm, i64 *old, Put put)
 {
     constexpr int T1 = AX == 0 ? 1 : 0, T2 = AX == 2 ? 1 : 2;
-#pragma unroll
-    for (int s = 0; s < 10; ++s) g[s] = fx_interp<AX>(P, A, txp, txm, flux_pop(AX, s));
-    g[10] = A(0, 0, 0, 0);
-    g[11] = g[12] = 0;
+    i64 m[3] = {A(0, 0, 0, 0), 0, 0};
 #pragma unroll
     for (int p = 1; p < NPOP; ++p) {
-        if (cc(AX, p)) continue;
-        const i64 x = fx_interp<AX>(P, A, txp, txm, p);
-        g[10] += x;
-        if (cc(T1, p)) g[11] += cc(T1, p) > 0 ? x : -x;
-        if (cc(T2, p)) g[12] += cc(T2, p) > 0 ? x : -x;
+        const bool z = AX < 2 && cz(p) != 0;
+        i64 x = fx_inplane<AX>(P, A, txp, txm, p, z && cz(p) < 0 ? 1 : 0);
+        if (z) {
+            i64 &o = old[flux_slot(2, p) < 0 ? 0 : flux_slot(2, p)];
+            const i64 n = x;
+            x = cz(p) > 0 ? fx_lerp(n, o, P.tz) : fx_lerp(o, n, P.tz);
+            o = n;
+        }
+        if (cc(AX, p)) {
+            put(flux_slot(AX, p), x);
+            continue;
+        }
+        m[0] += x;
+        if (cc(T1, p)) m[1] += cc(T1, p) > 0 ? x : -x;
+        if (cc(T2, p)) m[2] += cc(T2, p) > 0 ? x : -x;
     }
+#pragma unroll
+    for (int s = 0; s < 3; ++s) put(10 + s, m[s]);
 }
 
 // face value of crossing population p between the lower cell's a and the upper cell's b
@@ -336,56 +350,73 @@ __device__ __forceinline__ i64 fx_normal(int s, i64 a, i64 b, FxMul mp, FxMul mm
     return cc(AX, flux_pop(AX, s)) > 0 ? fx_lerp(a, b, mp) : fx_lerp(b, a, mm);
 }
 
-template <int W>
-constexpr size_t flux_fx_smem_bytes()
+// shared memory of flux_fx_kernel, in elements
+template <int R>
+struct FxSmem {
+    static constexpr int GX = 0, GY = GX + R * FXG * 34, YS = GY + (R + 2) * FXG * 32, XZ = YS + 2 * (R + 1) * 10 * 32,
+                         X0 = XZ + 2 * R * 4 * 33, DZ = X0 + 2 * R * 6, GZ = DZ + 2 * R * 4 * 32, N = GZ + R * FXG * 32;
+    static constexpr size_t bytes = sizeof(i64) * size_t(N);
+};
+
+// barrier of one group of warps
+__device__ __forceinline__ void fx_bar(int id, int threads)
 {
-    return sizeof(i64) * size_t((W - 1) * FXG * 34 + (W + 1) * FXG * 32 + W * 10 * 32 + (W - 1) * 10);
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// Stages (b)-(e).  A CTA is W warps: warps 1..W-1 one row of 32 cells each (lane =
-// x), marching a chunk of z planes; warp 0 is the halo.  Per plane:
-//   1. every warp forms its cells' transverse values for x and y faces and
-//      publishes them in shared memory (gx, gy); the halo warp those of the rows
-//      below and above the tile and of the columns left and right of it;
-//   2. after a barrier every thread evaluates its +x, +z and +y faces, the halo
-//      warp the -y faces of the first row and the -x faces of the first column; y
-//      fluxes are published (ysh), the -x flux comes from lane-1;
-//   3. after a second barrier the cells are updated.
-// The transverse values and flux of the z faces are carried from plane to plane in
-// registers.
-template <int W, int MINB, int FAX>
-__global__ void __launch_bounds__(32 * W, MINB) flux_fx_kernel(const i64 *__restrict__ fb, const double *f_in,
-                                                               double *f_out, const FxParams P, int kchunk,
-                                                               const int *flag)
+// Stages (b)-(e).  A CTA holds R rows of 32 cells (lane = x) and marches a chunk of z
+// planes.  Each axis has warps of its own: R + 1 for x (the last one, the halo warp, the
+// columns left and right of the tile), R + 2 for y (the rows -1 .. R), R for z.  Per plane:
+//   1. every warp forms its cells' transverse values; those of x and y are published in
+//      shared memory (gx, gy), those of z carried from plane to plane in registers;
+//   2. after a barrier of the axis' own warps it evaluates its faces (x: +x, the halo warp
+//      -x of the first column; y: the face below its row; z: +z) and publishes the fluxes
+//      that other warps need;
+//   3. after a barrier of the CTA the x, y and z warp of a row update a third of its
+//      populations each: those whose flux differences they hold, so that four of the ten
+//      fluxes of an axis cross over (fxz, ysh, dzs; double-buffered, read until the
+//      next such barrier).
+// Bound by latency: with one warp per row doing all of it (values of all three axes and
+// z carries in registers) the loads' latency showed between spills, issue 33 %; split by
+// axis a thread carries few values, three times the warps share a tile and their phases
+// overlap, issue 40 %, ALU pipe 40 %.  256 x 128 x 128 channel: 1.45 -> 1.06 ms; 64 x 32 x
+// 32: a step 78 -> 37 us.  R = 4 (15 warps, no spills at 128 registers); R = 7 (24 warps,
+// 80 registers) 1.01 ms there but 43 us at 64 x 32 x 32; R = 5, 6 (five and six warps on
+// some schedulers) 1.2 to 1.3 ms.  Waits split into arrive and wait (mbarriers), with the
+// next plane's values in between, were slower (1.5 ms), and so was an even split of all
+// planes over one CTA per SM (1.09 ms: tiles next to each other, at different planes, no
+// longer share rows in L2).
+template <int R, int MINB, int FAX>
+__global__ void __launch_bounds__(32 * (3 * R + 3), MINB) flux_fx_kernel(const i64 *__restrict__ fb, const double *f_in,
+                                                                         double *f_out, const FxParams P, const int *flag)
 {
-    constexpr int R = W - 1;
+    using L = FxSmem<R>;
     extern __shared__ __align__(16) i64 sm[];
-    i64(*gx)[FXG][34] = reinterpret_cast<i64(*)[FXG][34]>(sm);
-    i64(*gy)[FXG][32] = reinterpret_cast<i64(*)[FXG][32]>(sm + R * FXG * 34);
-    i64(*ysh)[10][32] = reinterpret_cast<i64(*)[10][32]>(sm + R * FXG * 34 + (R + 2) * FXG * 32);
-    i64(*xsh)[10] = reinterpret_cast<i64(*)[10]>(sm + R * FXG * 34 + (R + 2) * FXG * 32 + (R + 1) * 10 * 32);
+    i64(*gx)[FXG][34] = reinterpret_cast<i64(*)[FXG][34]>(sm + L::GX);               // [row]
+    i64(*gy)[FXG][32] = reinterpret_cast<i64(*)[FXG][32]>(sm + L::GY);               // [row + 1]
+    i64(*ysh)[R + 1][10][32] = reinterpret_cast<i64(*)[R + 1][10][32]>(sm + L::YS);  // [parity][face below row]
+    i64(*fxz)[R][4][33] = reinterpret_cast<i64(*)[R][4][33]>(sm + L::XZ);            // x fluxes of populations 11..14
+    i64(*xs0)[R][6] = reinterpret_cast<i64(*)[R][6]>(sm + L::X0);                    // -x fluxes of the first column, 1, 2, 7..10
+    i64(*dzs)[R][4][32] = reinterpret_cast<i64(*)[R][4][32]>(sm + L::DZ);            // z differences of populations 15..18
     if (*flag) return;  // a value out of range: the step is redone in FP64
 
     const int lane = threadIdx.x, wr = threadIdx.y;
     const int nx = P.nx, ny = P.ny, nz = P.nz, xs = nx + 2;
-    const int c0 = blockIdx.x * 32;            // first column of the tile (0-based cell)
-    const int j0 = blockIdx.y * R;             // first row
-    const int kb = blockIdx.z * kchunk, ke = min(kb + kchunk, nz);
-    if (kb >= ke) return;
     const long long plane = (long long)ny * P.rs;
     auto wrap = [](int a, int n) { return a < 0 ? a + n : (a >= n ? a - n : a); };
     auto wrapc = [&](int a, int n) { a = wrap(a, n); return a < n ? a : n - 1; };  // rows past a ragged last tile: any valid row
-    auto rows = [&](FxAt &A, int j) {
+    FxAt A;
+    auto rows = [&](int j) {
         A.row[0] = wrap(j - 1, ny) * P.rs;
         A.row[1] = j * P.rs;
         A.row[2] = wrap(j + 1, ny) * P.rs;
     };
-    auto cols = [&](FxAt &A, int c) {  // c = -1 .. nx (ghost columns at nx + 1 and nx)
+    auto cols = [&](int c) {  // c = -1 .. nx (ghost columns at nx + 1 and nx)
         A.col[0] = fx_col(c <= 0 ? nx + 1 : c - 1);
         A.col[1] = fx_col(c < 0 ? nx + 1 : c);
         A.col[2] = fx_col(min(c + 1, nx));
     };
-    auto planes = [&](FxAt &A, int k) {  // k = -1 .. nz
+    auto planes = [&](int k) {  // k = -1 .. nz
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             int q = k + d - 1;
@@ -397,167 +428,215 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_fx_kernel(const i64 *__rest
         const int2 m = __ldg(reinterpret_cast<const int2 *>(P.tab) + row * xs + I);
         return FxMul{m.x, m.y};
     };
-
-    const int gc = c0 + lane, gj = j0 + wr - 1;
-    const bool cell = wr >= 1 && gc < nx && gj < ny;
-    const int cc1 = min(gc, nx - 1);
-    const FxMul txp = at_x(cc1 + 1, FXT_TXP), txm = at_x(cc1 + 1, FXT_TXM);
-    const int row = wr == 0 ? wrap(j0 - 1, ny) : wrapc(gj, ny);
-    // cell whose x-face values the thread forms: its own; in the halo warp, lane by
-    // lane, the column left of the tile (lanes 0..R-1) and the one right of it
-    const int hs = lane >= R, hr = hs ? lane - R : lane;
-    const int xcol = wr ? min(gc, nx) : (hs ? min(c0 + 32, nx) : c0 - 1);
-    const int xrow = wr ? row : wrapc(j0 + min(hr, R - 1), ny);
-    i64 *gxw = &gx[wr ? wr - 1 : min(hr, R - 1)][0][wr ? lane + 1 : (hs ? 33 : 0)];
-    const bool gxs = wr || lane < 2 * R;
-    // x face the thread evaluates: I (between 1-based columns I and I+1) of tile row
-    // xr; a lane past the last column takes that column's face, a valid one
-    const int I = wr ? min(gc + 1, nx) : c0, xr = wr ? wr - 1 : min(lane, R - 1);
-    FxAt A;
-    i64 gzA[FXG], fz[10];
-
-    // z face between the planes holding a (below) and the one whose values b are given
-    auto z_face = [&](const i64 a[FXG], const i64 b[FXG], i64 v[10]) {
-        i64 m[3];
-#pragma unroll
-        for (int s = 0; s < 10; ++s) v[s] = fx_normal<2>(s, a[s], b[s], P.mz, P.mz);
-#pragma unroll
-        for (int s = 0; s < 3; ++s) m[s] = (a[10 + s] + b[10 + s]) >> 1;
-        fx_face_flux<2, FAX>(P, v, m);
-    };
-    auto y_face = [&](int r, i64 v[10]) {  // between tile rows r - 1 (gy[r]) and r
-        i64 m[3];
-#pragma unroll
-        for (int s = 0; s < 10; ++s) v[s] = fx_normal<1>(s, gy[r][s][lane], gy[r + 1][s][lane], P.my, P.my);
-#pragma unroll
-        for (int s = 0; s < 3; ++s) m[s] = (gy[r][10 + s][lane] + gy[r + 1][10 + s][lane]) >> 1;
-        fx_face_flux<1, FAX>(P, v, m);
-    };
-    // x face I (between 1-based cells I and I+1) of tile row r, gx columns q and q + 1
-    auto x_face = [&](int I, int r, int q, const i64 *row, i64 v[10]) {
-        i64 m[3];
-        const FxMul mp = at_x(I, FXT_MP), mm = at_x(I, FXT_MM);
-#pragma unroll
-        for (int s = 0; s < 10; ++s) v[s] = fx_normal<0>(s, gx[r][s][q], gx[r][s][q + 1], mp, mm);
-        if (P.stretched) {
-            // weight 1/2 + d on the upper cell, except for the rest population (1/2)
-            const FxMul d = at_x(I, FXT_D0);
-            const i64 rest = __ldg(row + fx_col(I)) - __ldg(row + fx_col(I == 0 ? nx + 1 : I - 1));
-#pragma unroll
-            for (int s = 0; s < 3; ++s) {
-                const i64 a = gx[r][10 + s][q], b = gx[r][10 + s][q + 1];
-                m[s] = fx_mad(b - a - (s == 0 ? rest : 0), d, (a + b) >> 1);
-            }
-        } else {
-#pragma unroll
-            for (int s = 0; s < 3; ++s) m[s] = (gx[r][10 + s][q] + gx[r][10 + s][q + 1]) >> 1;
-        }
-        if (!P.periodic_x) {
-            // bounce-back on the walls: populations entering the fluid take their opposites' values
-            if (I == 0) {
-                v[0] = v[1]; v[2] = v[5]; v[4] = v[3]; v[6] = v[9]; v[8] = v[7];
-            }
-            if (I == nx) {
-                v[1] = v[0]; v[5] = v[2]; v[3] = v[4]; v[9] = v[6]; v[7] = v[8];
-            }
-        }
-        fx_face_flux<0, FAX>(P, v, m);
+    const int c0 = blockIdx.x * 32;  // first column of the tile (0-based cell)
+    const int j0 = blockIdx.y * R;   // first row
+    const int kb = int((long long)nz * blockIdx.z / gridDim.z), ke = int((long long)nz * (blockIdx.z + 1) / gridDim.z);
+    const int gc = c0 + lane, cc1 = min(gc, nx - 1);
+    // f = 4/3 f-bar-plus - 1/3 f (less the flux differences) of population p of the cell at A
+    auto base = [&](int p, long long c) {
+        const i64 b = A(p, 0, 0, 0);
+        return fx_madr(b - fx_from_double(f_in[p * P.ps + c]), P.third, b);
     };
 
-    // plane k's f-bar-plus rows of the tile and f-tilde into L2 (halo warp), two planes ahead of use
-    auto prefetch = [&](int k) {
-        const int q = wrap(k, nz);
-        if (lane < R + 2)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(fb + q * plane + wrapc(wrap(j0 - 1 + lane, ny), ny) * (long long)P.rs + fx_col(c0)),
-                         "r"(unsigned(min(2, (P.pitch_b - c0) >> 4) * NPOP * 16 * 8)));
-        if (k < ke)
-            for (int t = lane; t < NPOP * R * 2; t += 32) {
-                const int p = t / (2 * R), r = (t >> 1) % R;
-                const long long o = p * P.ps + ((long long)k * ny + min(j0 + r, ny - 1)) * P.pitch + min(c0 + 16 * (t & 1), nx - 1);
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(f_in + o));
+    if (wr <= R) {
+        // --- x: cell whose values the thread forms: its own; in the halo warp, lane by
+        // lane, the column left of the tile (lanes 0..R-1) and the one right of it
+        const bool halo = wr == R;
+        const int hs = lane >= R, hr = min(hs ? lane - R : lane, R - 1);
+        const int row = wrapc(j0 + (halo ? hr : wr), ny);
+        const int r = halo ? hr : wr;
+        i64 *gxw = &gx[r][0][halo ? (hs ? 33 : 0) : lane + 1];
+        const bool gxs = !halo || lane < 2 * R;
+        // x face the thread evaluates: I (between 1-based columns I and I+1) of tile row
+        // xr; a lane past the last column takes that column's face, a valid one
+        const int I = halo ? c0 : min(gc + 1, nx), xr = halo ? min(lane, R - 1) : wr, q = I - c0;
+        const FxMul mp = at_x(I, FXT_MP), mm = at_x(I, FXT_MM), cxm = at_x(cc1 + 1, FXT_CX);
+        const bool cell = !halo && gc < nx && j0 + wr < ny;
+        const int restrow = wrapc(j0 + xr, ny) * P.rs;
+        rows(row);
+        cols(halo ? (hs ? min(c0 + 32, nx) : c0 - 1) : min(gc, nx));
+        i64 old[10];
+        planes(kb - 1);
+        fx_zparts<0>(P, A, FxMul{}, FxMul{}, old);
+        for (int k = kb; k < ke; ++k) {
+            planes(k);
+            fx_cell_values<0>(P, A, FxMul{}, FxMul{}, old, [&](int n, i64 x) {
+                if (gxs) gxw[n * 34] = x;
+            });
+            fx_bar(1, 32 * (R + 1));
+            i64 v[10], m[3];
+#pragma unroll
+            for (int s = 0; s < 10; ++s) v[s] = fx_normal<0>(s, gx[xr][s][q], gx[xr][s][q + 1], mp, mm);
+            if (P.stretched) {
+                // weight 1/2 + d on the upper cell, except for the rest population (1/2)
+                const FxMul d = at_x(I, FXT_D0);
+                const i64 *rr = A.pl[1] + restrow;
+                const i64 rest = __ldg(rr + fx_col(I)) - __ldg(rr + fx_col(I == 0 ? nx + 1 : I - 1));
+#pragma unroll
+                for (int s = 0; s < 3; ++s) {
+                    const i64 a = gx[xr][10 + s][q], b = gx[xr][10 + s][q + 1];
+                    m[s] = fx_mad(b - a - (s == 0 ? rest : 0), d, (a + b) >> 1);
+                }
+            } else {
+#pragma unroll
+                for (int s = 0; s < 3; ++s) m[s] = (gx[xr][10 + s][q] + gx[xr][10 + s][q + 1]) >> 1;
             }
-    };
-    // two rounds ahead of the first plane for the z values and flux below it
-    for (int k = kb - 2; k < ke; ++k) {
-        i64 fx[10], dz[10];
-        planes(A, k);
-        if (k >= kb) {
-            // 1. transverse values of the x and y faces
-            i64 g[FXG];
-            rows(A, xrow);
-            cols(A, xcol);
-            fx_cell_values<0>(P, A, txp, txm, g);
-            if (gxs) {
-#pragma unroll
-                for (int s = 0; s < FXG; ++s) gxw[s * 34] = g[s];
-            }
-            cols(A, cc1);
-#pragma unroll 1
-            for (int t = 0; t < (wr ? 1 : 2); ++t) {  // the halo warp: the rows below and above the tile
-                rows(A, t ? wrapc(j0 + R, ny) : row);
-                fx_cell_values<1>(P, A, txp, txm, g);
-                i64 *w = &gy[t ? R + 1 : wr][0][lane];
-#pragma unroll
-                for (int s = 0; s < FXG; ++s) w[s * 32] = g[s];
-            }
-            __syncthreads();
-            // 2. faces
-            x_face(I, xr, I - c0, A.pl[1] + (wr ? row : wrapc(j0 + xr, ny)) * P.rs, fx);
-            if (wr == 0 && lane < R) {
-#pragma unroll
-                for (int s = 0; s < 10; ++s) xsh[lane][s] = fx[s];
-            }
-            i64 v[10];
-            y_face(wr, v);
-#pragma unroll
-            for (int s = 0; s < 10; ++s) ysh[wr][s][lane] = v[s];
-        }
-        if (wr >= 1) {
-            i64 b[FXG], v[10];
-            planes(A, k + 1);
-            rows(A, row);
-            cols(A, cc1);
-            fx_cell_values<2>(P, A, txp, txm, b);
-            if (k >= kb - 1) {
-                z_face(gzA, b, v);
-#pragma unroll
-                for (int s = 0; s < 10; ++s) {
-                    dz[s] = cz(flux_pop(2, s)) > 0 ? fz[s] - v[s] : v[s] - fz[s];
-                    fz[s] = v[s];
+            if (!P.periodic_x) {
+                // bounce-back on the walls: populations entering the fluid take their opposites' values
+                if (I == 0) {
+                    v[0] = v[1]; v[2] = v[5]; v[4] = v[3]; v[6] = v[9]; v[8] = v[7];
+                }
+                if (I == nx) {
+                    v[1] = v[0]; v[5] = v[2]; v[3] = v[4]; v[9] = v[6]; v[7] = v[8];
                 }
             }
+            fx_face_flux<0, FAX>(P, v, m);
+            const int b = k & 1;
+            if (halo) {
+                if (lane < R) {
 #pragma unroll
-            for (int s = 0; s < FXG; ++s) gzA[s] = b[s];
-        } else if (k + 2 < ke + 1) {
-            prefetch(k + 2);
-        }
-        if (k < kb) continue;
-        __syncthreads();
-        // 3. update: f = 4/3 f-bar-plus - 1/3 f - sum of flux differences
-        if (wr >= 1) {
-            planes(A, k);
-            rows(A, row);
-            cols(A, cc1);
-            const FxMul cxm = at_x(cc1 + 1, FXT_CX);
-            const long long c = ((long long)k * ny + min(gj, ny - 1)) * P.pitch + cc1;
+                    for (int s = 0; s < 6; ++s) xs0[b][lane][s] = v[s];
 #pragma unroll
-            for (int p = 0; p < NPOP; ++p) {
-                const i64 b = A(p, 0, 0, 0);
-                i64 a = fx_madr(b - fx_from_double(f_in[p * P.ps + c]), P.third, b);
+                    for (int s = 0; s < 4; ++s) fxz[b][lane][s][0] = v[6 + s];
+                }
+                __syncthreads();
+                continue;
+            }
+#pragma unroll
+            for (int s = 0; s < 4; ++s) fxz[b][wr][s][lane + 1] = v[6 + s];
+            const long long c = ((long long)k * ny + min(j0 + wr, ny - 1)) * P.pitch + cc1;
+            i64 acc[7];  // populations 0, 1, 2, 7..10
+#pragma unroll
+            for (int n = 0; n < 7; ++n) acc[n] = base(n < 3 ? n : n + 4, c);
+            __syncthreads();
+#pragma unroll
+            for (int n = 0; n < 7; ++n) {
+                const int p = n < 3 ? n : n + 4;
+                i64 a = acc[n];
                 if (cx(p)) {
-                    const int s = flux_slot(0, p);
-                    i64 l = __shfl_up_sync(0xffffffffu, fx[s], 1);
-                    if (lane == 0) l = xsh[wr - 1][s];
-                    a = fx_madr(cx(p) > 0 ? l - fx[s] : fx[s] - l, cxm, a);
+                    const int s = flux_slot(0, p) < 0 ? 0 : flux_slot(0, p);
+                    i64 l = __shfl_up_sync(0xffffffffu, v[s], 1);
+                    if (lane == 0) l = xs0[b][wr][s];
+                    a = fx_madr(cx(p) > 0 ? l - v[s] : v[s] - l, cxm, a);
                 }
                 if (cy(p)) {
                     const int s = flux_slot(1, p);
-                    const i64 l = ysh[wr - 1][s][lane], u = ysh[wr][s][lane];
+                    const i64 l = ysh[b][wr][s][lane], u = ysh[b][wr + 1][s][lane];
                     a = fx_madr(cy(p) > 0 ? l - u : u - l, P.cy, a);
                 }
-                if (cz(p)) a = fx_madr(dz[flux_slot(2, p)], P.cz, a);
                 if (cell) f_out[p * P.ps + c] = fx_to_double(a);
             }
+        }
+    } else if (wr <= 2 * R + 2) {
+        // --- y: tile row yr - 1; the face below it (none for the last warp)
+        const int yr = wr - (R + 1), gj = j0 + yr - 1;
+        const FxMul txp = at_x(cc1 + 1, FXT_TXP), txm = at_x(cc1 + 1, FXT_TXM);
+        const bool cell = yr >= 1 && yr <= R && gc < nx && gj < ny;
+        rows(wrapc(gj, ny));
+        cols(cc1);
+        i64 *gyw = &gy[yr][0][lane];
+        // plane k's f-bar-plus rows of the tile and f-tilde into L2 (last warp), two planes ahead of use
+        auto prefetch = [&](int k) {
+            const int q = wrap(k, nz);
+            if (lane < R + 2)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(fb + q * plane + wrapc(wrap(j0 - 1 + lane, ny), ny) * (long long)P.rs + fx_col(c0)),
+                             "r"(unsigned(min(2, (P.pitch_b - c0) >> 4) * NPOP * 16 * 8)));
+            if (k < ke)
+                for (int t = lane; t < NPOP * R * 2; t += 32) {
+                    const int p = t / (2 * R), r = (t >> 1) % R;
+                    const long long o = p * P.ps + ((long long)k * ny + min(j0 + r, ny - 1)) * P.pitch + min(c0 + 16 * (t & 1), nx - 1);
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(f_in + o));
+                }
+        };
+        i64 old[10];
+        planes(kb - 1);
+        fx_zparts<1>(P, A, txp, txm, old);
+        for (int k = kb; k < ke; ++k) {
+            planes(k);
+            fx_cell_values<1>(P, A, txp, txm, old, [&](int n, i64 x) { gyw[n * 32] = x; });
+            fx_bar(2, 32 * (R + 2));
+            if (yr > R) {
+                if (k + 2 <= ke) prefetch(k + 2);
+                __syncthreads();
+                continue;
+            }
+            // face between tile rows yr - 1 (gy[yr]) and yr
+            i64 v[10], m[3];
+#pragma unroll
+            for (int s = 0; s < 10; ++s) v[s] = fx_normal<1>(s, gy[yr][s][lane], gy[yr + 1][s][lane], P.my, P.my);
+#pragma unroll
+            for (int s = 0; s < 3; ++s) m[s] = (gy[yr][10 + s][lane] + gy[yr + 1][10 + s][lane]) >> 1;
+            fx_face_flux<1, FAX>(P, v, m);
+            const int b = k & 1;
+#pragma unroll
+            for (int s = 0; s < 10; ++s) ysh[b][yr][s][lane] = v[s];
+            if (yr == 0) {
+                __syncthreads();
+                continue;
+            }
+            const long long c = ((long long)k * ny + min(gj, ny - 1)) * P.pitch + cc1;
+            i64 acc[6];  // populations 3, 4, 15..18
+#pragma unroll
+            for (int n = 0; n < 6; ++n) acc[n] = base(n < 2 ? 3 + n : 13 + n, c);
+            __syncthreads();
+#pragma unroll
+            for (int n = 0; n < 6; ++n) {
+                const int p = n < 2 ? 3 + n : 13 + n, s = flux_slot(1, p);
+                const i64 l = ysh[b][yr - 1][s][lane];
+                i64 a = fx_madr(cy(p) > 0 ? l - v[s] : v[s] - l, P.cy, acc[n]);
+                if (cz(p)) a = fx_madr(dzs[b][yr - 1][flux_slot(2, p) - 6][lane], P.cz, a);
+                if (cell) f_out[p * P.ps + c] = fx_to_double(a);
+            }
+        }
+    } else {
+        // --- z
+        const int r = wr - (2 * R + 3), gj = j0 + r;
+        const FxMul txp = at_x(cc1 + 1, FXT_TXP), txm = at_x(cc1 + 1, FXT_TXM), cxm = at_x(cc1 + 1, FXT_CX);
+        const bool cell = gc < nx && gj < ny;
+        rows(wrapc(gj, ny));
+        cols(cc1);
+        i64 *gz = sm + L::GZ + r * FXG * 32 + lane;  // the thread's values of the last plane
+        i64 fz[10];                                  // flux below plane k
+        planes(kb - 1);
+        fx_cell_values<2>(P, A, txp, txm, nullptr, [&](int n, i64 x) { gz[n * 32] = x; });
+        // one round ahead of the first plane for the flux below it
+        for (int k = kb - 1; k < ke; ++k) {
+            i64 v[10], m[3];
+            planes(k + 1);
+            fx_cell_values<2>(P, A, txp, txm, nullptr, [&](int n, i64 x) {
+                const i64 o = gz[n * 32];
+                gz[n * 32] = x;
+                if (n < 10)
+                    v[n < 10 ? n : 0] = fx_normal<2>(n < 10 ? n : 0, o, x, P.mz, P.mz);
+                else
+                    m[n < 10 ? 0 : n - 10] = (o + x) >> 1;
+            });
+            fx_face_flux<2, FAX>(P, v, m);
+            if (k >= kb) {
+                const int b = k & 1;
+#pragma unroll
+                for (int s = 0; s < 10; ++s) fz[s] = cz(flux_pop(2, s)) > 0 ? fz[s] - v[s] : v[s] - fz[s];
+#pragma unroll
+                for (int s = 0; s < 4; ++s) dzs[b][r][s][lane] = fz[6 + s];
+                planes(k);
+                const long long c = ((long long)k * ny + min(gj, ny - 1)) * P.pitch + cc1;
+                i64 acc[6];  // populations 5, 6, 11..14
+#pragma unroll
+                for (int n = 0; n < 6; ++n) acc[n] = fx_madr(fz[n], P.cz, base(n < 2 ? 5 + n : 9 + n, c));
+                __syncthreads();
+#pragma unroll
+                for (int n = 0; n < 6; ++n) {
+                    const int p = n < 2 ? 5 + n : 9 + n;
+                    i64 a = acc[n];
+                    if (cx(p)) {
+                        const i64 l = fxz[b][r][n - 2 < 0 ? 0 : n - 2][lane], u = fxz[b][r][n - 2 < 0 ? 0 : n - 2][lane + 1];
+                        a = fx_madr(cx(p) > 0 ? l - u : u - l, cxm, a);
+                    }
+                    if (cell) f_out[p * P.ps + c] = fx_to_double(a);
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < 10; ++s) fz[s] = v[s];
         }
     }
 }

@@ -57,18 +57,33 @@ __global__ void fx_decode_kernel(const i64 *__restrict__ fb, double *__restrict_
     for (int p = 0; p < NPOP; ++p) q[p * D.ps_b] = fx_to_double(src[p * 16]);
 }
 
-constexpr int FX_W = 8, FX_MINB = 2, REDO_W = 8, REDO_MINB = 2;
+constexpr int FX_R = 4, FX_MINB = 1, REDO_W = 8, REDO_MINB = 2;
+
+// z chunks of the flux kernel: the count (each about nz / chunks planes) whose waves of CTAs
+// take the least planes of work.  Beginning a chunk costs about 1.5 planes (FX_START: two
+// rounds of the z warps, part of one of the others).
+int flux_fx_chunks(long long tiles, int nz, long long slots)
+{
+    constexpr double FX_START = 1.5;
+    auto cost = [&](int c) {
+        return double((tiles * c + slots - 1) / slots) * (double((nz + c - 1) / c) + FX_START);
+    };
+    int best = 1;
+    for (int c = 2; c <= nz; ++c)
+        if (cost(c) < cost(best)) best = c;
+    return best;
+}
 
 template <int FAX>
 cudaError_t setup(FxPlan &L, int sms)
 {
-    constexpr size_t bytes = flux_fx_smem_bytes<FX_W>();
-    auto kern = flux_fx_kernel<FX_W, FX_MINB, FAX>;
+    constexpr size_t bytes = FxSmem<FX_R>::bytes;
+    auto kern = flux_fx_kernel<FX_R, FX_MINB, FAX>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
     int occ = 1;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * FX_W, bytes);
-    const long long cols = (long long)((L.P.nx + 31) / 32) * ((L.P.ny + FX_W - 2) / (FX_W - 1));
-    L.kchunk = choose_kchunk(L.P.nz, cols, (long long)sms * std::max(occ, 1));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * (3 * FX_R + 3), bytes);
+    const long long tiles = (long long)((L.P.nx + 31) / 32) * ((L.P.ny + FX_R - 1) / FX_R);
+    L.flux_chunks = flux_fx_chunks(tiles, L.P.nz, (long long)sms * std::max(occ, 1));
     return e;
 }
 
@@ -86,9 +101,9 @@ template <int FAX>
 cudaError_t flux(const FxPlan &L, const i64 *fb, const double *f_in, double *f_out, int *flag, cudaStream_t st)
 {
     const FxParams &P = L.P;
-    const dim3 grid((P.nx + 31) / 32, (P.ny + FX_W - 2) / (FX_W - 1), (P.nz + L.kchunk - 1) / L.kchunk);
-    flux_fx_kernel<FX_W, FX_MINB, FAX>
-        <<<grid, dim3(32, FX_W), flux_fx_smem_bytes<FX_W>(), st>>>(fb, f_in, f_out, P, L.kchunk, flag);
+    flux_fx_kernel<FX_R, FX_MINB, FAX>
+        <<<dim3((P.nx + 31) / 32, (P.ny + FX_R - 1) / FX_R, L.flux_chunks), dim3(32, 3 * FX_R + 3),
+           FxSmem<FX_R>::bytes, st>>>(fb, f_in, f_out, P, flag);
     return cudaGetLastError();
 }
 

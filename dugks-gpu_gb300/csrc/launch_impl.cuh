@@ -52,7 +52,7 @@ cudaError_t Kern<T, S>::fbar(const S *f, S *fb, const StepParams<T, S> &P, cudaS
 // (useful waves / launched waves) * (1 - 1/(3k)) * (1 - 1/(2k)) over chunk
 // lengths k >= 4, keeping at least two waves where the grid allows it so that
 // the scheduler can even out tiles of unequal work (partial rows).
-static int choose_kchunk(int nz, long long cols, long long slots)
+[[maybe_unused]] static int choose_kchunk(int nz, long long cols, long long slots)
 {
     const int kmin = std::min(nz, 4);
     const long long max_chunks = (nz + kmin - 1) / kmin;

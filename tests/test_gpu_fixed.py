@@ -40,6 +40,16 @@ def test_edges_of_tiles(nx, ny, nz, periodic_x):
     assert rel_err(eng.get_state(), _oracle(orc, f0, 3)) <= TOL
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(5, 3, 2), (31, 4, 1), (32, 5, 3), (33, 9, 16), (65, 13, 2), (40, 4, 33)])
+@pytest.mark.parametrize("periodic_x", [0, 1])
+def test_edges_of_four_row_tiles(nx, ny, nz, periodic_x):
+    """Tiles of four rows with warps per axis; z chunks of unequal length; the FP64 parity bound."""
+    eng, orc, f0 = _pair(nx=nx, ny=ny, nz=nz, xwidth=nx, ywidth=1.3 * ny, zwidth=nz, periods_x=periodic_x,
+                         ambient_fy=2e-5)
+    eng.run(1, 4)
+    assert rel_err(eng.get_state(), _oracle(orc, f0, 4)) <= TOL
+
+
 @pytest.mark.parametrize("axis", ["x", "y", "z", None])
 @pytest.mark.parametrize("mesh", ["uniform", "tanh"])
 def test_force_axes_and_meshes(axis, mesh):
