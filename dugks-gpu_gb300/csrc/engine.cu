@@ -34,6 +34,7 @@
 #include "../../include/dugks_gb300.h"
 #include "config.h"
 #include "fixed_launch.cuh"
+#include "host_pages.h"
 #include "launch.cuh"
 #include "spectral_kernels.cuh"
 
@@ -802,6 +803,7 @@ int get_state_form(dg_ctx *h, double *host_dump)
     double *tmp = state_staging(h, n * sizeof(double), &owned);
     if (!tmp) return h->fail(DG_ERR_CUDA, "cudaMalloc (state download staging) failed");
     cudaError_t e = K::soa_to_aos(static_cast<const S *>(h->f), tmp, params_for<T, S>(h, 0), h->stream);
+    if (e == cudaSuccess) populate_pages(host_dump, n * sizeof(double));
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_dump, tmp, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (owned) cudaFree(tmp);
