@@ -7,7 +7,7 @@
 // exactly (its values have fewer bits than the fixed point) and rounded once when
 // written.  f-bar-plus, written and read by these two kernels only, is held in
 // fixed point.  Step of the 256 x 128 x 128 channel: 6.65 ms with the FP64 kernels,
-// 1.27 ms here (stage (a) 0.21, flux 1.06); 64^3 box 0.63 -> 0.104 ms, 64 x 32 x 32
+// 1.22 ms here (stage (a) 0.21, flux 1.01); 64^3 box 0.63 -> 0.104 ms, 64 x 32 x 32
 // channel 0.229 -> 0.037 ms.
 //
 // Error of the state against an 80-bit run of the same scheme (relative 2-norm):
@@ -379,16 +379,15 @@ __device__ __forceinline__ void fx_bar(int id, int threads)
 // Bound by latency: with one warp per row doing all of it (values of all three axes and
 // z carries in registers) the loads' latency showed between spills, issue 33 %; split by
 // axis a thread carries few values, three times the warps share a tile and their phases
-// overlap, issue 40 %, ALU pipe 40 %.  256 x 128 x 128 channel: 1.45 -> 1.06 ms; 64 x 32 x
-// 32: a step 78 -> 37 us.  R = 4 (15 warps, no spills at 128 registers); R = 7 (24 warps,
-// 80 registers) 1.01 ms there but 43 us at 64 x 32 x 32; R = 5, 6 (five and six warps on
-// some schedulers) 1.2 to 1.3 ms.  Waits split into arrive and wait (mbarriers), with the
+// overlap, issue 40 %, ALU pipe 40 %.  256 x 128 x 128 channel: 1.45 -> 1.01 ms; 64 x 32 x
+// 32: a step 78 -> 37 us (R = 7 and 4, see flux_fx_tiling; R = 5 and 6, with warps that do
+// not divide evenly over the schedulers, 1.2 to 1.3 ms).  Waits split into arrive and wait (mbarriers), with the
 // next plane's values in between, were slower (1.5 ms), and so was an even split of all
 // planes over one CTA per SM (1.09 ms: tiles next to each other, at different planes, no
 // longer share rows in L2).
-template <int R, int MINB, int FAX>
-__global__ void __launch_bounds__(32 * (3 * R + 3), MINB) flux_fx_kernel(const i64 *__restrict__ fb, const double *f_in,
-                                                                         double *f_out, const FxParams P, const int *flag)
+template <int R, int FAX>
+__global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(const i64 *__restrict__ fb, const double *f_in,
+                                                                   double *f_out, const FxParams P, const int *flag)
 {
     using L = FxSmem<R>;
     extern __shared__ __align__(16) i64 sm[];

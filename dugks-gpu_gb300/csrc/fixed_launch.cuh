@@ -10,7 +10,7 @@ namespace dg {
 struct FxPlan {
     FxParams P;
     int fax;          // force axis (3: none)
-    int flux_chunks;  // z chunks of the flux kernel
+    int flux_rows, flux_chunks;  // tile rows and z chunks of the flux kernel
     int redo_blocks;  // cooperative grid of the redo kernel
     StepParams<double, double> D;
 };

@@ -57,34 +57,47 @@ __global__ void fx_decode_kernel(const i64 *__restrict__ fb, double *__restrict_
     for (int p = 0; p < NPOP; ++p) q[p * D.ps_b] = fx_to_double(src[p * 16]);
 }
 
-constexpr int FX_R = 4, FX_MINB = 1, REDO_W = 8, REDO_MINB = 2;
+constexpr int REDO_W = 8, REDO_MINB = 2;
 
-// z chunks of the flux kernel: the count (each about nz / chunks planes) whose waves of CTAs
-// take the least planes of work.  Beginning a chunk costs about 1.5 planes (FX_START: two
-// rounds of the z warps, part of one of the others).
-int flux_fx_chunks(long long tiles, int nz, long long slots)
+// The flux kernel has tiles of four rows (128 registers, no spills) and of seven (80, 24
+// warps per SM, fewer rows formed twice).  A plane of a seven-row tile takes 1.65 times one
+// of four rows (7.8 against 4.7 us), and beginning a z chunk costs about 1.5 planes (two
+// rounds of the z warps, part of one of the others).  Rows and chunk count are those whose
+// waves of CTAs take the least time: 256 x 128 x 128 channel 1.01 ms with seven rows, 1.06
+// with four; 64 x 32 x 32 channel, whole step, 43 and 37 us; 64^3 box 107 and 104 us.
+struct FxTiling {
+    int rows, chunks;
+};
+FxTiling flux_fx_tiling(int nx, int ny, int nz, int slots)
 {
-    constexpr double FX_START = 1.5;
-    auto cost = [&](int c) {
-        return double((tiles * c + slots - 1) / slots) * (double((nz + c - 1) / c) + FX_START);
-    };
-    int best = 1;
-    for (int c = 2; c <= nz; ++c)
-        if (cost(c) < cost(best)) best = c;
+    FxTiling best{4, 1};
+    double least = 1e300;
+    for (int rows : {4, 7}) {
+        const long long tiles = (long long)((nx + 31) / 32) * ((ny + rows - 1) / rows);
+        for (int c = 1; c <= nz; ++c) {
+            const double cost = double((tiles * c + slots - 1) / slots) * ((nz + c - 1) / c + 1.5) * (rows == 7 ? 1.65 : 1.0);
+            if (cost < least) {
+                least = cost;
+                best = FxTiling{rows, c};
+            }
+        }
+    }
     return best;
+}
+
+template <int FAX, int R>
+cudaError_t allow_smem()
+{
+    return cudaFuncSetAttribute(flux_fx_kernel<R, FAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(FxSmem<R>::bytes));
 }
 
 template <int FAX>
 cudaError_t setup(FxPlan &L, int sms)
 {
-    constexpr size_t bytes = FxSmem<FX_R>::bytes;
-    auto kern = flux_fx_kernel<FX_R, FX_MINB, FAX>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-    int occ = 1;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * (3 * FX_R + 3), bytes);
-    const long long tiles = (long long)((L.P.nx + 31) / 32) * ((L.P.ny + FX_R - 1) / FX_R);
-    L.flux_chunks = flux_fx_chunks(tiles, L.P.nz, (long long)sms * std::max(occ, 1));
-    return e;
+    const FxTiling t = flux_fx_tiling(L.P.nx, L.P.ny, L.P.nz, sms);  // one CTA per SM
+    L.flux_rows = t.rows;
+    L.flux_chunks = t.chunks;
+    return t.rows == 4 ? allow_smem<FAX, 4>() : allow_smem<FAX, 7>();
 }
 
 template <int FAX>
@@ -97,14 +110,20 @@ cudaError_t stage_a(const FxPlan &L, const double *f_in, i64 *fb, int *flag, cud
     return cudaGetLastError();
 }
 
+template <int FAX, int R>
+cudaError_t flux_rows(const FxPlan &L, const i64 *fb, const double *f_in, double *f_out, int *flag, cudaStream_t st)
+{
+    const FxParams &P = L.P;
+    const dim3 grid((P.nx + 31) / 32, (P.ny + R - 1) / R, L.flux_chunks);
+    flux_fx_kernel<R, FAX><<<grid, dim3(32, 3 * R + 3), FxSmem<R>::bytes, st>>>(fb, f_in, f_out, P, flag);
+    return cudaGetLastError();
+}
+
 template <int FAX>
 cudaError_t flux(const FxPlan &L, const i64 *fb, const double *f_in, double *f_out, int *flag, cudaStream_t st)
 {
-    const FxParams &P = L.P;
-    flux_fx_kernel<FX_R, FX_MINB, FAX>
-        <<<dim3((P.nx + 31) / 32, (P.ny + FX_R - 1) / FX_R, L.flux_chunks), dim3(32, 3 * FX_R + 3),
-           FxSmem<FX_R>::bytes, st>>>(fb, f_in, f_out, P, flag);
-    return cudaGetLastError();
+    return L.flux_rows == 4 ? flux_rows<FAX, 4>(L, fb, f_in, f_out, flag, st)
+                            : flux_rows<FAX, 7>(L, fb, f_in, f_out, flag, st);
 }
 
 }  // namespace

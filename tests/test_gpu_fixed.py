@@ -50,6 +50,15 @@ def test_edges_of_four_row_tiles(nx, ny, nz, periodic_x):
     assert rel_err(eng.get_state(), _oracle(orc, f0, 4)) <= TOL
 
 
+@pytest.mark.parametrize("nx,ny,nz,periodic_x", [(63, 133, 80, 0), (96, 126, 96, 1), (160, 129, 64, 0)])
+def test_seven_row_tiles(nx, ny, nz, periodic_x):
+    """Grids whose planes the flux kernel takes seven rows at a time, with ragged last tiles; the FP64 parity bound."""
+    eng, orc, f0 = _pair(nx=nx, ny=ny, nz=nz, xwidth=nx, ywidth=1.1 * ny, zwidth=nz, periods_x=periodic_x,
+                         ambient_fz=2e-5)
+    eng.run(1, 2)
+    assert rel_err(eng.get_state(), _oracle(orc, f0, 2)) <= TOL
+
+
 @pytest.mark.parametrize("axis", ["x", "y", "z", None])
 @pytest.mark.parametrize("mesh", ["uniform", "tanh"])
 def test_force_axes_and_meshes(axis, mesh):
