@@ -572,10 +572,10 @@ __global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *_
     fbar_block<T, S>(f, fb, P, threadIdx.x, blockIdx.x, blockDim.x, blockIdx.y, blockIdx.z);
 }
 
-// Stage (a) of the float forms, one thread per cell.  GHOST = 0: the interior of
-// f-bar-plus only.  GHOST = 2: the interior and its periodic images in y and z (the
-// 16-bit forms between walls, whose flux kernel forms the wall ghost columns itself).
-// GHOST = 1 (FP32): the ghost layer is written by the threads that hold its sources --
+// Stage (a) of the float forms, one thread per cell.  GHOST = 2: the interior of
+// f-bar-plus and its periodic images in y and z (the 16-bit forms between walls, whose
+// flux kernel forms the wall ghost columns itself).  GHOST = 1 (FP32, and the 16-bit forms
+// when periodic): the ghost layer is written by the threads that hold its sources --
 // a cell of the first/last row or plane also writes its periodic images in y and z
 // (src/dugks.cu:1256-1273, src/parallel.cu:192-199), the first/last cell of a row the
 // periodic x copy (src/dugks.cu:1212-1229), and between walls the warp next to a wall
@@ -599,7 +599,8 @@ __global__ void __launch_bounds__(128) fbar_float_kernel(const S *__restrict__ f
     const int j0 = blockIdx.y * rows, j1 = min(j0 + rows, ny);
     const bool in = i >= 0 && i < nx;
     const int w0 = i - (threadIdx.x & 31);  // cell of lane 0
-    const bool lo = GHOST == 1 && !P.periodic_x && w0 <= 0, hi = GHOST == 1 && !P.periodic_x && w0 <= nx - 1 && w0 + 31 >= nx - 1;
+    constexpr bool WALLS = GHOST == 1 && sizeof(S) == 4;
+    const bool lo = WALLS && !P.periodic_x && w0 <= 0, hi = WALLS && !P.periodic_x && w0 <= nx - 1 && w0 + 31 >= nx - 1;
     if (!in && !lo && !hi) return;
     const int ic = in ? i : (i < 0 ? 0 : nx - 1);  // lanes past the row read a valid cell and store nothing
     const S *src = f + ((long long)k * ny + j0) * P.pitch;
@@ -650,8 +651,6 @@ __global__ void __launch_bounds__(128) fbar_float_kernel(const S *__restrict__ f
 #pragma unroll
             for (int p = 0; p < NPOP; ++p) row[p * P.ps_b + ic + 1] = enc[p];
         }
-        if (GHOST == 0) continue;
-
         // periodic images of this row and plane (uniform over the block): J = 1 -> ny+1,
         // J = ny -> 0, likewise K, and the corner image
         const long long rstep = P.pitch_b, pstep = (long long)(ny + 2) * P.pitch_b;
