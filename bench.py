@@ -383,7 +383,7 @@ def main():
     achieved = flux_bytes / (ms_b / K / 1e3) / 1e9
     peak, peak_kind = measured_peak_hbm()
     traffic, traffic_src = ncu_traffic(args.precision, grid)
-    names = ("fbar_fx_kernel", "flux_fx_kernel") if args.precision == "fp64" else ("fbar_kernel", "flux_tma_kernel")
+    names = ("fbar_fx_kernel", "flux_fx_kernel") if args.precision == "fp64" else ("fbar_float_kernel", "flux_tma_kernel")
     roof = {"bound": "hbm", "kernel": names[1], "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic, "traffic_from": traffic_src,
             "peak_source": peak_kind, "alg_bytes_per_cell": 57 * info_bytes,

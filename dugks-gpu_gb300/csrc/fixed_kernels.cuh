@@ -379,7 +379,7 @@ __device__ __forceinline__ void fx_bar(int id, int threads)
 // Bound by latency: with one warp per row doing all of it (values of all three axes and
 // z carries in registers) the loads' latency showed between spills, issue 33 %; split by
 // axis a thread carries few values, three times the warps share a tile and their phases
-// overlap, issue 40 %, ALU pipe 40 %.  256 x 128 x 128 channel: 1.45 -> 1.01 ms; 64 x 32 x
+// overlap, issue 40 to 45 %, ALU pipe 40 %.  256 x 128 x 128 channel: 1.45 -> 1.01 ms; 64 x 32 x
 // 32: a step 78 -> 37 us (R = 7 and 4, see flux_fx_tiling; R = 5 and 6, with warps that do
 // not divide evenly over the schedulers, 1.2 to 1.3 ms).  Waits split into arrive and wait (mbarriers), with the
 // next plane's values in between, were slower (1.5 ms), and so was an even split of all
