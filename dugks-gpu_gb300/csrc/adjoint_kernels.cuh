@@ -116,16 +116,23 @@ __host__ __device__ inline long long adj_cell(int i, int j, int k, int nx, int n
     return ((long long)(k - 1) * ny + (j - 1)) * nx + (i - 1);
 }
 
-// Layout of the adjoint face values LX, LY, LZ: per row (k, j) blocks of 32 columns with
-// the 19 populations of a block one after another, so that a population step is an
+// Layout of the adjoint face values LX, LY, LZ: per row (k, j) blocks of kAdjBlk columns
+// with the 19 populations of a block one after another, so that a population step is an
 // immediate of the load and a row's address serves all of them.  Column of the x face I,
-// 1 <= I <= nx, and of the y and z faces at i: adj_col; the x face 0 between walls: nx.
-__host__ __device__ constexpr int adj_col(int c) { return (c >> 5) * (NPOP * 32) + (c & 31); }
-__host__ __device__ inline int adj_xcol(int I, int nx) { return adj_col(I >= 1 ? I - 1 : nx); }
-__host__ __device__ inline int adj_rowlen(int nx) { return (nx + 32) / 32 * (NPOP * 32); }
+// 1 <= I <= nx, and of the y and z faces at i: adj_col.  The x faces I = 0 between walls
+// are an array of their own, X0, with the rows as its columns.
+constexpr int kAdjBlk = 8;  // 16 and 32 are as fast and pad narrow rows more
+__host__ __device__ constexpr long long adj_col(long long c)
+{
+    return c / kAdjBlk * (NPOP * kAdjBlk) + c % kAdjBlk;
+}
 __host__ __device__ inline long long adj_row(int j, int k, int nx, int ny)
 {
-    return ((long long)(k - 1) * ny + (j - 1)) * adj_rowlen(nx);
+    return ((long long)(k - 1) * ny + (j - 1)) * ((nx + kAdjBlk - 1) / kAdjBlk * (NPOP * kAdjBlk));
+}
+__host__ __device__ inline long long adj_x0len(int ny, int nz)
+{
+    return ((long long)ny * nz + kAdjBlk - 1) / kAdjBlk * (NPOP * kAdjBlk);
 }
 
 // Per-face adjoint of the face values v: take the flux adjoint from the two adjacent
@@ -247,7 +254,8 @@ __device__ __forceinline__ void adj_face_flux(const StepParams<T, S> &P, T v[NPO
 // only_x0: x faces I = 0 only (one thread per row and plane).
 template <class T, class S, int AX>
 __global__ void __launch_bounds__(128) adj_face_kernel(const S *__restrict__ fb, const S *__restrict__ lam_next,
-                                                       T *__restrict__ lamv, T *__restrict__ lamF_face,
+                                                       T *__restrict__ lamv, T *__restrict__ x0,
+                                                       T *__restrict__ lamF_face,
                                                        const StepParams<T, S> P, int only_x0)
 {
     const int nx = P.nx, ny = P.ny, nz = P.nz;
@@ -287,9 +295,10 @@ __global__ void __launch_bounds__(128) adj_face_kernel(const S *__restrict__ fb,
         face_tri<T, S, AX>(P, R, F, j, k, v);
     adj_face_flux<T, S, AX>(P, v, lam_next, F, j, k, lv, lf);
     if (lamF_face) lamF_face[q] = lf;
-    T *o = lamv + adj_row(j, k, nx, ny) + (AX == 0 ? adj_xcol(F, nx) : adj_col(F - 1));
+    T *o = AX == 0 && F == 0 ? x0 + adj_col((long long)(k - 1) * ny + (j - 1))
+                             : lamv + adj_row(j, k, nx, ny) + adj_col(F - 1);
 #pragma unroll
-    for (int p = 0; p < NPOP; ++p) o[p * 32] = lv[p];
+    for (int p = 0; p < NPOP; ++p) o[p * kAdjBlk] = lv[p];
 }
 
 // The three faces +x (I = i), +y (J = j) and +z (K = k) of every cell, with
@@ -380,12 +389,12 @@ __global__ void __launch_bounds__(32 * W, MINB) adj_faces_tma_kernel(const __gri
             adj_face_flux<T, S, 0>(P, v, lam_next, gi, gj, k, lv, lf);
             LFX[qx] = lf;
 #pragma unroll
-            for (int p = 0; p < NPOP; ++p) LX[o + p * 32] = lv[p];
+            for (int p = 0; p < NPOP; ++p) LX[o + p * kAdjBlk] = lv[p];
             face_tri_x2<S, 1, true>(P, R, gi, gj, k, oy, v);
             adj_face_flux<T, S, 1>(P, v, lam_next, gi, gj, k, lv, lf);
             LFY[qc] = lf;
 #pragma unroll
-            for (int p = 0; p < NPOP; ++p) LY[o + p * 32] = lv[p];
+            for (int p = 0; p < NPOP; ++p) LY[o + p * kAdjBlk] = lv[p];
             T Z[NPOP];
             plane_z_x2<S, true>(P, R, gi, gj, k + 1, Z);
             face_z_x2<S, true>(P, R, Y, Z, v);
@@ -393,7 +402,7 @@ __global__ void __launch_bounds__(32 * W, MINB) adj_faces_tma_kernel(const __gri
             LFZ[qc] = lf;
 #pragma unroll
             for (int p = 0; p < NPOP; ++p) {
-                LZ[o + p * 32] = lv[p];
+                LZ[o + p * kAdjBlk] = lv[p];
                 Y[p] = Z[p];
             }
         }
@@ -405,15 +414,16 @@ __global__ void __launch_bounds__(32 * W, MINB) adj_faces_tma_kernel(const __gri
 
 // Where the transposed stencil of one cell reads: population 0 of the face rows around
 // row j, plane k, [dk+1][dj+1] (y faces: dj = -1, 0; z faces: dk = -1, 0; the periodic
-// images in y and z folded in), x faces at stored column cf, y and z faces at cc.
+// images in y and z folded in), x faces at stored column cf (of X0 if negative), y and z
+// faces at cc.
 template <class T>
 struct AdjAt {
     const T *x[3][3], *y[3][2], *z[2][3];
 };
 
 template <class T>
-__device__ __forceinline__ AdjAt<T> adj_at(const T *LX, const T *LY, const T *LZ, int j, int k, int cf, int cc, int nx,
-                                           int ny, int nz)
+__device__ __forceinline__ AdjAt<T> adj_at(const T *LX, const T *LY, const T *LZ, const T *X0, int j, int k, int cf,
+                                           int cc, int nx, int ny, int nz)
 {
     AdjAt<T> A;
     const int js[3] = {j == 1 ? ny : j - 1, j, j == ny ? 1 : j + 1};
@@ -423,7 +433,7 @@ __device__ __forceinline__ AdjAt<T> adj_at(const T *LX, const T *LY, const T *LZ
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
             const long long o = adj_row(js[b], ks[a], nx, ny);
-            A.x[a][b] = LX + o + cf;
+            A.x[a][b] = cf < 0 ? X0 + adj_col((long long)(ks[a] - 1) * ny + (js[b] - 1)) : LX + o + cf;
             if (b < 2) A.y[a][b] = LY + o + cc;
             if (a < 2) A.z[a][b] = LZ + o + cc;
         }
@@ -439,9 +449,9 @@ struct AdjPop {
     const StepParams<T, S> &P;
     static constexpr int ax = cx(p), ay = cy(p), az = cz(p), rp = xrep(p);
 
-    __device__ __forceinline__ T X(int dk, int dj) const { return __ldg(A.x[dk + 1][dj + 1] + p * 32); }
-    __device__ __forceinline__ T Y(int dk, int dj) const { return __ldg(A.y[dk + 1][dj + 1] + p * 32); }
-    __device__ __forceinline__ T Z(int dk, int dj) const { return __ldg(A.z[dk + 1][dj + 1] + p * 32); }
+    __device__ __forceinline__ T X(int dk, int dj) const { return __ldg(A.x[dk + 1][dj + 1] + p * kAdjBlk); }
+    __device__ __forceinline__ T Y(int dk, int dj) const { return __ldg(A.y[dk + 1][dj + 1] + p * kAdjBlk); }
+    __device__ __forceinline__ T Z(int dk, int dj) const { return __ldg(A.z[dk + 1][dj + 1] + p * kAdjBlk); }
     __device__ __forceinline__ T xsum() const
     {
         const T tyo = p == 0 ? T(1) : P.ty_om, tym = P.ty_m, tzo = p == 0 ? T(1) : P.tz_om, tzm = P.tz_m;
@@ -552,12 +562,13 @@ __device__ __forceinline__ T xface_share(const StepParams<T, S> &P, int I, int g
 // the columns of one row, run on into the rows below it (so that a row length that is no
 // multiple of a warp leaves no lanes idle); the outermost lanes only form the sums their
 // neighbours need.
-// Bound by the latency of the face values' loads (128 registers: 16 warps per SM).  FP32,
-// 128 x 96 x 96 channel: 199 us, and 15 us less without a kernel for the wall ghosts; as two
-// kernels that formed the neighbours' sums again and handed the 19 sums over in memory
-// 221 us.  A row per warp beats the populations of a row over four warps (240 us: the row
-// addresses formed four times), 16 warps per SM beat 12 and 20, adjacent rows in a CTA
-// beat one row (they share the rows between them in L1).
+// Bound by the latency of the face values' loads (128 registers: 16 warps per SM).  The
+// adjoint step of the FP32 128 x 96 x 96 channel: 430 us with face rows of one column more
+// (the x faces 0 among them), 401 us with X0 apart; 480 us with kernels for the wall
+// ghosts, the stencil (each cell forming its neighbours' sums again) and the rest.  A row
+// per warp beats the populations of a row over four warps (the row addresses formed four
+// times), 16 warps per SM beat 12 and 20, adjacent rows in a CTA beat one row (they share
+// the rows between them in L1).
 constexpr int kAdjRows = 4;                                                      // warps, on adjacent rows, of a CTA
 __host__ __device__ inline int adj_halo(int periodic_x) { return periodic_x ? 1 : 2; }  // lanes below the first cell
 __host__ __device__ inline int adj_cols(int periodic_x) { return 31 - adj_halo(periodic_x); }
@@ -565,7 +576,7 @@ __host__ __device__ inline int adj_cols(int periodic_x) { return 31 - adj_halo(p
 template <class T, class S>
 __global__ void __launch_bounds__(32 * kAdjRows, 4)
     adj_cell_kernel(const S *__restrict__ f, const S *__restrict__ lam_next, const T *__restrict__ LX,
-                    const T *__restrict__ LY, const T *__restrict__ LZ, S *lam_out,
+                    const T *__restrict__ LY, const T *__restrict__ LZ, const T *__restrict__ X0, S *lam_out,
                     const T *__restrict__ LFX, const T *__restrict__ LFY, const T *__restrict__ LFZ,
                     double *__restrict__ dphi, const StepParams<T, S> P)
 {
@@ -581,8 +592,8 @@ __global__ void __launch_bounds__(32 * kAdjRows, 4)
     {
         // x face and column whose sums the lane forms: its own, or the periodic image at the ends
         const int nx = P.nx, per = P.periodic_x;
-        const int cf = adj_xcol(i == 0 ? (per ? nx : 0) : min(i, nx), nx);
-        const int cc = adj_col((i == 0 ? (per ? nx : 1) : (i == nx + 1 && per ? 1 : min(i, nx))) - 1);
+        const int cf = i == 0 && !per ? -1 : int(adj_col((i == 0 ? nx : min(i, nx)) - 1));
+        const int cc = int(adj_col((i == 0 ? (per ? nx : 1) : (i == nx + 1 && per ? 1 : min(i, nx))) - 1));
         const int ic = min(max(i, 1), nx);
         AdjXw<T> X;
 #pragma unroll
@@ -594,7 +605,7 @@ __global__ void __launch_bounds__(32 * kAdjRows, 4)
         X.t[1] = adj_tw(P, 2, ic, 0);
         X.n[0] = adj_tw(P, 1, ic == nx ? (per ? 1 : nx) : ic + 1, 1);
         X.n[1] = adj_tw(P, 2, ic == 1 ? (per ? nx : 1) : ic - 1, 1);
-        const AdjAt<T> A = adj_at(LX, LY, LZ, j, k, cf, cc, nx, P.ny, P.nz);
+        const AdjAt<T> A = adj_at(LX, LY, LZ, X0, j, k, cf, cc, nx, P.ny, P.nz);
         const bool wall = !per && __any_sync(0xffffffffu, i <= 2 || i >= nx - 1);
         adj_stencil<T, S>(A, P, X, i, wall, mu);
     }

@@ -7,13 +7,13 @@
 //                   extrapolation), which replaces the reference's extend_fb_x /
 //                   extend_fb_x_wall / extend_fb_y kernels and the MPI z exchange
 //                   (src/dugks.cu:348-377, src/parallel.cu:185-234): written by
-//                   fb_ghost_kernel (FP64; 16-bit forms with periodic x), by
-//                   fbar_float_kernel itself (FP32; 16-bit forms between walls: the y / z
-//                   images, the wall columns formed by the flux kernel in shared memory).
+//                   fb_ghost_kernel (FP64), by fbar_float_kernel itself (float forms;
+//                   16-bit between walls: the y / z images, the wall columns formed by
+//                   the flux kernel in shared memory).
 //
 // Kernels:
 //   fbar_kernel      stage (a), src/dugks.cu:1131-1196 (calc_fb1), in FP64
-//   fbar_float_kernel  the same in the float forms, with or without the ghost writes
+//   fbar_float_kernel  the same in the float forms, with the ghost writes
 //   fb_ghost_kernel  the ghost layer of f-bar-plus in a separate pass
 //   flux_kernel      stages (c) (d) (e) in FP64, src/dugks.cu:715-959 (calc_fx_tri) or
 //                    the central-difference variant 421-649 (calc_fx); every face

@@ -916,7 +916,7 @@ int adjoint_form(dg_ctx *h, int istep, const void *f_n, const void *lam_next, vo
         // 19 adjoint values and one dJ/dF (force-field face term) per face
         const long long n = adj_nface(0, h->nx, h->ny, h->nz) + 2 * adj_nface(1, h->nx, h->ny, h->nz);
         const long long nl = adj_row(1, h->nz + 1, h->nx, h->ny);
-        CK(cudaMalloc(&h->adj, (3 * size_t(nl) + size_t(n)) * sizeof(T)),
+        CK(cudaMalloc(&h->adj, (3 * size_t(nl) + size_t(adj_x0len(h->ny, h->nz)) + size_t(n)) * sizeof(T)),
            "cudaMalloc (adjoint scratch)");
     }
     if (h->ffield && !h->dphi) {

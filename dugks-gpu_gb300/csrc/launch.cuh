@@ -80,7 +80,7 @@ struct Kern {
     static cudaError_t moments_partials(const S *f, const StepParams<T, S> &P, double *partial, int nblocks,
                                         cudaStream_t st);
     // Adjoint of one step (adjoint_kernels.cuh): recomputes f-bar-plus of f_n into fb,
-    // per-face adjoints into lamv (T-typed scratch: three face arrays of adj_row(1, nz + 1), then dJ/dF per face),
+    // per-face adjoints into lamv (T-typed scratch: three face arrays of adj_row(1, nz + 1), the x faces 0 (adj_x0len), then dJ/dF per face),
     // then lam_out = (dS/df)^T lam_next.  FP64 and FP32 forms only.
     // dphi (optional, FP64, dump order [k][j][i]): += dJ/dphi of this step when a force field is set;
     // tmap_adj: f-bar-plus tensor map with AdjCfg::W + 2 rows (TMA forms)

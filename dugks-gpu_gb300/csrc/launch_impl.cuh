@@ -223,7 +223,8 @@ cudaError_t Kern<T, S>::adjoint(const S *f_n, S *fb, const S *lam_next, S *lam_o
         const long long nfx = adj_nface(0, P.nx, P.ny, P.nz), nfc = adj_nface(1, P.nx, P.ny, P.nz);
         const long long nl = adj_row(1, P.nz + 1, P.nx, P.ny);  // values of one face array
         T *LX = lamv, *LY = lamv + nl, *LZ = LY + nl;
-        T *LFX = LZ + nl, *LFY = LFX + nfx, *LFZ = LFY + nfc;  // per-face dJ/dF (force field)
+        T *X0 = LZ + nl;  // x faces 0 between walls
+        T *LFX = X0 + adj_x0len(P.ny, P.nz), *LFY = LFX + nfx, *LFZ = LFY + nfc;  // per-face dJ/dF (force field)
         if constexpr (TileCfg<T, S>::TMA) {
             // +x, +y, +z faces of every cell from the TMA-staged tile; x faces I = 0 apart
             if (!tmap_adj) return cudaErrorInvalidValue;
@@ -245,17 +246,17 @@ cudaError_t Kern<T, S>::adjoint(const S *f_n, S *fb, const S *lam_next, S *lam_o
             // between walls; one warp per block: the few wall faces spread over every SM
             const long long n0 = (long long)P.ny * P.nz;
             if (!P.periodic_x)
-                adj_face_kernel<T, S, 0><<<unsigned((n0 + 31) / 32), 32, 0, st>>>(fb, lam_next, LX, LFX, P, 1);
+                adj_face_kernel<T, S, 0><<<unsigned((n0 + 31) / 32), 32, 0, st>>>(fb, lam_next, LX, X0, LFX, P, 1);
         } else {
-            adj_face_kernel<T, S, 0><<<unsigned((nfx + 127) / 128), 128, 0, st>>>(fb, lam_next, LX, LFX, P, 0);
-            adj_face_kernel<T, S, 1><<<unsigned((nfc + 127) / 128), 128, 0, st>>>(fb, lam_next, LY, LFY, P, 0);
-            adj_face_kernel<T, S, 2><<<unsigned((nfc + 127) / 128), 128, 0, st>>>(fb, lam_next, LZ, LFZ, P, 0);
+            adj_face_kernel<T, S, 0><<<unsigned((nfx + 127) / 128), 128, 0, st>>>(fb, lam_next, LX, X0, LFX, P, 0);
+            adj_face_kernel<T, S, 1><<<unsigned((nfc + 127) / 128), 128, 0, st>>>(fb, lam_next, LY, nullptr, LFY, P, 0);
+            adj_face_kernel<T, S, 2><<<unsigned((nfc + 127) / 128), 128, 0, st>>>(fb, lam_next, LZ, nullptr, LFZ, P, 0);
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         const long long seq = (long long)((P.ny + kAdjRows - 1) / kAdjRows) * (P.nx + 2);
         const dim3 grid(unsigned((seq - 2 + adj_cols(P.periodic_x) - 1) / adj_cols(P.periodic_x)), P.nz);
-        adj_cell_kernel<T, S><<<grid, 32 * kAdjRows, 0, st>>>(f_n, lam_next, LX, LY, LZ, lam_out, LFX, LFY, LFZ, dphi, P);
+        adj_cell_kernel<T, S><<<grid, 32 * kAdjRows, 0, st>>>(f_n, lam_next, LX, LY, LZ, X0, lam_out, LFX, LFY, LFZ, dphi, P);
         return cudaGetLastError();
     }
 }
