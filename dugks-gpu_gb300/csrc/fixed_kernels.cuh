@@ -21,7 +21,8 @@
 // stay in that box, which bounds density (0.4 .. 1.98), momentum (|j| < 0.27),
 // 3 c_p.u (< 1.67, reached with the populations moving along c_p at the upper and
 // the others at the lower end) and the equilibrium polynomial (< 3.9) at every cell
-// and face, so that no sum or product overflows.  Stage (a) checks the box per value
+// and face, so that no sum or product overflows (the sums over the populations that do not
+// cross a face reach 1.32, see fx_mean).  Stage (a) checks the box per value
 // (NaN and infinities fail it) and raises a device flag; the flux kernel then does
 // nothing and fp64_redo_kernel does the whole step in FP64.  The parameters have to
 // fit too (make_fixed_plan in engine.cu): a single force axis, interpolation weights
@@ -343,6 +344,10 @@ __device__ __forceinline__ void fx_cell_values(const FxParams &P, const FxAt &A,
     for (int s = 0; s < 3; ++s) put(10 + s, m[s]);
 }
 
+// mean of the two cells' sum s (0: values, 1 and 2: tangential momenta).  The values' sums
+// are positive and below 1.32 each, not below 2 together: added as unsigned numbers
+DG_FX i64 fx_mean(int s, i64 a, i64 b) { return s == 0 ? i64((u64(a) + u64(b)) >> 1) : (a + b) >> 1; }
+
 // face value of crossing population p between the lower cell's a and the upper cell's b
 template <int AX>
 __device__ __forceinline__ i64 fx_normal(int s, i64 a, i64 b, FxMul mp, FxMul mm)
@@ -474,11 +479,11 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(const i64 *__
 #pragma unroll
                 for (int s = 0; s < 3; ++s) {
                     const i64 a = gx[xr][10 + s][q], b = gx[xr][10 + s][q + 1];
-                    m[s] = fx_mad(b - a - (s == 0 ? rest : 0), d, (a + b) >> 1);
+                    m[s] = fx_mad(b - a - (s == 0 ? rest : 0), d, fx_mean(s, a, b));
                 }
             } else {
 #pragma unroll
-                for (int s = 0; s < 3; ++s) m[s] = (gx[xr][10 + s][q] + gx[xr][10 + s][q + 1]) >> 1;
+                for (int s = 0; s < 3; ++s) m[s] = fx_mean(s, gx[xr][10 + s][q], gx[xr][10 + s][q + 1]);
             }
             if (!P.periodic_x) {
                 // bounce-back on the walls: populations entering the fluid take their opposites' values
@@ -564,7 +569,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(const i64 *__
 #pragma unroll
             for (int s = 0; s < 10; ++s) v[s] = fx_normal<1>(s, gy[yr][s][lane], gy[yr + 1][s][lane], P.my, P.my);
 #pragma unroll
-            for (int s = 0; s < 3; ++s) m[s] = (gy[yr][10 + s][lane] + gy[yr + 1][10 + s][lane]) >> 1;
+            for (int s = 0; s < 3; ++s) m[s] = fx_mean(s, gy[yr][10 + s][lane], gy[yr + 1][10 + s][lane]);
             fx_face_flux<1, FAX>(P, v, m);
             const int b = k & 1;
 #pragma unroll
@@ -608,7 +613,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(const i64 *__
                 if (n < 10)
                     v[n < 10 ? n : 0] = fx_normal<2>(n < 10 ? n : 0, o, x, P.mz, P.mz);
                 else
-                    m[n < 10 ? 0 : n - 10] = (o + x) >> 1;
+                    m[n < 10 ? 0 : n - 10] = fx_mean(n - 10, o, x);
             });
             fx_face_flux<2, FAX>(P, v, m);
             if (k >= kb) {
