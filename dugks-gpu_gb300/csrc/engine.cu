@@ -1209,9 +1209,18 @@ int make_fixed_plan(dg_ctx *h)
     };
     P.cell = force(c.bw0, c.bw2, c.hdt * F);
     P.face = force(c.fw0 / s, c.fw2 / s, 0.5 * c.hdt * F);
-    // bw1 = 1 - bw2 to the last place: the rest population takes the difference of the
-    // density and the others
-    P.bw1 = fx_split(i64((1ull << 63) - 9ull * u64(P.cell.B)));
+    // Stage (a) with the doubles that the reference has for bw1, bw2 and the weights: 1/18
+    // (1 + e1), 1/36 (1 + e1) and 1/3 (1 + e0) (src/dugks.cu:97-125, src/lbm_d3q19.cu:17-19).
+    // drift: what the sum of f-bar-plus then misses of the density.
+    const double w18 = 1.0 / 18.0, e1 = std::fma(w18, 18, -1), e0 = std::fma(1.0 / 3.0, 3, -1);
+    const double hi = std::min(c.bw2 * w18, 0.4999), lo = std::fma(c.bw2, w18, -hi);
+    P.cell.B = i64(std::llrint(std::ldexp(hi, 64))) + i64(std::llrint(std::ldexp(lo, 64)));
+    if (!(std::fabs(c.bw1) < 1 - 0x1p-31)) fit = false;
+    P.bw1 = fx_split(fit ? i64(std::llrint(std::ldexp(c.bw1, 63))) : 0);
+    const double sum = c.bw1 + c.bw2, rest = (c.bw1 - (sum - c.bw2)) + (c.bw2 - (sum - (sum - c.bw2)));  // sum + rest exactly
+    const double drift = (sum - 1) + rest + c.bw2 * (e1 + (e0 - e1) / 3);
+    if (!(std::fabs(drift) < 0x1p-48)) fit = false;
+    P.drift = fit ? int(std::lrint(std::ldexp(drift, 78))) : 0;
     P.third = fx_split(0x5555555555555555ll);
     const double ty = c.hdt / c.dy, tz = c.hdt / c.dz;
     P.ty = weight(ty); P.tz = weight(tz);

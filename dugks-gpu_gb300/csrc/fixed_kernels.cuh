@@ -10,10 +10,11 @@
 // 1.22 ms here (stage (a) 0.21, flux 1.01); 64^3 box 0.63 -> 0.104 ms, 64 x 32 x 32
 // channel 0.229 -> 0.037 ms.
 //
-// Error of the state against an 80-bit run of the same scheme (relative 2-norm):
-// 5e-17 after one step, the rounding of the stored values (FP64 kernels 2.4e-16 to
-// 3.2e-16), 6e-16 to 2e-15 after 1000 steps (2e-14 to 2.3e-13); total mass drifts by
-// 1e-17 in 1000 steps between walls (2e-13).
+// Error of the state against an 80-bit run of the scheme with the reference's double
+// coefficients (relative 2-norm; periodic box and laminar channel): 5e-17 after one step, the
+// rounding of the stored values (FP64 kernels 1.7e-16 to 2.2e-16), 4e-16 to 1e-15 after 1000
+// steps (5.6e-14), 4e-15 to 1.3e-14 after 10^4 (5.6e-13); total mass follows those coefficients,
+// 1.4e-16 a step in the channel (tests/test_gpu_fixed_long.py).
 //
 // Range.  The scaling is chosen for states near unit density: every f-tilde and
 // f-bar-plus (wall ghosts included) within (FX_LO, FX_HI) w_p, which holds up to
@@ -56,6 +57,7 @@ struct FxParams {
     int periodic_x;
     int esh;                // fluxes are held divided by fw1 2^esh, fw1 2^esh in (1/4, 1]
     int stretched;          // x-face weights of the c_x = 0 populations differ from 1/2
+    int drift;              // sum f-bar-plus / rho - 1, scaled 2^78 (see fx_stage_a)
     FxForce cell, face;
     FxMul bw1;              // 2 f (2^63) -> bw1 f (2^62)
     FxMul third;            // 1/3
@@ -145,14 +147,17 @@ DG_UNROLL
 }
 
 // f-bar-plus of one cell from f-tilde: bw1 f + K feq-polynomial; the rest
-// population from the density (sum f-bar-plus = rho exactly).
+// population from the density: the sum of f-bar-plus is rho (1 + drift).  The scheme
+// conserves mass (drift 0), but its coefficients as doubles (weights, bw1, bw2) miss their
+// sums by about 1e-16, which is 1.4e-12 of the mass after 10^4 steps, and the parity of this
+// form is with the reference's step, which has these doubles (make_fixed_plan in engine.cu).
 template <int FAX>
 DG_FX void fx_stage_a(const FxParams &P, const i64 v[NPOP], i64 ob[NPOP])
 {
     i64 rho, j[3];
     fx_moments(v, rho, j);
     const FxEq E = fx_eq<FAX>(rho, j, P.cell, P.third);
-    i64 rest = rho;
+    i64 rest = rho + (fx_wide(int(rho >> 32), P.drift, 1ll << 45) >> 46);
 DG_UNROLL
     for (int p = 1; p < NPOP; ++p) {
         const int q = opp(p);
