@@ -103,16 +103,15 @@ __global__ void __launch_bounds__(1024) stats_partials_kernel(const S *__restric
 }
 
 // The same with density and velocity of a cell in fixed point (fixed.cuh) where its
-// values are in the range of fixed_kernels.cuh, and its extremes as integers: 14
-// FP64 instructions per cell (four conversions, ten sums) instead of about 130, most
-// of them the three divisions.  Other cells take stats_cell.  Both sums of products
-// and the reduction stay in FP64.  256 x 128 x 128 FP64 cells: 125 us (5.1 TB/s; the
-// reads alone take 95 us at the copy rate) against about 0.9 ms.  shift: hdt F,
-// scaled 2^60.
-struct FxShift {
-    i64 s[3];
-};
-
+// values are in the range of fixed_kernels.cuh, and its extremes as integers: 11
+// FP64 instructions per cell (the density's conversion, ten sums), one more per axis with a
+// force, instead of about 130, most of them the three divisions.  The moments are exact; a
+// velocity is their quotient formed at a scale of its own and rounded once to FP64 (relative
+// error below 2^-52 at any size, no bias).  Other cells take stats_cell.  Both sums of
+// products and the reduction stay in FP64.  dg_stats_values of 256 x 128 x 128 FP64 cells: 174
+// us, against 1654 us with FP64 cells and one chain; the reads alone take 95 us.  Bound by
+// latency at 16 warps per SM (99 registers; 24 warps, at 80, 185 us).  210 us with the
+// velocities' conversions and the test for a force as FP64 instructions.
 // one stored value, scaled 2^62 (FP64) or 2^30 (float values of 2^-7 and more are
 // multiples of 2^-30: their moments fit 32-bit integers exactly)
 __device__ __forceinline__ i64 stats_int(double x) { return fx_from_double(x); }
@@ -129,10 +128,27 @@ __device__ __forceinline__ bool stats_bad(float x, int p)
     return __float_as_uint(x) - lo >= hi - lo;
 }
 
+// The FP64 value nearest to v / 2^s, |v| < 2^63, in integer operations
+__device__ __forceinline__ double fx_pack(i64 v, int s)
+{
+    const u64 m = v < 0 ? -v : v;
+    const int c = __clzll(m);
+    const u64 t = m << (c & 63);
+    const u64 b = (t >> 11) + ((t >> 10) & 1) + (u64(1023 + 62 - c - s) << 52);  // the leading one adds 1 to the exponent
+    return __longlong_as_double(m ? i64(b) | (v & (1ll << 63)) : 0);
+}
+
+// FP64 numbers as integers that compare alike, and back
+__device__ __forceinline__ i64 stats_key(double x)
+{
+    const i64 b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double stats_unkey(i64 k) { return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll)); }
+
 template <class T, class S>
 __global__ void __launch_bounds__(256) stats_fx_kernel(const S *__restrict__ f, const StepParams<T, S> P,
-                                                       const FxShift shift, double sx, double sy, double sz,
-                                                       double *__restrict__ partial)
+                                                       double sx, double sy, double sz, double *__restrict__ partial)
 {
     using I = decltype(stats_int(T(0)));
     const int i = blockIdx.y * blockDim.x + threadIdx.x;
@@ -140,7 +156,10 @@ __global__ void __launch_bounds__(256) stats_fx_kernel(const S *__restrict__ f, 
     const FxMul third = fx_split(0x5555555555555555ll);
     double acc[NSTAT];
     stats_init(acc);
-    i64 lo[4], hi[4];
+    const double shift[3] = {sx, sy, sz};
+    // compared as integers: the compiler would compare the doubles in every cell
+    const bool forced[3] = {__double_as_longlong(sx) != 0, __double_as_longlong(sy) != 0, __double_as_longlong(sz) != 0};
+    i64 lo[4], hi[4], key[4];
 #pragma unroll
     for (int a = 0; a < 4; ++a) lo[a] = 0x7fffffffffffffffll, hi[a] = -0x7fffffffffffffffll;
     const int rows = P.ny * P.nz;
@@ -166,22 +185,28 @@ __global__ void __launch_bounds__(256) stats_fx_kernel(const S *__restrict__ f, 
             }
             constexpr int up = sizeof(I) == 8 ? 0 : 32;
             const i64 rho = i64(r) << up;
-            const FxMul M = fx_recip3(rho);  // 3 / (16 rho)
-            i64 m[4] = {rho, 0, 0, 0};
+            const FxMul M3 = fx_recip3(rho);  // 3 / (16 rho)
+            const FxMul M = fx_split(fx_mul(i64(M3.h) * (1ll << 32) + M3.l, third));
+            q[0] = fx_to_double(rho, 62);
+            key[0] = rho;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) m[a + 1] = fx_mul(fx_mul((i64(j[a]) << up) << 2, M), third) + shift.s[a];
+            for (int a = 0; a < 3; ++a) {
+                const i64 ja = i64(j[a]) << up;
+                const int n = __clzll(ja < 0 ? -ja : ja) - 2;  // |j| < 2^61: shifted to 2^61 .. 2^62
+                q[a + 1] = fx_pack(fx_madr(ja << n, M, 0), 58 + n);
+                if (forced[a]) q[a + 1] += shift[a];
+                key[a + 1] = stats_key(q[a + 1]);
+            }
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                lo[a] = min(lo[a], m[a]);
-                hi[a] = max(hi[a], m[a]);
-                q[a] = fx_to_double(m[a], a ? 60 : 62);
+                lo[a] = min(lo[a], key[a]);
+                hi[a] = max(hi[a], key[a]);
             }
         } else {
             double d[NPOP];
-            const double s[3] = {sx, sy, sz};
 #pragma unroll
             for (int p = 0; p < NPOP; ++p) d[p] = double(v[p]);
-            stats_cell(d, s, q);
+            stats_cell(d, shift, q);
             stats_extremes(acc, q);
         }
         stats_add(acc, q);
@@ -189,8 +214,8 @@ __global__ void __launch_bounds__(256) stats_fx_kernel(const S *__restrict__ f, 
     if (lo[0] <= hi[0]) {
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            acc[10 + a] = fmin(acc[10 + a], fx_to_double(lo[a], a ? 60 : 62));
-            acc[14 + a] = fmax(acc[14 + a], fx_to_double(hi[a], a ? 60 : 62));
+            acc[10 + a] = fmin(acc[10 + a], a ? stats_unkey(lo[a]) : fx_to_double(lo[a], 62));
+            acc[14 + a] = fmax(acc[14 + a], a ? stats_unkey(hi[a]) : fx_to_double(hi[a], 62));
         }
     }
     double *out = partial + (size_t)blockIdx.x * NSTAT * P.nx + i;

@@ -173,7 +173,7 @@ cudaError_t Kern<T, S>::soa_to_aos(const S *src, double *dst, const StepParams<T
 // Smallest FP64 state whose statistics take the fixed-point cells and the parallel
 // reduction chains.  Those are faster at every size (64 x 32 x 32 cells: about 45 us
 // with the host copy, against 100 us with FP64 cells and one chain; 256 x 128 x 128:
-// 160 us, against 1.66 ms), but the laminar example's profiles-2.dat, recorded byte
+// 174 us, against 1.65 ms), but the laminar example's profiles-2.dat, recorded byte
 // for byte on 65,536 cells, holds the FP64 rounding of covariances near 1e-17: twice
 // that grid is where the FP64 cells start to cost more than a launch-bound step.
 constexpr long long kStatsFxCells = 1 << 17;
@@ -182,7 +182,7 @@ template <class T, class S>
 bool Kern<T, S>::stats_fp64_cells(const StepParams<T, S> &P, double hdt, const double F[3])
 {
     for (int a = 0; a < 3; ++a)
-        if (!(std::fabs(F[a] * hdt) < 0.1)) return true;  // beyond the fixed point's velocities
+        if (!(std::fabs(F[a] * hdt) < 0.1)) return true;  // the extremes of the fixed-point cells take finite velocities
     return sizeof(T) == 8 && (long long)P.nx * P.ny * P.nz < kStatsFxCells;
 }
 
@@ -195,9 +195,7 @@ cudaError_t Kern<T, S>::stats_partials(const S *f, const StepParams<T, S> &P, do
     if (stats_fp64_cells(P, hdt, F)) {
         stats_partials_kernel<T, S><<<grid, bx, 0, st>>>(f, P, hdt, F[0], F[1], F[2], partial);
     } else {
-        FxShift q;
-        for (int a = 0; a < 3; ++a) q.s[a] = i64(std::llrint(std::ldexp(F[a] * hdt, 60)));
-        stats_fx_kernel<T, S><<<grid, bx, 0, st>>>(f, P, q, F[0] * hdt, F[1] * hdt, F[2] * hdt, partial);
+        stats_fx_kernel<T, S><<<grid, bx, 0, st>>>(f, P, F[0] * hdt, F[1] * hdt, F[2] * hdt, partial);
     }
     return cudaGetLastError();
 }
