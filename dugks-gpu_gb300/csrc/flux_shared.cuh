@@ -141,14 +141,6 @@ __device__ __forceinline__ void cell_values(const StepParams<float, S> &P, const
     g[12] = (v[1].x - v[1].y) + (d.x + d.y);
 }
 
-// 1/r to within the last bit: the hardware's approximate reciprocal and one Newton step
-__device__ __forceinline__ float recip_newton(float r)
-{
-    float x;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(r));
-    return fmaf(x, fmaf(-r, x, 1.0f), x);
-}
-
 // Face equilibrium and flux divided by fw1 (src/dugks.cu:675-709, 912-943) of the 10
 // crossing populations, in place, from their face values and the sums m over the
 // others (density, t1 and t2 momentum).  face_flux of dugks_kernels.cuh for float.
@@ -177,7 +169,7 @@ __device__ __forceinline__ void face_flux_sh(const StepParams<float, S> &P, floa
         j[1] = m[2] + (s34.x - s34.y);
         j[2] = (v[0] - v[1]) + (n.x + n.y);
     }
-    const float inv = recip_newton(r);
+    const float inv = recip(r);
     float u = j[0] * inv, vv = j[1] * inv, w = j[2] * inv;
     float B = P.fw2s;
     float F[3] = {P.F[0], P.F[1], P.F[2]};
