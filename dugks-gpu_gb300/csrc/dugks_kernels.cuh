@@ -547,14 +547,11 @@ __device__ __forceinline__ void fbar_cell(const StepParams<T, S> &P, int ic, int
     }
 }
 
-// Stage (a) in FP64: the interior of f-bar-plus (fb_ghost_kernel fills the ghost
-// layer).  One block of the grid, block (bx, j, k) of bdim threads; tid: the thread
-// within it.
+// Stage (a) in FP64: the interior of f-bar-plus (fb_ghost_kernel fills the ghost layer).
 template <class T, class S>
-__device__ __forceinline__ void fbar_block(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> &P,
-                                           int tid, int bx, int bdim, int j, int k)
+__global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> P)
 {
-    const int i = bx * bdim + tid;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
     if (i >= P.nx) return;
     const long long c = ((long long)k * P.ny + j) * P.pitch + i;
     const long long cb = ((long long)(k + 1) * (P.ny + 2) + (j + 1)) * P.pitch_b + i + 1;
@@ -564,12 +561,6 @@ __device__ __forceinline__ void fbar_block(const S *__restrict__ f, S *__restric
     fbar_cell(P, i, j, k, v, ob);
 #pragma unroll
     for (int p = 0; p < NPOP; ++p) fb[p * P.ps_b + cb] = P.codec.encode_h(p, ob[p], 0u);
-}
-
-template <class T, class S>
-__global__ void __launch_bounds__(256) fbar_kernel(const S *__restrict__ f, S *__restrict__ fb, const StepParams<T, S> P)
-{
-    fbar_block<T, S>(f, fb, P, threadIdx.x, blockIdx.x, blockDim.x, blockIdx.y, blockIdx.z);
 }
 
 // Stage (a) of the float forms, one thread per cell.  GHOST = 2: the interior of
@@ -819,19 +810,6 @@ struct FbRead {
     __device__ __forceinline__ T dec(int p, T x) const { return codec.dec(p, x); }
     __device__ __forceinline__ T dec_e(int p, T x) const { return codec.dec_e(p, x); }
     __device__ __forceinline__ float2 dec_e2(int p, int q, float2 x) const { return codec.dec_e2(p, q, x); }
-};
-
-// The same for f-bar-plus written earlier in the same launch by other SMs (coherent loads)
-template <class T, class S>
-struct FbReadCoherent : FbRead<T, S> {
-    using FbRead<T, S>::fb;
-    using FbRead<T, S>::ps;
-    using FbRead<T, S>::codec;
-    __device__ __forceinline__ T operator()(int p, long long row, int col) const
-    {
-        return codec.dec(p, T(__ldcg(fb + p * ps + row + col)));
-    }
-    __device__ __forceinline__ T raw(int p, long long row, int col) const { return T(__ldcg(fb + p * ps + row + col)); }
 };
 
 // 19 reconstructed values of one face, trilinear characteristic interpolation
@@ -1582,7 +1560,7 @@ __device__ __forceinline__ void face_fluxes(const StepParams<T, S> &P, const RD 
     face_flux<T, S, AX, FF>(P, v, out, FF ? face_field<T, S, AX>(P, i, j, k) : T(0));
 }
 
-template <class T, class S, int W, int RECON, bool FF, class RD = FbRead<T, S>>
+template <class T, class S, int W, int RECON, bool FF>
 __device__ __forceinline__ void flux_block(const S *__restrict__ fb, const S *f_in, S *f_out,
                                            const StepParams<T, S> &P, int kchunk, int bx, int by, int bz)
 {
@@ -1595,7 +1573,7 @@ __device__ __forceinline__ void flux_block(const S *__restrict__ fb, const S *f_
     const int j0 = by * (W - 1) + 1;      // first row of the tile (1-based)
     const int kb = bz * kchunk + 1;
     const int ke = min(kb + kchunk, nz + 1);
-    const RD R{fb, P.ps_b, P.pitch_b, ny, nz, P.codec};
+    const FbRead<T, S> R{fb, P.ps_b, P.pitch_b, ny, nz, P.codec};
 
     // warps 1..W-1: cell (gi, gj); warp 0: halo
     const int gi = i0 + lane;

@@ -167,7 +167,8 @@ struct dg_ctx {
     // its per-column table and flags on the device
     std::unique_ptr<FxPlan> fx;
     FxMul *fx_tab = nullptr;
-    int *fx_flag = nullptr;  // [0] range flag, [1] last step redone in FP64
+    int *fx_words = nullptr;  // FXW_WORDS device words
+    StepParams<double, double> *fx_step = nullptr;
     bool fb_fixed = false;  // f-bar-plus holds fixed-point values
     bool fb_shown = false;  // the caller holds f-bar-plus's address: it is kept in FP64
 
@@ -186,7 +187,8 @@ struct dg_ctx {
         if (step_graph) cudaGraphExecDestroy(step_graph);
         if (cap_stream) cudaStreamDestroy(cap_stream);
         if (fx_tab) cudaFree(fx_tab);
-        if (fx_flag) cudaFree(fx_flag);
+        if (fx_words) cudaFree(fx_words);
+        if (fx_step) cudaFree(fx_step);
         if (spec) cudaFree(spec);
         if (spec_order) cudaFree(spec_order);
         if (spec_off) cudaFree(spec_off);
@@ -673,7 +675,7 @@ cudaError_t launch_stage_a(dg_ctx *h, const S *in, const StepParams<T, S> &P, cu
 {
     if constexpr (std::is_same<S, double>::value) {
         h->fb_fixed = uses_fixed(h);
-        if (h->fb_fixed) return launch_fixed_a(*h->fx, in, h->fb, h->fx_flag, st);
+        if (h->fb_fixed) return launch_fixed_a(*h->fx, in, h->fb, h->fx_words, st);
     }
     return Kern<T, S>::fbar(in, static_cast<S *>(h->fb), P, st);
 }
@@ -681,7 +683,7 @@ template <class T, class S>
 cudaError_t launch_flux(dg_ctx *h, const S *in, S *out, const StepParams<T, S> &P, cudaStream_t st)
 {
     if constexpr (std::is_same<S, double>::value) {
-        if (h->fb_fixed) return launch_fixed_flux(*h->fx, in, out, h->fb, h->fx_flag, st);
+        if (h->fb_fixed) return launch_fixed_flux(*h->fx, in, out, h->fb, h->fx_words, st);
     }
     return Kern<T, S>::flux(static_cast<S *>(h->fb), in, out, P, h->recon, h->have_tmap ? &h->tmap : nullptr, st);
 }
@@ -1248,10 +1250,13 @@ int make_fixed_plan(dg_ctx *h)
     if (!fit) return DG_OK;
     CK(cudaMalloc(&h->fx_tab, tab.size() * sizeof(FxMul)), "cudaMalloc (fixed-point table)");
     CK(cudaMemcpy(h->fx_tab, tab.data(), tab.size() * sizeof(FxMul), cudaMemcpyHostToDevice), "table upload");
-    CK(cudaMalloc(&h->fx_flag, 2 * sizeof(int)), "cudaMalloc (range flag)");
-    CK(cudaMemset(h->fx_flag, 0, 2 * sizeof(int)), "cudaMemset (range flag)");
-    P.tab = h->fx_tab;
+    CK(cudaMalloc(&h->fx_words, FXW_WORDS * sizeof(int)), "cudaMalloc (step words)");
+    CK(cudaMemset(h->fx_words, 0, FXW_WORDS * sizeof(int)), "cudaMemset (step words)");
     L->D = params_for<double, double>(h, 0);
+    CK(cudaMalloc(&h->fx_step, sizeof(L->D)), "cudaMalloc (FP64 step parameters)");
+    CK(cudaMemcpy(h->fx_step, &L->D, sizeof(L->D), cudaMemcpyHostToDevice), "step parameters upload");
+    P.tab = h->fx_tab;
+    P.step = h->fx_step;
     CK(fixed_plan_setup(*L), "fixed-point kernel setup");
     h->fx = std::move(L);
     return DG_OK;
@@ -1932,10 +1937,10 @@ static const void *show_fb(dg_t *h)
     if (h->fx && !h->fb_shown) {
         if (h->fb_fixed) {
             const size_t bytes = size_t(h->ps_b) * 19 * sizeof(double);
-            int redone = 0;
-            cudaError_t e = cudaMemcpyAsync(&redone, h->fx_flag + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+            int fixed = 0;
+            cudaError_t e = cudaMemcpyAsync(&fixed, h->fx_words + FXW_FIXED, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-            if (e == cudaSuccess && !redone) {
+            if (e == cudaSuccess && fixed) {
                 double *tmp = nullptr;
                 e = cudaMalloc(&tmp, bytes);
                 if (e == cudaSuccess) e = launch_fixed_decode(*h->fx, h->fb, tmp, h->stream);

@@ -24,8 +24,8 @@
 // the others at the lower end) and the equilibrium polynomial (< 3.9) at every cell
 // and face, so that no sum or product overflows (the sums over the populations that do not
 // cross a face reach 1.32, see fx_mean).  Stage (a) checks the box per value
-// (NaN and infinities fail it) and raises a device flag; the flux kernel then does
-// nothing and fp64_redo_kernel does the whole step in FP64.  The parameters have to
+// (NaN and infinities fail it) and raises a device flag; the flux kernel then does stage
+// (a) again in FP64 and fp64_redo_kernel the rest of the step.  The parameters have to
 // fit too (make_fixed_plan in engine.cu): a single force axis, interpolation weights
 // within (0, 1/2), dt/dx below about 1/2.
 #pragma once
@@ -35,6 +35,9 @@
 
 #include "d3q19.cuh"
 #include "fixed.cuh"
+#ifdef __CUDACC__
+#include "dugks_kernels.cuh"
+#endif
 
 namespace dg {
 
@@ -66,6 +69,7 @@ struct FxParams {
     FxMul cy, cz;           // fw1 2^esh dt/dy, dt/dz
     FxMul q0, q1;           // wall ghosts: extrapolation weight q, less 2
     const FxMul *tab;       // [FXT_ROWS][nx + 2] per column / x face
+    const void *step;       // StepParams<double, double> on the device, for steps out of range
 };
 constexpr int FXT_TXP = 0;  // transverse x weight of c_x > 0 at column i
 constexpr int FXT_TXM = 1;  // ... of c_x < 0
@@ -218,11 +222,16 @@ __device__ __forceinline__ bool fx_bad(i64 x, int p)
     return unsigned(x >> 32) - lo >= hi - lo;
 }
 
+// Device words of a handle: the range flag, raised by stage (a) and lowered by the step
+// that it redoes; what f-bar-plus holds after the last step (0: FP64, 1: fixed point); CTAs of
+// fp64_redo_kernel that have read the flag.
+constexpr int FXW_FLAG = 0, FXW_FIXED = 1, FXW_DONE = 2, FXW_WORDS = 3;
+
 // Stage (a), one thread per cell, x ghost columns included.  xoff: cells shifted by
 // one thread when nx = 1 (mod 32), so that cells nx-2 and nx-1 share a warp.
 template <int FAX>
 __global__ void __launch_bounds__(128) fbar_fx_kernel(const double *__restrict__ f, i64 *__restrict__ fb,
-                                                      const FxParams P, int xoff, int *flag)
+                                                      const FxParams P, int xoff, int *words)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x - xoff;
     const int j = blockIdx.y, k = blockIdx.z, nx = P.nx;
@@ -237,6 +246,8 @@ __global__ void __launch_bounds__(128) fbar_fx_kernel(const double *__restrict__
         bad |= fx_bad_double(x, p);
         v[p] = fx_from_double(x);
     }
+    // another block's cell is out of range already: nothing here is read
+    if (__any_sync(0xffffffffu, __ldcg(words + FXW_FLAG))) return;
     fx_stage_a<FAX>(P, v, ob);
     i64 *row = fb + ((long long)k * P.ny + j) * P.rs;
     i64 *dst = row + fx_col(ic);
@@ -270,7 +281,7 @@ __global__ void __launch_bounds__(128) fbar_fx_kernel(const double *__restrict__
             }
         }
     }
-    if (bad && in) atomicOr(flag, 1);
+    if (bad && in) atomicOr(words + FXW_FLAG, 1);
 }
 
 // Where f-bar-plus is read around a cell: plane pointers k-1..k+1, row and column
@@ -374,6 +385,49 @@ __device__ __forceinline__ void fx_bar(int id, int threads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Stage (a) in FP64 with its ghost layer (fbar_kernel and fb_ghost_kernel in one pass), tasks
+// t, t + step, ...: first every cell with its periodic images, then, between walls, the
+// ghost of every row's end, which forms the values of its two cells again (in tasks of
+// their own: beside a row's other cells they would take the whole warp's time twice).  A
+// call, so that its registers are not the flux kernel's.
+template <int R>
+__device__ __noinline__ void fp64_stage_a(const double *f, double *fb, const StepParams<double, double> &P, long long t,
+                                          long long step)
+{
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
+    const long long n = (long long)nx * ny * nz, tasks = n + (P.periodic_x ? 0 : 2LL * ny * nz);
+    for (; t < tasks; t += step) {
+        const bool cell = t < n;
+        const long long r = cell ? t / nx : (t - n) >> 1;
+        const int i = cell ? int(t - r * nx) : ((t - n) & 1 ? nx - 1 : 0), j = int(r % ny), k = int(r / ny);
+        const double q = i == 0 ? P.q0 : P.q1;
+        double ob[NPOP];
+#pragma unroll 1
+        for (int m = cell; m < 2; ++m) {  // the cell itself last
+            const int c = m ? i : (i == 0 ? 1 : nx - 2);
+            const double *src = f + ((long long)k * ny + j) * P.pitch + c;
+            double v[NPOP], o[NPOP];
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) v[p] = src[p * P.ps];
+            fbar_cell(P, c, j, k, v, o);
+#pragma unroll
+            for (int p = 0; p < NPOP; ++p) ob[p] = cell ? o[p] : (m ? q * o[p] + ob[p] : (1.0 - q) * o[p]);
+        }
+        // column I of this row and plane, and its periodic images (rows 0, ny + 1, planes 0, nz + 1)
+        auto put = [&](int I) {
+            for (int K = k == nz - 1 ? 0 : k + 1; K <= nz + 1; K = K == 0 ? k + 1 : (K == k + 1 && k == 0 ? nz + 1 : nz + 2))
+                for (int J = j == ny - 1 ? 0 : j + 1; J <= ny + 1; J = J == 0 ? j + 1 : (J == j + 1 && j == 0 ? ny + 1 : ny + 2)) {
+                    double *d = fb + ((long long)K * (ny + 2) + J) * P.pitch_b + I;
+#pragma unroll
+                    for (int p = 0; p < NPOP; ++p) d[p * P.ps_b] = ob[p];
+                }
+        };
+        put(cell ? i + 1 : (i == 0 ? 0 : nx + 1));
+        if (cell && P.periodic_x && i == 0) put(nx + 1);
+        if (cell && P.periodic_x && i == nx - 1) put(0);
+    }
+}
+
 // Stages (b)-(e).  A CTA holds R rows of 32 cells (lane = x) and marches a chunk of z
 // planes.  Each axis has warps of its own: R + 1 for x (the last one, the halo warp, the
 // columns left and right of the tile), R + 2 for y (the rows -1 .. R), R for z.  Per plane:
@@ -396,8 +450,8 @@ __device__ __forceinline__ void fx_bar(int id, int threads)
 // planes over one CTA per SM (1.09 ms: tiles next to each other, at different planes, no
 // longer share rows in L2).
 template <int R, int FAX>
-__global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(const i64 *__restrict__ fb, const double *f_in,
-                                                                   double *f_out, const FxParams P, const int *flag)
+__global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, const double *f_in, double *f_out,
+                                                                   const FxParams P, const int *words)
 {
     using L = FxSmem<R>;
     extern __shared__ __align__(16) i64 sm[];
@@ -407,7 +461,14 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(const i64 *__
     i64(*fxz)[R][4][33] = reinterpret_cast<i64(*)[R][4][33]>(sm + L::XZ);            // x fluxes of populations 11..14
     i64(*xs0)[R][6] = reinterpret_cast<i64(*)[R][6]>(sm + L::X0);                    // -x fluxes of the first column, 1, 2, 7..10
     i64(*dzs)[R][4][32] = reinterpret_cast<i64(*)[R][4][32]>(sm + L::DZ);            // z differences of populations 15..18
-    if (*flag) return;  // a value out of range: the step is redone in FP64
+    if (words[FXW_FLAG]) {  // a value out of range: fp64_redo_kernel does the rest of the step
+        // a warp takes every n-th 32 tasks, neighbours on different SMs: an incomplete last round spreads over all
+        const long long ctas = (long long)gridDim.x * gridDim.y * gridDim.z;
+        const long long cta = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
+        fp64_stage_a<R>(f_in, reinterpret_cast<double *>(fb), *static_cast<const StepParams<double, double> *>(P.step),
+                        (threadIdx.y * ctas + cta) * 32 + threadIdx.x, ctas * (32 * (3 * R + 3)));
+        return;
+    }
 
     const int lane = threadIdx.x, wr = threadIdx.y;
     const int nx = P.nx, ny = P.ny, nz = P.nz, xs = nx + 2;

@@ -11,7 +11,7 @@ struct FxPlan {
     FxParams P;
     int fax;          // force axis (3: none)
     int flux_rows, flux_chunks;  // tile rows and z chunks of the flux kernel
-    int redo_blocks;  // cooperative grid of the redo kernel
+    int redo_blocks, redo_kchunk;  // grid and z chunk of the redo kernel
     StepParams<double, double> D;
 };
 
@@ -20,10 +20,9 @@ cudaError_t fixed_plan_setup(FxPlan &L);
 
 // One step f_in -> f_out (which may be the same array) in two calls: stage (a);
 // flux / update and the FP64 redo that returns at once when the state was in
-// range.  flag: two words of the handle, the range flag (0 between steps) and whether the
-// last step was redone in FP64.
-cudaError_t launch_fixed_a(const FxPlan &L, const double *f_in, void *fb, int *flag, cudaStream_t st);
-cudaError_t launch_fixed_flux(const FxPlan &L, const double *f_in, double *f_out, void *fb, int *flag, cudaStream_t st);
+// range.  words: FXW_WORDS words of the handle, zero at first.
+cudaError_t launch_fixed_a(const FxPlan &L, const double *f_in, void *fb, int *words, cudaStream_t st);
+cudaError_t launch_fixed_flux(const FxPlan &L, const double *f_in, double *f_out, void *fb, int *words, cudaStream_t st);
 
 // f-bar-plus of the last fixed-point step as FP64 in the layout of StepParams, ghosts included
 cudaError_t launch_fixed_decode(const FxPlan &L, const void *fb, double *dst, cudaStream_t st);

@@ -1,47 +1,41 @@
 // Launchers of the fixed-point FP64 step (fixed_kernels.cuh) and of the FP64
 // kernel that redoes a step whose state left its range.
-#include <cooperative_groups.h>
-
 #include "fixed_launch.cuh"
 #include "launch_impl.cuh"
 
 namespace dg {
 namespace {
 
-// A whole FP64 step in one cooperative launch, run by every step of the fixed-point
-// path behind its two kernels: returns at once unless stage (a) raised the flag.
-// Then f-tilde is still the step's input, and stage (a), the ghost layer and the
-// flux / update follow with grid-wide barriers in between; the flag is lowered.
-// flag[1]: whether the last step was redone (f-bar-plus is then FP64).
-template <int W, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB) fp64_redo_kernel(const double *f_in, double *f_out, double *fb,
-                                                                 const StepParams<double, double> P, int *flag)
+constexpr int REDO_W = TileCfg<double, double>::W, REDO_MINB = TileCfg<double, double>::MINB;
+
+// Stages (b)-(e) in FP64 of a step out of range, whose f-bar-plus the flux kernel has formed
+// in FP64: the tiles of flux_kernel, each CTA every gridDim.x-th.  Run behind every
+// fixed-point flux kernel, it returns at once after a step in range.  (An ordinary launch: a
+// step needs no more of the GPU than is free.)  A step out of range takes, with all three
+// kernels, 237 us on 64 x 32 x 32 cells, 683 us on 64^3 and 6.76 ms on 256 x 128 x 128, against
+// 221, 635 and 6.63 with the FP64 kernels alone; as one cooperative launch with grid-wide
+// barriers it took 749, 840 and 7.02.
+__global__ void __launch_bounds__(32 * REDO_W, REDO_MINB)
+    fp64_redo_kernel(const double *__restrict__ fb, const double *f_in, double *f_out, const StepParams<double, double> P,
+                     int kc, int *words)
 {
-    const int tid = threadIdx.y * 32 + threadIdx.x, nb = gridDim.x;
-    const int redo = flag[0];
-    if (blockIdx.x == 0 && tid == 0) flag[1] = redo;
-    if (!redo) return;
-    namespace cg = cooperative_groups;
-    const cg::grid_group grid = cg::this_grid();
-    const int gx = (P.nx + 32 * W - 1) / (32 * W);
-    const long long blocks = (long long)gx * P.ny * P.nz;
-    for (long long b = blockIdx.x; b < blocks; b += nb) {
-        const long long r = b / gx;
-        fbar_block<double, double>(f_in, fb, P, tid, int(b - r * gx), 32 * W, int(r % P.ny), int(r / P.ny));
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    if (!__ldcg(words + FXW_FLAG)) {
+        if (blockIdx.x == 0 && tid == 0) words[FXW_FIXED] = 1;
+        return;
     }
-    grid.sync();
-    const long long ghosts = fb_ghosts(P.nx, P.ny, P.nz);
-    for (long long q = (long long)blockIdx.x * (32 * W) + tid; q < ghosts; q += (long long)nb * (32 * W))
-        fb_ghost_cell(fb, P, q);
-    grid.sync();
-    if (blockIdx.x == 0 && tid == 0) flag[0] = 0;
-    const int tx = (P.nx + 31) / 32, ty = (P.ny + W - 2) / (W - 1);
-    constexpr int kc = 8;
+    __syncthreads();
+    // the last CTA to have read the flag lowers it
+    if (tid == 0 && atomicAdd(words + FXW_DONE, 1) == int(gridDim.x) - 1) {
+        words[FXW_FLAG] = 0;
+        words[FXW_FIXED] = 0;
+        words[FXW_DONE] = 0;
+    }
+    const int tx = (P.nx + 31) / 32, ty = (P.ny + REDO_W - 2) / (REDO_W - 1);
     const long long tiles = (long long)tx * ty * ((P.nz + kc - 1) / kc);
-    for (long long b = blockIdx.x; b < tiles; b += nb) {
+    for (long long b = blockIdx.x; b < tiles; b += gridDim.x) {
         const long long r = b / tx;
-        flux_block<double, double, W, 0, false, FbReadCoherent<double, double>>(
-            fb, f_in, f_out, P, kc, int(b - r * tx), int(r % ty), int(r / ty));
+        flux_block<double, double, REDO_W, 0, false>(fb, f_in, f_out, P, kc, int(b - r * tx), int(r % ty), int(r / ty));
         __syncthreads();  // the next tile reuses the shared flux rows
     }
 }
@@ -56,8 +50,6 @@ __global__ void fx_decode_kernel(const i64 *__restrict__ fb, double *__restrict_
     double *q = dst + ((long long)(k + 1) * (P.ny + 2) + (j + 1)) * D.pitch_b + i + 1;
     for (int p = 0; p < NPOP; ++p) q[p * D.ps_b] = fx_to_double(src[p * 16]);
 }
-
-constexpr int REDO_W = 8, REDO_MINB = 2;
 
 // The flux kernel has tiles of four rows (128 registers, no spills) and of seven (80, 24
 // warps per SM, fewer rows formed twice).  A plane of a seven-row tile takes 1.65 times one
@@ -101,29 +93,29 @@ cudaError_t setup(FxPlan &L, int sms)
 }
 
 template <int FAX>
-cudaError_t stage_a(const FxPlan &L, const double *f_in, i64 *fb, int *flag, cudaStream_t st)
+cudaError_t stage_a(const FxPlan &L, const double *f_in, i64 *fb, int *words, cudaStream_t st)
 {
     const FxParams &P = L.P;
     const int xoff = P.nx % 32 == 1 ? 1 : 0;
     const int bx = P.nx + xoff >= 128 ? 128 : ((P.nx + xoff + 31) / 32) * 32;
-    fbar_fx_kernel<FAX><<<dim3((P.nx + xoff + bx - 1) / bx, P.ny, P.nz), bx, 0, st>>>(f_in, fb, P, xoff, flag);
+    fbar_fx_kernel<FAX><<<dim3((P.nx + xoff + bx - 1) / bx, P.ny, P.nz), bx, 0, st>>>(f_in, fb, P, xoff, words);
     return cudaGetLastError();
 }
 
 template <int FAX, int R>
-cudaError_t flux_rows(const FxPlan &L, const i64 *fb, const double *f_in, double *f_out, int *flag, cudaStream_t st)
+cudaError_t flux_rows(const FxPlan &L, i64 *fb, const double *f_in, double *f_out, int *words, cudaStream_t st)
 {
     const FxParams &P = L.P;
     const dim3 grid((P.nx + 31) / 32, (P.ny + R - 1) / R, L.flux_chunks);
-    flux_fx_kernel<R, FAX><<<grid, dim3(32, 3 * R + 3), FxSmem<R>::bytes, st>>>(fb, f_in, f_out, P, flag);
+    flux_fx_kernel<R, FAX><<<grid, dim3(32, 3 * R + 3), FxSmem<R>::bytes, st>>>(fb, f_in, f_out, P, words);
     return cudaGetLastError();
 }
 
 template <int FAX>
-cudaError_t flux(const FxPlan &L, const i64 *fb, const double *f_in, double *f_out, int *flag, cudaStream_t st)
+cudaError_t flux(const FxPlan &L, i64 *fb, const double *f_in, double *f_out, int *words, cudaStream_t st)
 {
-    return L.flux_rows == 4 ? flux_rows<FAX, 4>(L, fb, f_in, f_out, flag, st)
-                            : flux_rows<FAX, 7>(L, fb, f_in, f_out, flag, st);
+    return L.flux_rows == 4 ? flux_rows<FAX, 4>(L, fb, f_in, f_out, words, st)
+                            : flux_rows<FAX, 7>(L, fb, f_in, f_out, words, st);
 }
 
 }  // namespace
@@ -133,33 +125,34 @@ cudaError_t fixed_plan_setup(FxPlan &L)
     const int sms = device_sms();
     cudaError_t e = L.fax == 0 ? setup<0>(L, sms) : L.fax == 1 ? setup<1>(L, sms) : L.fax == 2 ? setup<2>(L, sms) : setup<3>(L, sms);
     int occ = 1;
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fp64_redo_kernel<REDO_W, REDO_MINB>, 32 * REDO_W, 0);
-    L.redo_blocks = sms * std::max(occ, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fp64_redo_kernel, 32 * REDO_W, 0);
+    const long long cols = (long long)((L.P.nx + 31) / 32) * ((L.P.ny + REDO_W - 2) / (REDO_W - 1));
+    const long long slots = (long long)sms * std::max(occ, 1);
+    L.redo_kchunk = choose_kchunk(L.P.nz, cols, slots);
+    L.redo_blocks = int(std::min(slots, cols * ((L.P.nz + L.redo_kchunk - 1) / L.redo_kchunk)));
     return e;
 }
 
-cudaError_t launch_fixed_a(const FxPlan &L, const double *f_in, void *fb, int *flag, cudaStream_t st)
+cudaError_t launch_fixed_a(const FxPlan &L, const double *f_in, void *fb, int *words, cudaStream_t st)
 {
     i64 *b = static_cast<i64 *>(fb);
-    return L.fax == 0   ? stage_a<0>(L, f_in, b, flag, st)
-           : L.fax == 1 ? stage_a<1>(L, f_in, b, flag, st)
-           : L.fax == 2 ? stage_a<2>(L, f_in, b, flag, st)
-                        : stage_a<3>(L, f_in, b, flag, st);
+    return L.fax == 0   ? stage_a<0>(L, f_in, b, words, st)
+           : L.fax == 1 ? stage_a<1>(L, f_in, b, words, st)
+           : L.fax == 2 ? stage_a<2>(L, f_in, b, words, st)
+                        : stage_a<3>(L, f_in, b, words, st);
 }
 
-cudaError_t launch_fixed_flux(const FxPlan &L, const double *f_in, double *f_out, void *fb, int *flag, cudaStream_t st)
+cudaError_t launch_fixed_flux(const FxPlan &L, const double *f_in, double *f_out, void *fb, int *words, cudaStream_t st)
 {
-    const i64 *b = static_cast<const i64 *>(fb);
-    const cudaError_t e = L.fax == 0   ? flux<0>(L, b, f_in, f_out, flag, st)
-                          : L.fax == 1 ? flux<1>(L, b, f_in, f_out, flag, st)
-                          : L.fax == 2 ? flux<2>(L, b, f_in, f_out, flag, st)
-                                       : flux<3>(L, b, f_in, f_out, flag, st);
+    i64 *b = static_cast<i64 *>(fb);
+    const cudaError_t e = L.fax == 0   ? flux<0>(L, b, f_in, f_out, words, st)
+                          : L.fax == 1 ? flux<1>(L, b, f_in, f_out, words, st)
+                          : L.fax == 2 ? flux<2>(L, b, f_in, f_out, words, st)
+                                       : flux<3>(L, b, f_in, f_out, words, st);
     if (e != cudaSuccess) return e;
-    double *fbd = static_cast<double *>(fb);
-    void *args[] = {const_cast<const double **>(&f_in), &f_out, &fbd, const_cast<StepParams<double, double> *>(&L.D), &flag};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fp64_redo_kernel<REDO_W, REDO_MINB>),
-                                       dim3(L.redo_blocks), dim3(32, REDO_W), args, 0, st);
+    fp64_redo_kernel<<<L.redo_blocks, dim3(32, REDO_W), 0, st>>>(static_cast<const double *>(fb), f_in, f_out, L.D,
+                                                                 L.redo_kchunk, words);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_fixed_decode(const FxPlan &L, const void *fb, double *dst, cudaStream_t st)
