@@ -123,6 +123,7 @@ struct StepParams {
     const T *ffield;             // [k][j][pitch] like one population of f-tilde; nullptr = none
     int ffaxis;
     Codec<T, S> codec;           // storage decode / encode constants
+    int *fb_fixed;               // FP64: device word, zeroed when f-bar-plus gets FP64 values; nullptr = none
 };
 
 // ---------------------------------------------------------------------------
@@ -721,6 +722,16 @@ __host__ __device__ inline long long fb_ghosts(int nx, int ny, int nz)
     return 2LL * (ny + 2) * (nz + 2) + 2LL * nx * (nz + 2) + 2LL * nx * ny;
 }
 
+// put(J, K): the stored row and plane of 0-based row j and plane k, and those of its periodic
+// images (0 and ny + 1, 0 and nz + 1)
+template <class Put>
+__device__ __forceinline__ void fb_images(int j, int k, int ny, int nz, Put put)
+{
+    for (int K = k == nz - 1 ? 0 : k + 1; K <= nz + 1; K = K == 0 ? k + 1 : (K == k + 1 && k == 0 ? nz + 1 : nz + 2))
+        for (int J = j == ny - 1 ? 0 : j + 1; J <= ny + 1; J = J == 0 ? j + 1 : (J == j + 1 && j == 0 ? ny + 1 : ny + 2))
+            put(J, K);
+}
+
 template <class T, class S>
 __device__ __forceinline__ void fb_ghost_cell(S *__restrict__ fb, const StepParams<T, S> &P, long long q)
 {
@@ -774,6 +785,7 @@ __device__ __forceinline__ void fb_ghost_cell(S *__restrict__ fb, const StepPara
 template <class T, class S>
 __global__ void __launch_bounds__(256) fb_ghost_kernel(S *__restrict__ fb, const StepParams<T, S> P)
 {
+    if (P.fb_fixed && blockIdx.x == 0 && threadIdx.x == 0) *P.fb_fixed = 0;
     fb_ghost_cell(fb, P, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 

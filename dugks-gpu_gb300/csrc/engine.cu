@@ -169,8 +169,7 @@ struct dg_ctx {
     FxMul *fx_tab = nullptr;
     int *fx_words = nullptr;  // FXW_WORDS device words
     StepParams<double, double> *fx_step = nullptr;
-    bool fb_fixed = false;  // f-bar-plus holds fixed-point values
-    bool fb_shown = false;  // the caller holds f-bar-plus's address: it is kept in FP64
+    bool fb_shown = false;  // the caller holds f-bar-plus's address: steps keep it in FP64
 
     ~dg_ctx()
     {
@@ -582,6 +581,7 @@ StepParams<T, S> make_params(const dg_ctx *h, const RefCoef<R> &c)
     P.gw = reinterpret_cast<const T *>(base + h->tab_off[8]);
     P.grad_st = (h->recon == 1 && h->mesh != 0) ? 1 : 0;
     P.err = h->dev_err;
+    P.fb_fixed = h->fx_words ? h->fx_words + FXW_FIXED : nullptr;
     P.pert_x = reinterpret_cast<const T *>(base + h->tab_off[3]);
     P.pert_y = reinterpret_cast<const T *>(base + h->tab_off[4]);
     P.pert_z = reinterpret_cast<const T *>(base + h->tab_off[5]);
@@ -674,8 +674,7 @@ template <class T, class S>
 cudaError_t launch_stage_a(dg_ctx *h, const S *in, const StepParams<T, S> &P, cudaStream_t st)
 {
     if constexpr (std::is_same<S, double>::value) {
-        h->fb_fixed = uses_fixed(h);
-        if (h->fb_fixed) return launch_fixed_a(*h->fx, in, h->fb, h->fx_words, st);
+        if (uses_fixed(h)) return launch_fixed_a(*h->fx, in, h->fb, h->fx_words, st);
     }
     return Kern<T, S>::fbar(in, static_cast<S *>(h->fb), P, st);
 }
@@ -683,7 +682,7 @@ template <class T, class S>
 cudaError_t launch_flux(dg_ctx *h, const S *in, S *out, const StepParams<T, S> &P, cudaStream_t st)
 {
     if constexpr (std::is_same<S, double>::value) {
-        if (h->fb_fixed) return launch_fixed_flux(*h->fx, in, out, h->fb, h->fx_words, st);
+        if (uses_fixed(h)) return launch_fixed_flux(*h->fx, in, out, h->fb, h->fx_words, st);
     }
     return Kern<T, S>::flux(static_cast<S *>(h->fb), in, out, P, h->recon, h->have_tmap ? &h->tmap : nullptr, st);
 }
@@ -729,7 +728,6 @@ int step_form(dg_ctx *h, int istep0, int n, cudaEvent_t *ev)
         const int rc = ensure_step_graph<T, S>(h, P);
         if (rc) return rc;
         for (; s + kGraphSteps <= n; s += kGraphSteps) CK(cudaGraphLaunch(h->step_graph, h->stream), "graph launch");
-        h->fb_fixed = uses_fixed(h);
     }
     if (ev) CK(cudaEventRecord(ev[0], h->stream), "event record");
     for (; s < n; ++s) {
@@ -771,7 +769,6 @@ int step_between_form(dg_ctx *h, int istep0, int n, const void *src, void *dst)
 double *state_staging(dg_ctx *h, size_t bytes, bool *owned)
 {
     *owned = false;
-    h->fb_fixed = false;
     if (h->fb && size_t(h->ps_b) * 19 * storage_bytes(h->prec) >= bytes) return static_cast<double *>(h->fb);
     double *tmp = nullptr;
     if (cudaMalloc(&tmp, bytes) != cudaSuccess) return nullptr;
@@ -925,7 +922,6 @@ int adjoint_form(dg_ctx *h, int istep, const void *f_n, const void *lam_next, vo
         CK(cudaMalloc(&h->dphi, h->ncell() * sizeof(double)), "cudaMalloc (field gradient)");
         CK(cudaMemsetAsync(h->dphi, 0, h->ncell() * sizeof(double), h->stream), "cudaMemset (field gradient)");
     }
-    h->fb_fixed = false;
     CK(K::adjoint(static_cast<const S *>(f_n), static_cast<S *>(h->fb), static_cast<const S *>(lam_next),
                   static_cast<S *>(lam_out), static_cast<T *>(h->adj), params_for<T, S>(h, istep),
                   h->ffield ? h->dphi : nullptr, h->have_tmap ? &h->tmap_adj : nullptr, h->stream),
@@ -1929,31 +1925,39 @@ int dg_read_dump(dg_t *h, int step)
     return dg_set_state(h, f.data());
 }
 
-// The caller gets f-bar-plus's address: from here on it is kept in FP64, and what
-// the last fixed-point step left there is converted (unless that step was redone in
-// FP64).  NULL when the conversion fails.
+// The caller gets f-bar-plus's address: from here on it holds FP64 values.  Enqueued on the
+// stream, without waiting for it (and so also while it is captured): what the last
+// fixed-point step left there is converted, by way of a copy in stream-ordered memory, and
+// fixed-point steps captured earlier are told to run in FP64 when replayed.  Where the device
+// has no memory for the copy it is made in host memory, and the call waits.  NULL when that
+// fails too.
 static const void *show_fb(dg_t *h)
 {
-    if (h->fx && !h->fb_shown) {
-        if (h->fb_fixed) {
-            const size_t bytes = size_t(h->ps_b) * 19 * sizeof(double);
-            int fixed = 0;
-            cudaError_t e = cudaMemcpyAsync(&fixed, h->fx_words + FXW_FIXED, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-            if (e == cudaSuccess && fixed) {
-                double *tmp = nullptr;
-                e = cudaMalloc(&tmp, bytes);
-                if (e == cudaSuccess) e = launch_fixed_decode(*h->fx, h->fb, tmp, h->stream);
-                if (e == cudaSuccess) e = cudaMemcpyAsync(h->fb, tmp, bytes, cudaMemcpyDeviceToDevice, h->stream);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-                if (tmp) cudaFree(tmp);
-            }
-            if (e != cudaSuccess) {
-                h->cuda_fail(e, "f-bar-plus in FP64");
-                return nullptr;
-            }
-            h->fb_fixed = false;
-        }
+    if (!h->fx || h->fb_shown) return h->fb;
+    const size_t bytes = size_t(h->fx->P.rs) * h->ny * h->nz * sizeof(i64);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(h->stream, &cap);
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    void *tmp = nullptr;
+    bool on_host = false;
+    if (e == cudaSuccess) e = cudaMallocAsync(&tmp, bytes, h->stream);
+    if (e != cudaSuccess && !capturing) {
+        cudaGetLastError();
+        on_host = true;
+        e = cudaMallocHost(&tmp, bytes);
+    }
+    if (e == cudaSuccess) {
+        e = cudaMemcpyAsync(tmp, h->fb, bytes, cudaMemcpyDefault, h->stream);
+        if (e == cudaSuccess) e = launch_fixed_decode(*h->fx, tmp, h->fb, h->fx_words, h->stream);
+        if (e == cudaSuccess && on_host) e = cudaStreamSynchronize(h->stream);
+        const cudaError_t f = on_host ? cudaFreeHost(tmp) : cudaFreeAsync(tmp, h->stream);
+        if (e == cudaSuccess) e = f;
+    }
+    if (e != cudaSuccess) {
+        h->cuda_fail(e, "f-bar-plus in FP64");
+        return nullptr;
+    }
+    if (!capturing) {  // a graph may never be launched
         h->fb_shown = true;
         h->drop_graph();
     }

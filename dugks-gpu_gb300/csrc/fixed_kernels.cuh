@@ -223,9 +223,10 @@ __device__ __forceinline__ bool fx_bad(i64 x, int p)
 }
 
 // Device words of a handle: the range flag, raised by stage (a) and lowered by the step
-// that it redoes; what f-bar-plus holds after the last step (0: FP64, 1: fixed point); CTAs of
-// fp64_redo_kernel that have read the flag.
-constexpr int FXW_FLAG = 0, FXW_FIXED = 1, FXW_DONE = 2, FXW_WORDS = 3;
+// that it redoes; what f-bar-plus holds (0: FP64, 1: fixed point); CTAs of fp64_redo_kernel that
+// have read the flag; whether the caller has f-bar-plus's address (every step runs in FP64).
+constexpr int FXW_FLAG = 0, FXW_FIXED = 1, FXW_DONE = 2, FXW_SHOWN = 3, FXW_WORDS = 4;
+__device__ __forceinline__ bool fx_in_fp64(const int *words) { return __ldcg(words + FXW_FLAG) | __ldcg(words + FXW_SHOWN); }
 
 // Stage (a), one thread per cell, x ghost columns included.  xoff: cells shifted by
 // one thread when nx = 1 (mod 32), so that cells nx-2 and nx-1 share a warp.
@@ -246,8 +247,8 @@ __global__ void __launch_bounds__(128) fbar_fx_kernel(const double *__restrict__
         bad |= fx_bad_double(x, p);
         v[p] = fx_from_double(x);
     }
-    // another block's cell is out of range already: nothing here is read
-    if (__any_sync(0xffffffffu, __ldcg(words + FXW_FLAG))) return;
+    // another block's cell is out of range already (or all steps run in FP64): nothing here is read
+    if (__any_sync(0xffffffffu, fx_in_fp64(words))) return;
     fx_stage_a<FAX>(P, v, ob);
     i64 *row = fb + ((long long)k * P.ny + j) * P.rs;
     i64 *dst = row + fx_col(ic);
@@ -413,14 +414,12 @@ __device__ __noinline__ void fp64_stage_a(const double *f, double *fb, const Ste
 #pragma unroll
             for (int p = 0; p < NPOP; ++p) ob[p] = cell ? o[p] : (m ? q * o[p] + ob[p] : (1.0 - q) * o[p]);
         }
-        // column I of this row and plane, and its periodic images (rows 0, ny + 1, planes 0, nz + 1)
         auto put = [&](int I) {
-            for (int K = k == nz - 1 ? 0 : k + 1; K <= nz + 1; K = K == 0 ? k + 1 : (K == k + 1 && k == 0 ? nz + 1 : nz + 2))
-                for (int J = j == ny - 1 ? 0 : j + 1; J <= ny + 1; J = J == 0 ? j + 1 : (J == j + 1 && j == 0 ? ny + 1 : ny + 2)) {
-                    double *d = fb + ((long long)K * (ny + 2) + J) * P.pitch_b + I;
+            fb_images(j, k, ny, nz, [&](int J, int K) {
+                double *d = fb + ((long long)K * (ny + 2) + J) * P.pitch_b + I;
 #pragma unroll
-                    for (int p = 0; p < NPOP; ++p) d[p * P.ps_b] = ob[p];
-                }
+                for (int p = 0; p < NPOP; ++p) d[p * P.ps_b] = ob[p];
+            });
         };
         put(cell ? i + 1 : (i == 0 ? 0 : nx + 1));
         if (cell && P.periodic_x && i == 0) put(nx + 1);
@@ -461,7 +460,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
     i64(*fxz)[R][4][33] = reinterpret_cast<i64(*)[R][4][33]>(sm + L::XZ);            // x fluxes of populations 11..14
     i64(*xs0)[R][6] = reinterpret_cast<i64(*)[R][6]>(sm + L::X0);                    // -x fluxes of the first column, 1, 2, 7..10
     i64(*dzs)[R][4][32] = reinterpret_cast<i64(*)[R][4][32]>(sm + L::DZ);            // z differences of populations 15..18
-    if (words[FXW_FLAG]) {  // a value out of range: fp64_redo_kernel does the rest of the step
+    if (fx_in_fp64(words)) {  // a value out of range: fp64_redo_kernel does the rest of the step
         // a warp takes every n-th 32 tasks, neighbours on different SMs: an incomplete last round spreads over all
         const long long ctas = (long long)gridDim.x * gridDim.y * gridDim.z;
         const long long cta = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);

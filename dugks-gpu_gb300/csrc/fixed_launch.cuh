@@ -24,7 +24,9 @@ cudaError_t fixed_plan_setup(FxPlan &L);
 cudaError_t launch_fixed_a(const FxPlan &L, const double *f_in, void *fb, int *words, cudaStream_t st);
 cudaError_t launch_fixed_flux(const FxPlan &L, const double *f_in, double *f_out, void *fb, int *words, cudaStream_t st);
 
-// f-bar-plus of the last fixed-point step as FP64 in the layout of StepParams, ghosts included
-cudaError_t launch_fixed_decode(const FxPlan &L, const void *fb, double *dst, cudaStream_t st);
+// f-bar-plus in FP64 in the layout of StepParams, ghosts included, if the last step left it in
+// fixed point, and fixed-point steps run in FP64 from here on.  copy: fb's first
+// rs ny nz elements.
+cudaError_t launch_fixed_decode(const FxPlan &L, const void *copy, void *fb, int *words, cudaStream_t st);
 
 }  // namespace dg

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(32 * REDO_W, REDO_MINB)
                      int kc, int *words)
 {
     const int tid = threadIdx.y * 32 + threadIdx.x;
-    if (!__ldcg(words + FXW_FLAG)) {
+    if (!fx_in_fp64(words)) {
         if (blockIdx.x == 0 && tid == 0) words[FXW_FIXED] = 1;
         return;
     }
@@ -40,15 +40,28 @@ __global__ void __launch_bounds__(32 * REDO_W, REDO_MINB)
     }
 }
 
-// f-bar-plus as the FP64 kernels store it (interior cells)
-__global__ void fx_decode_kernel(const i64 *__restrict__ fb, double *__restrict__ dst, const FxParams P,
-                                 const StepParams<double, double> D)
+// f-bar-plus as the FP64 kernels store it, a block per row: the cells, the two ghost columns
+// and their periodic images
+__global__ void __launch_bounds__(128) fx_decode_kernel(const i64 *__restrict__ copy, double *__restrict__ dst,
+                                                        const FxParams P, const StepParams<double, double> D,
+                                                        const int *words)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
-    if (i >= P.nx) return;
-    const i64 *src = fb + ((long long)k * P.ny + j) * P.rs + fx_col(i);
-    double *q = dst + ((long long)(k + 1) * (P.ny + 2) + (j + 1)) * D.pitch_b + i + 1;
-    for (int p = 0; p < NPOP; ++p) q[p * D.ps_b] = fx_to_double(src[p * 16]);
+    if (!words[FXW_FIXED]) return;
+    const int j = blockIdx.x, k = blockIdx.y, ny = P.ny, nz = P.nz;
+    const i64 *row = copy + ((long long)k * ny + j) * P.rs;
+    for (int c = threadIdx.x; c < P.nx + 2; c += blockDim.x) {
+        const int I = c == P.nx + 1 ? 0 : c + 1;  // the lower ghost is the last column there, the first here
+        const i64 *src = row + fx_col(c);
+        fb_images(j, k, ny, nz, [&](int J, int K) {
+            double *q = dst + ((long long)K * (ny + 2) + J) * D.pitch_b + I;
+            for (int p = 0; p < NPOP; ++p) q[p * D.ps_b] = fx_to_double(src[p * 16]);
+        });
+    }
+}
+__global__ void fx_shown_kernel(int *words)
+{
+    words[FXW_FIXED] = 0;
+    words[FXW_SHOWN] = 1;
 }
 
 // The flux kernel has tiles of four rows (128 registers, no spills) and of seven (80, 24
@@ -155,12 +168,11 @@ cudaError_t launch_fixed_flux(const FxPlan &L, const double *f_in, double *f_out
     return cudaGetLastError();
 }
 
-cudaError_t launch_fixed_decode(const FxPlan &L, const void *fb, double *dst, cudaStream_t st)
+cudaError_t launch_fixed_decode(const FxPlan &L, const void *copy, void *fb, int *words, cudaStream_t st)
 {
-    const int nx = L.P.nx, ny = L.P.ny, nz = L.P.nz;
-    fx_decode_kernel<<<dim3((nx + 127) / 128, ny, nz), 128, 0, st>>>(static_cast<const i64 *>(fb), dst, L.P, L.D);
-    const long long g = fb_ghosts(nx, ny, nz);
-    fb_ghost_kernel<double, double><<<unsigned((g + 255) / 256), 256, 0, st>>>(dst, L.D);
+    fx_decode_kernel<<<dim3(L.P.ny, L.P.nz), 128, 0, st>>>(static_cast<const i64 *>(copy), static_cast<double *>(fb), L.P,
+                                                           L.D, words);
+    fx_shown_kernel<<<1, 1, 0, st>>>(words);
     return cudaGetLastError();
 }
 

@@ -48,8 +48,11 @@ typedef struct dg_ctx dg_t;
                                  * of every step and of the host state transfers (dg_set_state,
                                  * dg_get_state, dg_copy_ddf, dg_dump), which may overwrite it; the
                                  * fp16 / bf16 forms between walls do not store its x ghost columns;
-                                 * fp64 handles step faster while its address has not been asked for
-                                 * (they then hold it in fixed point) */
+                                 * fp64 handles hold it in fixed point, and step faster, until its
+                                 * address is asked for: that call enqueues its conversion on the
+                                 * handle's stream (which may be capturing), by way of a copy of its
+                                 * size in stream-ordered device memory or, where there is none, in
+                                 * host memory (it then waits); NULL if neither can be had */
 #define DG_BUF_RHO 2            /* ghosted scalar macro arrays (after dg_upload_macro) */
 #define DG_BUF_UX 3
 #define DG_BUF_UY 4
