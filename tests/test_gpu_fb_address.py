@@ -1,6 +1,9 @@
 """dg_device_ptr(DG_BUF_FB) of an FP64 handle that steps in fixed point: a query that neither
 waits nor needs the stream free, with f-bar-plus in FP64 from there on."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -117,21 +120,24 @@ class _PoolProps(ctypes.Structure):  # CUmemPoolProps
                 ("usage", ctypes.c_ushort), ("reserved", ctypes.c_ubyte * 54)]
 
 
-def test_query_without_device_memory_for_the_copy():
-    """The device's stream-ordered pool limited to less than f-bar-plus (14 MB)."""
+def _query_with_a_small_pool():
     eng, orc, f0 = _pair(64, 32, 32, periods_x=0)
     eng.step(1)
     eng.sync()
     cu = ctypes.CDLL("libcuda.so.1")
-    props, pool, old = _PoolProps(allocType=1, locType=1, locId=0, maxSize=2 << 20), ctypes.c_void_p(), ctypes.c_void_p()
+    props, pool = _PoolProps(allocType=1, locType=1, locId=0, maxSize=2 << 20), ctypes.c_void_p()
     assert cu.cuMemPoolCreate(ctypes.byref(pool), ctypes.byref(props)) == 0
-    assert cu.cuDeviceGetMemPool(ctypes.byref(old), 0) == 0
     assert cu.cuDeviceSetMemPool(0, pool) == 0
-    try:
-        ptr = eng.device_ptr(pydugks.DG_BUF_FB)
-    finally:
-        assert cu.cuDeviceSetMemPool(0, old) == 0
-        assert cu.cuMemPoolDestroy(pool) == 0
+    ptr = eng.device_ptr(pydugks.DG_BUF_FB)
     assert ptr
     want = pyoracle.interior(orc.fbar(pyoracle.to_ghosted(f0)))
     assert rel_err(_fb(eng, ptr)[1:-1, 1:-1, 1:-1], want) <= TOL
+
+
+def test_query_without_device_memory_for_the_copy():
+    """The device's stream-ordered pool limited to less than f-bar-plus (14 MB).  In a process of its
+    own, which keeps that pool: once it was destroyed the driver's cuStreamSynchronize crashed."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = ("import conftest, test_gpu_fb_address as t; t._query_with_a_small_pool()")
+    r = subprocess.run([sys.executable, "-c", code], cwd=here, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
