@@ -453,6 +453,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
                                                                    const FxParams P, const int *words)
 {
     using L = FxSmem<R>;
+    constexpr int ALL = 32 * (3 * R + 3);  // threads of the CTA, which meet at barrier 0 from the branches of the three axes
     extern __shared__ __align__(16) i64 sm[];
     i64(*gx)[FXG][34] = reinterpret_cast<i64(*)[FXG][34]>(sm + L::GX);               // [row]
     i64(*gy)[FXG][32] = reinterpret_cast<i64(*)[FXG][32]>(sm + L::GY);               // [row + 1]
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
         const long long ctas = (long long)gridDim.x * gridDim.y * gridDim.z;
         const long long cta = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
         fp64_stage_a<R>(f_in, reinterpret_cast<double *>(fb), *static_cast<const StepParams<double, double> *>(P.step),
-                        (threadIdx.y * ctas + cta) * 32 + threadIdx.x, ctas * (32 * (3 * R + 3)));
+                        (threadIdx.y * ctas + cta) * 32 + threadIdx.x, ctas * ALL);
         return;
     }
 
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
 #pragma unroll
                     for (int s = 0; s < 4; ++s) fxz[b][lane][s][0] = v[6 + s];
                 }
-                __syncthreads();
+                fx_bar(0, ALL);
                 continue;
             }
 #pragma unroll
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
             i64 acc[7];  // populations 0, 1, 2, 7..10
 #pragma unroll
             for (int n = 0; n < 7; ++n) acc[n] = base(n < 3 ? n : n + 4, c);
-            __syncthreads();
+            fx_bar(0, ALL);
 #pragma unroll
             for (int n = 0; n < 7; ++n) {
                 const int p = n < 3 ? n : n + 4;
@@ -626,7 +627,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
             fx_bar(2, 32 * (R + 2));
             if (yr > R) {
                 if (k + 2 <= ke) prefetch(k + 2);
-                __syncthreads();
+                fx_bar(0, ALL);
                 continue;
             }
             // face between tile rows yr - 1 (gy[yr]) and yr
@@ -640,14 +641,14 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
 #pragma unroll
             for (int s = 0; s < 10; ++s) ysh[b][yr][s][lane] = v[s];
             if (yr == 0) {
-                __syncthreads();
+                fx_bar(0, ALL);
                 continue;
             }
             const long long c = ((long long)k * ny + min(gj, ny - 1)) * P.pitch + cc1;
             i64 acc[6];  // populations 3, 4, 15..18
 #pragma unroll
             for (int n = 0; n < 6; ++n) acc[n] = base(n < 2 ? 3 + n : 13 + n, c);
-            __syncthreads();
+            fx_bar(0, ALL);
 #pragma unroll
             for (int n = 0; n < 6; ++n) {
                 const int p = n < 2 ? 3 + n : 13 + n, s = flux_slot(1, p);
@@ -692,7 +693,7 @@ __global__ void __launch_bounds__(32 * (3 * R + 3)) flux_fx_kernel(i64 *fb, cons
                 i64 acc[6];  // populations 5, 6, 11..14
 #pragma unroll
                 for (int n = 0; n < 6; ++n) acc[n] = fx_madr(fz[n], P.cz, base(n < 2 ? 5 + n : 9 + n, c));
-                __syncthreads();
+                fx_bar(0, ALL);
 #pragma unroll
                 for (int n = 0; n < 6; ++n) {
                     const int p = n < 2 ? 5 + n : 9 + n;
