@@ -1,10 +1,12 @@
 """Statistics of slow flows: velocities far below the density's scale keep the relative
 precision of FP64, in every form, against exact integer moments."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import pydugks
-from seeded import CX, CY, CZ, W, uniform_sym
+from seeded import CX, CY, CZ, W, seeded_state, uniform_sym
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +51,25 @@ def test_slow_flows_keep_their_digits(prec, u0, force):
         # variances: <uu> and <u>^2 carry the errors of two factors each and cancel down to them
         var = (u[a] * u[a]).mean((0, 1)) - want * want
         assert np.abs(prof[:, 6 + a] - var).max() <= 4 * MEAN * float((u[a] * u[a]).max())
+
+
+def test_both_entry_points_agree_where_the_cells_are_in_fixed_point():
+    """dg_stats_values_noalloc has FP64 cells and one chain of sums at every size; here
+    dg_stats_values has neither.  Sums of n values below 1 in any order: a few n^(1/2) 2^-53."""
+    torch = pytest.importorskip("torch")
+    nx, ny, nz = 65, 64, 63
+    cfg = pydugks.make_config(nx=nx, ny=ny, nz=nz, xwidth=nx, ywidth=ny, zwidth=nz, CFL=0.5, visc=0.02, ambient_fz=1e-5)
+    eng = pydugks.Engine(cfg)
+    eng.set_state(seeded_state(nx, ny, nz, seed=6, umax=0.02, eps=0.005))
+    diag, prof = eng.stats_values()
+    out = torch.full((12 + 9 * nx + 1,), float("nan"), dtype=torch.float64, device="cuda")
+    i = eng.info
+    rc = pydugks.lib().dg_stats_values_noalloc(
+        ctypes.c_void_p(eng.device_ptr(pydugks.DG_BUF_F)), nx, ny, nz, i.pitch, i.pop_stride, i.dt / 2.0, i.ambient[0],
+        i.ambient[1], i.ambient[2], ctypes.c_void_p(out.data_ptr()), None)
+    assert rc == 0
+    torch.cuda.synchronize()
+    o = out.cpu().numpy()
+    assert o[-1] == 0
+    assert np.abs(diag - o[:12]).max() <= 1e-13
+    assert np.abs(prof - o[12:-1].reshape(nx, 9)).max() <= 1e-13
