@@ -9,6 +9,14 @@
 
 namespace dg {
 
+static int device_sms()
+{
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 template <class T, class S>
 cudaError_t Kern<T, S>::fbar(const S *f, S *fb, const StepParams<T, S> &P, cudaStream_t st)
 {
@@ -19,7 +27,7 @@ cudaError_t Kern<T, S>::fbar(const S *f, S *fb, const StepParams<T, S> &P, cudaS
     // four rows per block where that leaves two waves of blocks (one row: 0.143 -> 0.164 ms on the
     // 256 x 128 x 128 channel in FP32), one row on small grids, which need the blocks
     const long long blocks = (long long)((P.nx + xoff + bx - 1) / bx) * P.ny * P.nz;
-    const int rows = blocks * bx >= 4LL * 2 * 152 * 1024 ? 4 : 1;
+    const int rows = blocks * bx >= 4LL * 2 * 1024 * device_sms() ? 4 : 1;
     const dim3 grid((P.nx + xoff + bx - 1) / bx, (P.ny + rows - 1) / rows, P.nz);
     if constexpr (std::is_same<S, float>::value) {
         // FP32: stage (a) writes the ghost layer itself (one launch)
@@ -67,14 +75,6 @@ cudaError_t Kern<T, S>::fbar(const S *f, S *fb, const StepParams<T, S> &P, cudaS
         }
     }
     return best_k;
-}
-
-static int device_sms()
-{
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
 }
 
 // z chunk of a flux kernel whose CTAs are tiles of 32 x (W-1) cells
