@@ -10,11 +10,12 @@
 // 1.22 ms here (stage (a) 0.21, flux 1.01); 64^3 box 0.63 -> 0.104 ms, 64 x 32 x 32
 // channel 0.229 -> 0.037 ms.
 //
-// Error of the state against an 80-bit run of the scheme with the reference's double
-// coefficients (relative 2-norm; periodic box and laminar channel): 5e-17 after one step, the
-// rounding of the stored values (FP64 kernels 1.7e-16 to 2.2e-16), 4e-16 to 1e-15 after 1000
-// steps (5.6e-14), 4e-15 to 1.3e-14 after 10^4 (5.6e-13); total mass follows those coefficients,
-// 1.4e-16 a step in the channel (tests/test_gpu_fixed_long.py).
+// Error of the state against the double scheme in extended precision (the reference's double
+// coefficients, no rounding of the arithmetic; relative 2-norm, channel and periodic box):
+// 5e-17 after one step, the rounding of the stored values (FP64 kernels 1.7e-16 to 2.3e-16),
+// 1.1e-16 after 100 (5.6e-15); tests/test_extended_oracle.py.  After 10^4 steps the state is
+// within 1e-14 of the oracle in double (FP64 kernels 5.6e-13), mass included, which those
+// coefficients let drift by 1.4e-16 a step in the channel; tests/test_gpu_fixed_long.py.
 //
 // Range.  The scaling is chosen for states near unit density: every f-tilde and
 // f-bar-plus (wall ghosts included) within (FX_LO, FX_HI) w_p, which holds up to

@@ -35,3 +35,15 @@ int oracle_max_threads(void) { return omp_get_max_threads(); }
 #include "dugks_oracle_impl.h"
 #undef REAL
 #undef SFX
+#undef IDX
+#undef SIDX
+
+/* Extended precision (80 bits on x86, 128 on Arm) with the double instance's coefficients:
+ * what the double-precision scheme gives without the rounding of its arithmetic. */
+#undef COEF
+#define COEF double
+#define REAL long double
+#define SFX _ld
+#include "dugks_oracle_impl.h"
+#undef REAL
+#undef SFX

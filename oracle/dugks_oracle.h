@@ -45,6 +45,9 @@ int oracle_macro_f32(const oracle_cfg *c, const float *f, float *rho, float *ux,
 int oracle_stats_f32(int nx, int ny, int nz, const float *rhg, const float *uxg, const float *uyg,
                      const float *uzg, double *diag, double *prof);
 
+/* the double scheme in extended precision (dugks_oracle.c) */
+int oracle_run_ld(const oracle_cfg *c, long double *f, int istep0, int nsteps, int nthreads);
+
 int oracle_max_threads(void);
 
 #ifdef __cplusplus

@@ -18,6 +18,9 @@
  * plane copy (src/parallel.cu:185-234 with zprev=znext=self).
  */
 
+#ifndef COEF
+#define COEF REAL
+#endif
 #define CAT2(a, b) a##b
 #define CAT(a, b) CAT2(a, b)
 #define FN(name) CAT(name, SFX)
@@ -35,14 +38,14 @@ typedef struct {
     REAL tp[19];
 } FN(coef_t);
 
-/* Coefficient block, src/dugks.cu:97-125 (and the weights, 137-142). */
+/* Coefficient block, src/dugks.cu:97-125 (and the weights, 137-142); formed in COEF. */
 static void FN(make_coef)(const oracle_cfg *c, FN(coef_t) *q)
 {
-    const REAL RT = (REAL)(1. / 3.);              /* src/lbm_d3q19.cu:21 */
-    const REAL visc = (REAL)c->visc;
-    const REAL dt = (REAL)c->dt;
-    const REAL tau = visc / RT;
-    REAL hdt = dt / 2.;
+    const COEF RT = (COEF)(1. / 3.);              /* src/lbm_d3q19.cu:21 */
+    const COEF visc = (COEF)c->visc;
+    const COEF dt = (COEF)c->dt;
+    const COEF tau = visc / RT;
+    COEF hdt = dt / 2.;
     q->visc = visc;
     q->RT = RT;
     q->hdt = hdt;

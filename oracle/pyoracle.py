@@ -50,6 +50,7 @@ def lib():
             getattr(L, f"oracle_run_{sfx}").argtypes = [P, T, ctypes.c_int, ctypes.c_int, ctypes.c_int]
             getattr(L, f"oracle_macro_{sfx}").argtypes = [P, T, T, T, T, T]
             getattr(L, f"oracle_stats_{sfx}").argtypes = [ctypes.c_int] * 3 + [T] * 4 + [_D, _D]
+        L.oracle_run_ld.argtypes = [P, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int]
         L.oracle_max_threads.restype = ctypes.c_int
         _lib = L
     return _lib
@@ -161,6 +162,14 @@ class Oracle:
     def run(self, f, istep0, nsteps, nthreads=0):
         """Advance the ghosted state f in place."""
         rc = getattr(lib(), f"oracle_run_{self.sfx}")(ctypes.byref(self.cfg), self._p(f), istep0, nsteps, nthreads)
+        assert rc == 0, rc
+        return f
+
+    def run_extended(self, f, istep0, nsteps, nthreads=0):
+        """The same for a ghosted state of extended precision (np.longdouble), with the double
+        scheme's coefficients."""
+        assert self.sfx == "f64" and f.dtype == np.longdouble and f.flags.c_contiguous and f.shape == self.shape
+        rc = lib().oracle_run_ld(ctypes.byref(self.cfg), f.ctypes.data, istep0, nsteps, nthreads)
         assert rc == 0, rc
         return f
 
