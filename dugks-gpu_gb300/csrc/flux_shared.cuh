@@ -8,7 +8,7 @@
 // axis, and the face adds the mean of two such values and the normal derivative.  The 9
 // populations that do not cross a face enter it only through its density and
 // tangential momentum, so a cell contributes their three sums.  A step of the 97 x 66 x
-// 130 channel on the stretched mesh, FP32: 0.174 -> 0.137 ms against faces that each
+// 130 channel on the stretched mesh, FP32: 0.174 -> 0.129 ms against faces that each
 // form their own derivatives.  (The trilinear reconstruction gains too, FP32 15 % a
 // step, but in another order of its lerps: its results would change in the last place
 // of FP32, so it keeps flux_tma_kernel.)
@@ -241,11 +241,10 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_sh_kernel(const __grid_cons
                                                                S *f_out, const StepParams<float, S> P, int kchunk)
 {
     using AT = TileAt<S, W>;
-    // FP32: a cell's x, y and z contributions in one go, which shares a third of their
-    // shared-memory reads, and f-tilde fetched into L2 a plane ahead (0.277 -> 0.243 ms on
-    // the 256 x 128 x 128 channel with lerps for derivatives).  In the 16-bit forms, whose
-    // widened values need more registers, both measured slower (0.306 -> 0.33 ms).
-    constexpr bool JOINT = sizeof(S) == 4;
+    // FP32: f-tilde fetched into L2 a plane ahead (256 x 128 x 128 channel 0.290 -> 0.286 ms).  A
+    // cell's x, y and z contributions in one go, which shares a third of their reads, were
+    // slower for the registers they take: 0.314 ms, FP16 0.410 against 0.370.
+    constexpr bool PREFETCH = sizeof(S) == 4;
     constexpr int R = W - 1, BXT = AT::BXT;
     extern __shared__ __align__(128) unsigned char smem[];
     S *ring = reinterpret_cast<S *>(smem);
@@ -389,30 +388,18 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_sh_kernel(const __grid_cons
         if (k >= kb) {
             // 1. contributions to the faces
             at(xoff, sm1, s0, s1);
-            if (JOINT && wr >= 1) {
-                cell_values<S, W, 0>(P, A, X, gax);
-                cell_values<S, W, 1>(P, A, X, gay);
-                A.b[1] = A.b[2];
-                cell_values<S, W, 2>(P, A, X, gzn);
+            cell_values<S, W, 0>(P, A, X, gax);
+            if (wr || lane < 2 * R) {
 #pragma unroll
-                for (int s = 0; s < SHG; ++s) {
-                    gxw[s * 34] = gax[s];
-                    gy[wr][s][lane] = gay[s];
-                }
-            } else {
-                cell_values<S, W, 0>(P, A, X, gax);
-                if (wr || lane < 2 * R) {
-#pragma unroll
-                    for (int s = 0; s < SHG; ++s) gxw[s * 34] = gax[s];
-                }
+                for (int s = 0; s < SHG; ++s) gxw[s * 34] = gax[s];
+            }
 #pragma unroll 1
-                for (int t = wr ? 0 : 1; t >= 0; --t) {  // the halo warp: the rows above and below the tile
-                    at(t ? (R + 1) * BXT + tx : yoff, sm1, s0, s1);
-                    cell_values<S, W, 1>(P, A, X, gay);
-                    float *w = &gy[t ? R + 1 : wr][0][lane];
+            for (int t = wr ? 0 : 1; t >= 0; --t) {  // the halo warp: the rows above and below the tile
+                at(t ? (R + 1) * BXT + tx : yoff, sm1, s0, s1);
+                cell_values<S, W, 1>(P, A, X, gay);
+                float *w = &gy[t ? R + 1 : wr][0][lane];
 #pragma unroll
-                    for (int s = 0; s < SHG; ++s) w[s * 32] = gay[s];
-                }
+                for (int s = 0; s < SHG; ++s) w[s * 32] = gay[s];
             }
             __syncthreads();
             issue(k + 2, sm1);  // plane k-1 is no longer read
@@ -478,7 +465,7 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_sh_kernel(const __grid_cons
         // z, between planes k and k+1
         if (wr >= 1) {
             at(xoff, sm1, s0, s1);
-            if (!JOINT || k < kb) {
+            {
                 AT B = A;
                 B.b[1] = A.b[2];
                 cell_values<S, W, 2>(P, B, X, gzn);
@@ -556,7 +543,7 @@ __global__ void __launch_bounds__(32 * W, MINB) flux_sh_kernel(const __grid_cons
                 }
             }
         }
-        if (JOINT && wr == 0 && k + 1 < ke && k + 1 >= kb) prefetch(k + 1);
+        if (PREFETCH && wr == 0 && k + 1 < ke && k + 1 >= kb) prefetch(k + 1);
         const int s = sm1;
         sm1 = s0;
         s0 = s1;

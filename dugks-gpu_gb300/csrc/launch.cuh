@@ -34,10 +34,9 @@ struct TileCfg<double, double> {
     static constexpr bool TMA = false;
 };
 
-// CTA of flux_sh_kernel (float forms, gradient reconstruction).  FP32 by (W, CTAs per SM),
-// ms per flux launch of a 256 x 128 x 128 channel, trilinear values in place of the
-// derivatives: (5, 3) 0.243, (7, 2) 0.265, (8, 2) 0.273, (4, 4) 0.29, (16, 1) 0.32; FP16:
-// (8, 2) 0.310, (6, 2) 0.32, (7, 2) 0.34, (16, 1) 0.35, (7, 3) 0.41.
+// CTA of flux_sh_kernel (float forms, gradient reconstruction).  ms per flux launch of a 256 x
+// 128 x 128 channel by (W, CTAs per SM): FP32 (5, 3) 0.286, (8, 2) 0.293, (6, 2) 0.303, (7, 2)
+// 0.316, (4, 4) 0.318, (16, 1) 0.341; FP16 (8, 2) 0.370, (6, 2) 0.391, (16, 1) 0.408, (7, 2) 0.421.
 template <class S>
 struct GradCfg {
     static constexpr int W = 8, MINB = 2;
