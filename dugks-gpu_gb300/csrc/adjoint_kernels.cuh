@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(128) adj_face_kernel(const S *__restrict__ fb,
     const FbRead<T, S> R{fb, P.ps_b, P.pitch_b, ny, nz, P.codec};
     T v[NPOP], lv[NPOP], lf;
     if (Fp64Form<T>::value)
-        face_tri_cw<T, S, AX>(P, R, F, j, k, v);  // the forward's own face values
+        face_tri_cw<T, S, AX>(P, R, F, j, k, v);  // those of the FP64 kernels (in fixed point they differ by rounding)
     else
         face_tri<T, S, AX>(P, R, F, j, k, v);
     adj_face_flux<T, S, AX>(P, v, lam_next, F, j, k, lv, lf);

@@ -225,7 +225,8 @@ __global__ void __launch_bounds__(256) stats_fx_kernel(const S *__restrict__ f, 
 
 // Ordered reduction over blocks of the statistics partials of x index i:
 // sum / min / max over b0 <= b < b1 of partial[b][s][i] (b ascending).  Shared by
-// stats_reduce_kernel and the allocation-free statistics.
+// stats_reduce_kernel, over one chain or several (launch_stats_reduce), and the
+// allocation-free statistics, over one.
 __device__ __forceinline__ double stats_combine(const double *__restrict__ partial, int b0, int b1, int nx, int i, int s)
 {
     const double *q = partial + size_t(s) * nx + i;

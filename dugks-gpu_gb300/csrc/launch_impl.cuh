@@ -171,11 +171,12 @@ cudaError_t Kern<T, S>::soa_to_aos(const S *src, double *dst, const StepParams<T
 }
 
 // Smallest FP64 state whose statistics take the fixed-point cells and the parallel
-// reduction chains.  Those are faster at every size (64 x 32 x 32 cells: about 45 us
-// with the host copy, against 100 us with FP64 cells and one chain; 256 x 128 x 128:
-// 174 us, against 1.65 ms), but the laminar example's profiles-2.dat, recorded byte
-// for byte on 65,536 cells, holds the FP64 rounding of covariances near 1e-17: twice
-// that grid is where the FP64 cells start to cost more than a launch-bound step.
+// reduction chains.  Those are faster at every size (64 x 32 x 32 cells: 43 us
+// with the host copy, against 98 us with FP64 cells and one chain; 256 x 128 x 128:
+// 174 us, against 1.65 ms) and no less exact.  The line preserves recorded output: the
+// laminar example's profiles-2.dat is kept byte for byte on 65,536 cells, with the rounding
+// of FP64 cells and one chain in covariances that are zero up to 1e-17.  It lies at twice
+// that grid, and costs smaller FP64 states the 55 us.
 constexpr long long kStatsFxCells = 1 << 17;
 
 template <class T, class S>

@@ -6,9 +6,11 @@
 // want statistics: host programs that hand all device memory to their own
 // pool or arena up front and forbid later allocations, and callers whose
 // memory budget the state arrays have already spent.  For them this file
-// provides dg_stats_values_noalloc: the same reduction over an FP64 state that
+// provides dg_stats_values_noalloc: the same statistics of an FP64 state that
 // the caller holds in device memory, with its scratch in a fixed
-// file-scope __device__ array instead of an allocation.
+// file-scope __device__ array instead of an allocation.  Its cells are in FP64 and its sums
+// one chain at every size (dg_stats_values has both only for small states, kStatsFxCells),
+// so on large grids the two agree to rounding.
 //
 // The scratch array is sized for nx <= DG_NOALLOC_MAX_NX x-indices; it is part
 // of the library's device image, so every GPU that loads the library holds it
@@ -74,7 +76,7 @@ __global__ void noalloc_reduce_kernel(const double *__restrict__ partial, int nb
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nx) return;
     double acc[dg::NSTAT];
-    dg::stats_combine_blocks(partial, nblocks, nx, i, acc);  // the reduction of dg_stats_values
+    dg::stats_combine_blocks(partial, nblocks, nx, i, acc);
     for (int s = 0; s < dg::NSTAT; ++s) total[size_t(i) * dg::NSTAT + s] = acc[s];
     const double n = double(nyz);
     const double ua = acc[1] / n, va = acc[2] / n, wa = acc[3] / n;
