@@ -136,7 +136,7 @@ def _query_with_a_small_pool():
 
 def test_query_without_device_memory_for_the_copy():
     """The device's stream-ordered pool limited to less than f-bar-plus (14 MB).  In a process of its
-    own, which keeps that pool: once it was destroyed the driver's cuStreamSynchronize crashed."""
+    own, which keeps that pool: once it was destroyed libcuda's cuStreamSynchronize crashed."""
     here = os.path.dirname(os.path.abspath(__file__))
     code = ("import conftest, test_gpu_fb_address as t; t._query_with_a_small_pool()")
     r = subprocess.run([sys.executable, "-c", code], cwd=here, capture_output=True, text=True, timeout=120)
